@@ -175,6 +175,17 @@ reset_status sss_owner(const reset_table* t, const int4* desc, const int32_t* el
                        const int32_t* pa, const int32_t* pb, int64_t np, bool float_rule,
                        int32_t num, int32_t den, float thr, uint8_t* flags, int32_t* inter,
                        cudaStream_t st);
+// One pass over a CSR (clique.cu); synchronises `st`.
+struct RowStats {
+  unsigned long long longest = 0;     // keys of the longest row
+  unsigned long long descending = 0;  // adjacent key pairs in descending-or-equal order
+  unsigned long long straddling = 0;  // ... that straddle a row boundary
+  double cubes = 0;                   // sum of the cubed row lengths
+  // every row strictly ascending
+  bool ascending() const { return descending == straddling; }
+};
+reset_status row_stats(const int32_t* d_off, const int32_t* d_cols, int32_t n, int64_t m,
+                       cudaStream_t st, RowStats* out);
 // Counts launches of libreset's own kernels (reset_kernel_launches()).
 void note_launch(int k = 1);
 }  // namespace rst

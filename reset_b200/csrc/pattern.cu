@@ -89,36 +89,6 @@ __device__ __forceinline__ int lower_bound_key(const int32_t* a, int n, int x) {
   return lo;
 }
 
-// One pass over a CSR: out[0] = the longest row (atomicMax), out[1] =
-// adjacent key pairs in descending-or-equal order, out[2] = those pairs
-// that straddle a row boundary.  Every row is strictly ascending exactly
-// when out[1] == out[2].
-__global__ void row_stats_kernel(const int32_t* __restrict__ off,
-                                 const int32_t* __restrict__ cols, int32_t n, int64_t m,
-                                 unsigned long long* __restrict__ out) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  int mx = 0;
-  unsigned long long desc_pairs = 0, edges = 0;
-  for (int64_t i = t0; i < n; i += stride) {
-    const int a = __ldg(off + i), z = __ldg(off + i + 1);
-    mx = max(mx, z - a);
-    if (z > a && z < m) edges += __ldg(cols + z - 1) >= __ldg(cols + z);
-  }
-  for (int64_t e = t0; e + 1 < m; e += stride)
-    desc_pairs += __ldg(cols + e) >= __ldg(cols + e + 1);
-  for (int o = 16; o; o >>= 1) {
-    mx = max(mx, __shfl_xor_sync(kFull, mx, o));
-    desc_pairs += __shfl_xor_sync(kFull, desc_pairs, o);
-    edges += __shfl_xor_sync(kFull, edges, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomicMax(out, (unsigned long long)mx);
-    if (desc_pairs) atomicAdd(out + 1, desc_pairs);
-    if (edges) atomicAdd(out + 2, edges);
-  }
-}
-
 template <bool HIER>
 __global__ void __launch_bounds__(kPtThreads, 5)
     pattern_kernel(const int4* __restrict__ desc, const int32_t* __restrict__ off,
@@ -542,23 +512,10 @@ extern "C" reset_status reset_pattern_count(const reset_table* t, const int32_t*
   cudaStream_t st = as_stream(stream);
   RST_CUDA(cudaMemsetAsync(d_count, 0, sizeof(uint64_t), st));
   if (m == 0 || t->n == 0) return RESET_OK;
-  unsigned long long stats[3] = {0, 0, 0};
-  {
-    unsigned long long* d_st = nullptr;
-    RST_CUDA(scratch_malloc(reinterpret_cast<void**>(&d_st), sizeof(stats), st));
-    cudaError_t e = cudaMemsetAsync(d_st, 0, sizeof(stats), st);
-    if (e == cudaSuccess) {
-      note_launch();
-      row_stats_kernel<<<sm_count() * 4, 256, 0, st>>>(d_off, d_cols, t->n, m, d_st);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(stats, d_st, sizeof(stats), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFreeAsync(d_st, st);
-    if (e != cudaSuccess) return cuda_fail(e, "row stats", __FILE__, __LINE__);
-  }
-  const int32_t cap = stats[0] > 0 ? (int32_t)stats[0] : 1;
-  const int sorted = stats[1] == stats[2] ? 1 : 0;
+  RowStats stats;
+  RST_CHECK(row_stats(d_off, d_cols, t->n, m, st, &stats));
+  const int32_t cap = stats.longest > 0 ? (int32_t)stats.longest : 1;
+  const int sorted = stats.ascending() ? 1 : 0;
   const int64_t rows = pat.k > 3 ? pat.k - 3 : 1;
   const void* kf = t->hier ? (const void*)pattern_kernel<true> : (const void*)pattern_kernel<false>;
   int per_sm = 0;

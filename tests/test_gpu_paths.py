@@ -1,0 +1,87 @@
+"""Kernel paths at the sizes where they change: edges of tiles, packed words
+and work bins, remainders, and inputs that must take the general path.
+Whole-number results, compared exactly."""
+from math import comb
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def R(cuda, libreset):
+    from reset_b200 import api
+    return api
+
+
+def dev(x, torch):
+    return torch.from_numpy(np.ascontiguousarray(x)).cuda()
+
+
+def csr(rows):
+    off = np.zeros(len(rows) + 1, np.int32)
+    off[1:] = np.cumsum([len(r) for r in rows])
+    return off, np.array([x for r in rows for x in r], np.int32)
+
+
+# ------------------------------------------------------------- k-cliques --
+
+@pytest.mark.parametrize("n,k", [
+    (33, 4), (34, 5), (35, 6), (35, 9), (66, 5), (67, 6), (68, 7), (130, 5), (131, 6), (132, 5),
+    (258, 5), (260, 6), (513, 5), (515, 5), (769, 4), (1217, 4), (1219, 4)])
+def test_clique_bit_rows_at_size_limits(R, cuda, n, k):
+    """Complete graphs around every width of the packed rows (32, 64, 128, 256,
+    512 common neighbours), the longest row held as bits, and past both."""
+    off = np.zeros(n + 1, np.int32)
+    off[1:] = np.cumsum(np.arange(n - 1, -1, -1))
+    cols = np.concatenate([np.arange(u + 1, n, dtype=np.int32) for u in range(n)])
+    d_off, d_cols = dev(off, cuda), dev(cols, cuda)
+    t = R.Table(d_off, d_cols, hierarchical=bool(n % 2))
+    assert R.clique_count(t, d_off, d_cols, k) == comb(n, k)
+    t.check()
+
+
+@pytest.mark.parametrize("bucket", [1, 5])
+@pytest.mark.parametrize("kind", ["symmetric", "loops", "shuffled", "repeated"])
+def test_clique_rows_of_every_kind(R, cuda, oracle_mod, kind, bucket):
+    """Dense random digraphs (rows on both sides of 32 keys) whose rows are
+    sets, hold the vertex itself, are out of order, or repeat keys."""
+    rng = np.random.default_rng(0x5EED7C00 + bucket)
+    n = 90
+    rows = []
+    for u in range(n):
+        p = 0.1 if u % 3 else 0.6
+        keep = np.flatnonzero(rng.random(n) < p)
+        keep = keep[keep != u] if kind != "loops" else np.union1d(keep, [u])
+        rows.append(keep)
+    if kind == "repeated":
+        rows = [np.sort(np.concatenate([r, r[::3]])) for r in rows]
+    off, cols = csr(rows)
+    want = {k: oracle_mod.clique_k(off, cols, k) for k in (4, 5, 6)} if kind != "repeated" else None
+    if kind == "shuffled":
+        for u in range(n):
+            rng.shuffle(cols[off[u]:off[u + 1]])
+    d_off, d_cols = dev(off, cuda), dev(cols, cuda)
+    t = R.Table(d_off, d_cols, alpha=0.4, bucket=bucket)
+    if want is None:  # keys of the shorter row count as often as they occur there
+        want = {k: _clique_multiset(rows, k) for k in (4, 5)}
+    for k, w in want.items():
+        assert R.clique_count(t, d_off, d_cols, k) == w, k
+    t.check()
+
+
+def _clique_multiset(rows, k):
+    sets = [set(r.tolist()) for r in rows]
+
+    def below(c, left):
+        if left == 1:
+            return sum(sum(x in sets[w] for x in c) for w in c)
+        return sum(below([x for x in c if x in sets[w]], left - 1) for w in c)
+
+    total = 0
+    for u, r in enumerate(rows):
+        for v in r:
+            a, b = (v, u) if len(r) > len(rows[v]) else (u, v)
+            total += below([x for x in rows[a].tolist() if x in sets[b]], k - 3)
+    return total
