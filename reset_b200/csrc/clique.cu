@@ -530,38 +530,54 @@ __global__ void __launch_bounds__(kCbThreads, 2)
   if (lane == 0 && hits) atomicAdd(count, hits);
 }
 
-// One pass over a CSR: the longest row, adjacent key pairs in
-// descending-or-equal order, those of them that straddle a row boundary, and
-// the sum of the cubed row lengths.
-__global__ void row_stats_kernel(const int32_t* __restrict__ off,
-                                 const int32_t* __restrict__ cols, int32_t n, int64_t m,
-                                 RowStats* __restrict__ out) {
+// One pass over a CSR for RowStats.
+__global__ void __launch_bounds__(256)
+    row_stats_kernel(const int32_t* __restrict__ off, const int32_t* __restrict__ cols,
+                     int32_t n, int64_t m, RowStats* __restrict__ out) {
+  __shared__ unsigned s_lg[32];
+  if (threadIdx.x < 32) s_lg[threadIdx.x] = 0;
+  __syncthreads();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int mx = 0;
-  unsigned long long desc_pairs = 0, edges = 0;
+  unsigned long long desc_pairs = 0, edges = 0, outside = 0, d2 = 0;
   double d3 = 0;
   for (int64_t i = t0; i < n; i += stride) {
-    const int a = __ldg(off + i), z = __ldg(off + i + 1);
-    const double d = z - a;
-    mx = max(mx, z - a);
-    d3 += d * d * d;
+    const int a = __ldg(off + i), z = __ldg(off + i + 1), d = z - a;
+    mx = max(mx, d);
+    if (d > 0) {
+      d2 += (unsigned long long)d * d;
+      d3 += (double)d * d * d;
+      atomicAdd(&s_lg[31 - __clz(d)], 1u);
+    }
     if (z > a && z < m) edges += __ldg(cols + z - 1) >= __ldg(cols + z);
   }
-  for (int64_t e = t0; e + 1 < m; e += stride)
-    desc_pairs += __ldg(cols + e) >= __ldg(cols + e + 1);
+  for (int64_t e = t0; e < m; e += stride) {
+    const int x = __ldg(cols + e);
+    outside += (unsigned)x >= (unsigned)n;
+    if (e + 1 < m) desc_pairs += x >= __ldg(cols + e + 1);
+  }
   for (int o = 16; o; o >>= 1) {
     mx = max(mx, __shfl_xor_sync(kFull, mx, o));
     desc_pairs += __shfl_xor_sync(kFull, desc_pairs, o);
     edges += __shfl_xor_sync(kFull, edges, o);
+    outside += __shfl_xor_sync(kFull, outside, o);
+    d2 += __shfl_xor_sync(kFull, d2, o);
     d3 += __shfl_xor_sync(kFull, d3, o);
   }
   if ((threadIdx.x & 31) == 0) {
     atomicMax(&out->longest, (unsigned long long)mx);
     if (desc_pairs) atomicAdd(&out->descending, desc_pairs);
     if (edges) atomicAdd(&out->straddling, edges);
-    if (d3 > 0) atomicAdd(&out->cubes, d3);
+    if (outside) atomicAdd(&out->outside, outside);
+    if (d2) {
+      atomicAdd(&out->squares, d2);
+      atomicAdd(&out->cubes, d3);
+    }
   }
+  __syncthreads();
+  if (threadIdx.x < 32 && s_lg[threadIdx.x])
+    atomicAdd(&out->lg_rows[threadIdx.x], (unsigned long long)s_lg[threadIdx.x]);
 }
 
 }  // namespace

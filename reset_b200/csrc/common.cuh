@@ -180,7 +180,10 @@ struct RowStats {
   unsigned long long longest = 0;     // keys of the longest row
   unsigned long long descending = 0;  // adjacent key pairs in descending-or-equal order
   unsigned long long straddling = 0;  // ... that straddle a row boundary
-  double cubes = 0;                   // sum of the cubed row lengths
+  unsigned long long outside = 0;     // keys outside [0, n)
+  unsigned long long squares = 0;     // sum of the squared row lengths
+  double cubes = 0;                   // ... cubed
+  unsigned long long lg_rows[32] = {};  // rows of 2^i .. 2^(i+1) - 1 keys
   // every row strictly ascending
   bool ascending() const { return descending == straddling; }
 };

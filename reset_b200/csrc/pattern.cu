@@ -3,31 +3,49 @@
 // (SMOG/SMOG_hie/subgraph_match_hie.cu:58-406) over this library's tables,
 // for any pattern in SMOG's encoding (reset_pattern in reset.h).
 //
-// One warp per start edge (dynamic 1-edge work items, as the clique
-// kernels).  The edge fixes m_0 and m_1.  Level l >= 2 builds its
-// candidate set C_l in one pass: the base is the reused level's set or the
-// shortest row among the listed backward vertices; every base key is probed
-// into the tables of the other listed rows (early exit per lane), and the
-// hits are compacted into the warp's scratch row of level l (ballot/popc).
-// A level with nothing to probe keeps a view of its base, without a copy.
+// One warp per start edge.  The edge fixes m_0 and m_1.  Level l >= 2 builds
+// its candidate set C_l in one pass: the base is the reused level's set or
+// the shortest row among the listed backward vertices; every base key is
+// looked up in the other listed rows (early exit per lane), and the hits are
+// compacted into the warp's scratch row of level l (ballot/popc).  A level
+// with nothing to look up keeps a view of its base, without a copy.
 // The last level is only counted; earlier levels are walked 32 candidates
 // at a time, the next m_l being the first lane's key that passes the
 // level's check.  Where no later level reuses C_l, keys failing l's check
 // are dropped at compaction already.  The reference instead builds C_l by
 // one pass per listed row, and walks candidates one by one.
 //
-// With strictly ascending rows (checked on the device in the same pass that
-// finds the longest row), a restriction m_l < m_r cuts the base to its
-// prefix below m_r before any probe, and a last level with nothing to probe
-// is counted without a scan: the prefix length, or |C_l| less the earlier
-// vertices that a binary search finds in it.  Such a last level is not
+// Work distribution: the search below one start edge grows with the square or
+// cube of the rows it meets, so on a skewed graph a few hub edges outlast all
+// others (R-MAT scale 9, Q6: 8% of the warps active over the run).  Edges
+// whose first set may be long are cut into parts, listed ahead of the rest;
+// a part builds C_2 again (one pass) and walks its slice of it.
+//
+// Lookups: a row is its bit row of n bits where the graph's bit matrix fits
+// kBitBudget (else the longest rows' bit rows, as many as fit), one load and
+// a shift; other rows are probed in their hash table.  Bit rows need all keys
+// in [0, n), checked in the pass that finds the longest row.
+//
+// With strictly ascending rows (checked in the same pass), a restriction
+// m_l < m_r cuts the base to its prefix below m_r before any lookup, and a
+// last level with nothing to look up is counted without a scan: the prefix
+// length, or |C_l| less the earlier vertices in it.  Such a last level is not
 // entered at all: the level before it hands one candidate to each lane,
-// which counts the last level for it.  A last level that intersects a fixed
-// vertex's row with the row of the candidate just picked (N(m_a) ∩ N(x))
-// is not entered either: such intersections of at most kLaneMax keys run
-// one candidate per lane, longer ones by the whole warp.  A reusing
+// which counts the last level for it; what does not depend on the candidate
+// (which earlier vertices the base holds, and where) is found once per visit.
+// A last level that intersects a fixed vertex's row with the row of the
+// candidate just picked (N(m_a) ∩ N(x)) is not entered either: such
+// intersections of at most kLaneMax keys run one candidate per lane, longer
+// ones by the whole warp, as AND + popcount over the two bit rows where that
+// is less work than looking up the shorter row's keys.  A reusing
 // k-clique chain without checks (SMOG's Q0, Q3, Q5, Q7) runs the k-clique
-// kernel (clique.cu).
+// count (clique.cu).
+//
+// Bound by instruction issue and, on small graphs, by the longest part.
+// Against one edge per warp with every lookup a hash probe (R-MAT, ms):
+// Q6 scale 8 / 11: 3.2 / 116 -> 0.26 / 3.6; Q4 scale 8 / 13: 0.57 / 19.8 ->
+// 0.15 / 4.8; Q8 scale 13: 20.6 -> 3.7; Q1 scale 8 / 14: 0.16 / 16.3 ->
+// 0.12 / 6.5; Q2 scale 14: 11.9 -> 3.1.
 //
 // Semantics differ from the reference in one case only: where two listed
 // vertices of a level map to the same data vertex and that vertex has the
@@ -49,6 +67,17 @@ constexpr int kPtWarps = kPtThreads / 32;
 // Scratch rows of all resident warps together stay below this; a graph
 // whose largest row would need more runs fewer warps.
 constexpr size_t kPtScratchBudget = size_t(1) << 30;
+// Bytes of bit rows at most (2x the L2; n = 46340 vertices get a whole matrix).
+constexpr int64_t kBitBudget = int64_t(1) << 28;
+// Rows shorter than this get no bit row of their own on larger graphs: their
+// hash table spans no more cache lines than the bit row's hits would.
+constexpr int kBitMinRow = 64;
+// Start edges whose first set may hold more keys than this are cut into
+// parts of about as many; a paired or fused last level right after it takes
+// 32 candidates at a time, deeper patterns have far more below a candidate.
+constexpr int kPartDeep = 8, kPartFlat = 64;
+// ... and are made longer where there would be more parts than this.
+constexpr int64_t kMaxParts = int64_t(1) << 20;
 
 struct PatternDev {
   int32_t k, flags;
@@ -89,12 +118,91 @@ __device__ __forceinline__ int lower_bound_key(const int32_t* a, int n, int x) {
   return lo;
 }
 
+// The graph's bit rows: row[y] (or y itself, row NULL) is the row of vertex
+// y, -1 = none; `words` a row, a multiple of 4.
+struct BitRows {
+  const uint32_t* bits;
+  const int32_t* row;
+  int64_t words;
+  __device__ __forceinline__ const uint32_t* of(int y) const {
+    if (!bits) return nullptr;
+    const int r = row ? __ldg(row + y) : y;
+    return r < 0 ? nullptr : bits + r * words;
+  }
+};
+
+__device__ __forceinline__ bool bit_of(const uint32_t* br, int x) {
+  return (__ldg(br + (x >> 5)) >> (x & 31)) & 1u;
+}
+
+// Rows of at least `shortest` keys get the next bit rows, in any order.
+__global__ void bit_assign_kernel(const int4* __restrict__ desc, int32_t n, int shortest,
+                                  int32_t* __restrict__ row, int32_t* __restrict__ ctr) {
+  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n;
+       u += (int64_t)gridDim.x * blockDim.x)
+    row[u] = __ldg(desc + u).y >= shortest ? atomicAdd(ctr, 1) : -1;
+}
+
+// Sets the bit rows (zeroed, all keys in [0, n)), a warp per row, and counts
+// the vertices whose row holds themselves.
+__global__ void bit_fill_kernel(const int4* __restrict__ desc, const int32_t* __restrict__ cols,
+                                int32_t n, const int32_t* __restrict__ row, int64_t words,
+                                uint32_t* __restrict__ bits, int32_t* __restrict__ loops) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t u = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; u < n; u += nw) {
+    const int4 du = __ldg(desc + u);
+    const int r = row ? __ldg(row + u) : (int)u;
+    uint32_t* br = bits + r * words;
+    for (int j = lane; j < du.y; j += 32) {
+      const int x = __ldg(cols + du.x + j);
+      if (r >= 0) atomicOr(br + (x >> 5), 1u << (x & 31));
+      if (x == u) atomicAdd(loops, 1);
+    }
+  }
+}
+
+// Keys the first set of start edge (u, v) may hold: the shortest listed row,
+// counted no longer than u's so that the parts of all edges are bounded by
+// the sum of the squared row lengths.
+__device__ __forceinline__ int first_set(const PatternDev& p, int du, int dv) {
+  int s = du;
+  for (int j = 0; j < p.nb[2]; ++j) s = min(s, p.back[2][j] == 0 ? du : dv);
+  return s;
+}
+
+// Start edges with a first set above `part` keys, as (u, v, i, parts).
+__global__ void pattern_parts_kernel(const int4* __restrict__ desc,
+                                     const int32_t* __restrict__ cols, int32_t n, int64_t m,
+                                     const PatternDev pat, int part, int4* __restrict__ list,
+                                     int32_t* __restrict__ n_list) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t u = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; u < n; u += nw) {
+    const int4 du = __ldg(desc + u);
+    if (du.y <= part) continue;
+    const int d = (int)min((int64_t)du.y, m - du.x);
+    for (int j = lane; j < d; j += 32) {
+      const int v = __ldg(cols + du.x + j);
+      const int map[2] = {(int)u, v};
+      if ((unsigned)v >= (unsigned)n || !level_ok(pat, 1, v, map)) continue;
+      const int s = first_set(pat, du.y, __ldg(&desc[v].y));
+      if (s <= part) continue;
+      const int np = (s + part - 1) / part;
+      const int at = atomicAdd(n_list, np);
+      for (int i = 0; i < np; ++i) list[at + i] = make_int4((int)u, v, i, np);
+    }
+  }
+}
+
 template <bool HIER>
-__global__ void __launch_bounds__(kPtThreads, 5)
+__global__ void __launch_bounds__(kPtThreads, 4)
     pattern_kernel(const int4* __restrict__ desc, const int32_t* __restrict__ off,
                    const int32_t* __restrict__ cols, const int32_t* __restrict__ chunk_row,
                    int32_t n, int64_t m, const int32_t* __restrict__ table, int64_t bn, int b,
-                   int lg_max, const PatternDev pat, int sorted,
+                   int lg_max, const PatternDev pat, int sorted, const BitRows br,
+                   const int32_t* __restrict__ loops, const int4* __restrict__ parts_list,
+                   const int32_t* __restrict__ n_list, int part, int lg_grab,
                    int32_t* __restrict__ scratch, int32_t cap,
                    unsigned long long* __restrict__ count,
                    unsigned long long* __restrict__ cursor, int32_t* __restrict__ status) {
@@ -108,265 +216,387 @@ __global__ void __launch_bounds__(kPtThreads, 5)
   const int rows = k > 3 ? k - 3 : 1;
   int32_t* Sbase = scratch + gw * (int64_t)cap * rows;
   const int64_t me = min(m, (int64_t)__ldg(off + n));
-  const int64_t n_chunks = (me + 31) >> 5;
+  const int grab = 1 << lg_grab;  // start edges a warp takes at a time, at most 32
+  const int64_t n_grabs = (me + grab - 1) >> lg_grab;
+  const int n_parts = part > 0 ? *n_list : 0;
+  // no row holds its own vertex (known where bit rows were set)
+  const bool loop_free = br.bits && *loops == 0;
   unsigned long long hits = 0;
-  int map[kPatMax], sz[kPatMax], it[kPatMax];
+  // level l: m_l, its index in C_l, C_l (cs, sz), the next candidate (it)
+  int map[kPatMax], idx[kPatMax], sz[kPatMax], it[kPatMax];
   const int32_t* cs[kPatMax];
   int4 pd[kPatMax];
-  int u = 0;
+  const uint32_t* pbits[kPatMax];
+  // x in the row of desc dy with bit row by
+  auto holds = [&](const uint32_t* by, const int4& dy, int x) {
+    return by ? bit_of(by, x)
+              : probe_key<HIER>(x, table + desc_toff(dy), desc_lg(dy), lg_max, bn, b, status);
+  };
+  bool listed = n_parts > 0;
   for (;;) {
+    // the next listed part, then the next edges: one start edge per lane
     unsigned long long cc = 0;
-    if (lane == 0) cc = atomicAdd(cursor, 1ull);
-    const int64_t e = (int64_t)__shfl_sync(kFull, cc, 0);
-    if (e >= me) break;
-    if (lane == 0) {  // row of edge e: largest u with off[u] <= e
-      const int64_t c = e >> 5;
-      int lo = __ldg(chunk_row + c);
-      int hi = c + 1 < n_chunks ? __ldg(chunk_row + c + 1) : n - 1;
-      if ((unsigned)lo >= (unsigned)n) lo = 0;
-      if (hi < lo || hi >= n) hi = n - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(off + mid) <= e) lo = mid; else hi = mid - 1;
+    if (lane == 0) cc = atomicAdd(cursor + (listed ? 0 : 1), 1ull);
+    const int64_t c = (int64_t)__shfl_sync(kFull, cc, 0);
+    int4 item = make_int4(0, 0, 0, 1);
+    bool start;
+    if (listed) {
+      if (c >= n_parts) {
+        listed = false;
+        continue;
       }
-      u = lo;
+      start = lane == 0;
+      if (start) item = __ldg(parts_list + c);
+    } else {
+      if (c >= n_grabs) break;
+      const int64_t e0 = c << lg_grab;
+      const int64_t e = min(e0 + min(lane, grab - 1), me - 1);
+      int u0 = __ldg(chunk_row + (e0 >> 5));
+      if ((unsigned)u0 >= (unsigned)n) u0 = 0;
+      item.x = row_of_edge(off, n, u0, (int)e);
+      item.y = __ldg(cols + e);
+      start = lane < grab && e0 + lane < me && (unsigned)item.x < (unsigned)n;
+      if (start && (unsigned)item.y >= (unsigned)n) {
+        atomicOr(status, kErrBadId);
+        start = false;
+      }
+      if (start) {
+        const int ends[2] = {item.x, item.y};
+        start = level_ok(sp, 1, item.y, ends) &&
+                !(part > 0 &&
+                  first_set(sp, __ldg(&desc[item.x].y), __ldg(&desc[item.y].y)) > part);
+      }
     }
-    u = __shfl_sync(kFull, u, 0);
-    const int v = __ldg(cols + e);
-    if ((unsigned)v >= (unsigned)n) {
-      if (lane == 0) atomicOr(status, kErrBadId);
-      continue;
-    }
-    map[0] = u;
-    map[1] = v;
-    if (!level_ok(sp, 1, v, map)) continue;
-    int lv = 2;  // warp-uniform depth
-    bool build = true;
-    while (lv >= 2) {
-      if (build) {
-        build = false;
-        // the base of C_lv: the reused set, or the shortest listed row
-        const int32_t* src = cols;
-        int ns = 0, bv = -1;
-        const int r = sp.reuse[lv];
-        if (r >= 0) {
-          src = cs[r];
-          ns = sz[r];
-        } else {
-          ns = INT_MAX;
+    for (unsigned todo = __ballot_sync(kFull, start); todo; todo &= todo - 1) {
+      const int f = __ffs(todo) - 1;
+      map[0] = __shfl_sync(kFull, item.x, f);
+      map[1] = __shfl_sync(kFull, item.y, f);
+      const int my_part = __shfl_sync(kFull, item.z, f), parts = __shfl_sync(kFull, item.w, f);
+      int end2 = 0;  // candidates of level 2 end here (a part's slice of C_2)
+      int lv = 2;    // warp-uniform depth
+      bool build = true;
+      while (lv >= 2) {
+        if (build) {
+          build = false;
+          // the base of C_lv: the reused set, or the shortest listed row
+          const int32_t* src = cols;
+          int ns = 0, bv = -1;
+          const int r = sp.reuse[lv];
+          if (r >= 0) {
+            src = cs[r];
+            ns = sz[r];
+          } else {
+            ns = INT_MAX;
+            for (int j = 0; j < sp.nb[lv]; ++j) {
+              const int y = map[sp.back[lv][j]];
+              const int4 dy = __ldg(desc + y);
+              if (dy.y < ns) {
+                ns = dy.y;
+                bv = y;
+                src = cols + dy.x;
+              }
+            }
+          }
+          // the other listed rows, each once, are looked up
+          int np = 0;
           for (int j = 0; j < sp.nb[lv]; ++j) {
             const int y = map[sp.back[lv][j]];
+            if (y == bv) continue;
+            bool seen = false;
+            for (int q = 0; q < j; ++q) seen |= map[sp.back[lv][q]] == y;
+            if (seen) continue;
             const int4 dy = __ldg(desc + y);
-            if (dy.y < ns) {
-              ns = dy.y;
-              bv = y;
-              src = cols + dy.x;
-            }
+            if (dy.y == 0) ns = 0;
+            pbits[np] = br.of(y);
+            pd[np++] = dy;
           }
-        }
-        // the other listed rows, each once, are probed
-        int np = 0;
-        for (int j = 0; j < sp.nb[lv]; ++j) {
-          const int y = map[sp.back[lv][j]];
-          if (y == bv) continue;
-          bool seen = false;
-          for (int q = 0; q < j; ++q) seen |= map[sp.back[lv][q]] == y;
-          if (seen) continue;
-          const int4 dy = __ldg(desc + y);
-          if (dy.y == 0) ns = 0;
-          pd[np++] = dy;
-        }
-        const bool last = lv == k - 1;
-        const int rr = sp.restr[lv];
-        // ascending rows: the keys a restriction m_lv < m_rr admits are a
-        // prefix of the base (cut only where no later level reuses C_lv)
-        if (sorted && (sp.flags & RESET_PATTERN_RESTRICT) && rr >= 0 && (last || sp.filt[lv]))
-          ns = lower_bound_key(src, ns, map[rr]);
-        if (last && np == 0 && sorted) {
-          // C_lv is the base itself: |C_lv| less the earlier vertices in it
-          int c = ns;
-          if ((sp.flags & RESET_PATTERN_DISTINCT) && rr < 0)
-            for (int i = 0; i < lv; ++i) {
-              const int y = map[i];
-              bool seen = false;
-              for (int q = 0; q < i; ++q) seen |= map[q] == y;
-              if (seen) continue;
-              const int at = lower_bound_key(src, ns, y);
-              if (at < ns && src[at] == y) --c;
-            }
-          if (lane == 0) hits += c;
-          --lv;
-          continue;
-        }
-        if (np == 0 && !last) {  // a view of the base
-          cs[lv] = src;
-          sz[lv] = ns;
-          it[lv] = 0;
-        } else {
-          int32_t* dst = Sbase + (int64_t)(lv - 2) * cap;
-          const bool chk = last || sp.filt[lv];
-          int nw = 0;
-          for (int j0 = 0; j0 < ns; j0 += 32) {
-            const int j = j0 + lane;
-            bool in = false;
-            int x = 0;
-            if (j < ns) {
-              x = src[j];  // plain load: src may be this warp's scratch
-              in = !chk || level_ok(sp, lv, x, map);
-              for (int q = 0; in && q < np; ++q)
-                in = probe_key<HIER>(x, table + desc_toff(pd[q]), desc_lg(pd[q]), lg_max, bn, b,
-                                     status);
-            }
-            if (last) {
-              hits += in;
-            } else {
-              const unsigned msk = __ballot_sync(kFull, in);
-              if (in) {
-                const int pos = nw + __popc(msk & lt);
-                if (pos < cap) dst[pos] = x;
+          const bool last = lv == k - 1;
+          const int rr = sp.restr[lv];
+          // ascending rows: the keys a restriction m_lv < m_rr admits are a
+          // prefix of the base (cut only where no later level reuses C_lv);
+          // m_rr's own index where the base is m_rr's set
+          if (sorted && (sp.flags & RESET_PATTERN_RESTRICT) && rr >= 0 && (last || sp.filt[lv]))
+            ns = rr >= 2 && src == cs[rr] && idx[rr] < ns ? idx[rr]
+                                                          : lower_bound_key(src, ns, map[rr]);
+          if (last && np == 0 && sorted) {
+            // C_lv is the base itself: |C_lv| less the earlier vertices in it
+            int c2 = ns;
+            if ((sp.flags & RESET_PATTERN_DISTINCT) && rr < 0)
+              for (int i = 0; i < lv; ++i) {
+                const int y = map[i];
+                bool seen = false;
+                for (int q = 0; q < i; ++q) seen |= map[q] == y;
+                if (seen) continue;
+                const int at = lower_bound_key(src, ns, y);
+                if (at < ns && src[at] == y) --c2;
               }
-              nw += __popc(msk);
-            }
-          }
-          if (!last) {
-            if (nw > cap) {  // cannot happen: no set outgrows the longest row
-              if (lane == 0) atomicOr(status, kErrProbeLimit);
-              nw = cap;
-            }
-            __syncwarp();
-            cs[lv] = dst;
-            sz[lv] = nw;
-            it[lv] = 0;
-          }
-        }
-        if (last) {
-          --lv;
-          continue;
-        }
-      }
-      if (sp.pair && lv == k - 2) {
-        // the last level is N(m_a) ∩ N(x) for the candidate x: short
-        // intersections run one candidate per lane (each lane holds its own
-        // m_lv = x in its copy of map), long ones afterwards by the warp
-        const int L = k - 1, rr = sp.restr[L];
-        const bool rcut = sorted && (sp.flags & RESET_PATTERN_RESTRICT) && rr >= 0;
-        const int4 da = __ldg(desc + map[sp.pair_a]);
-        for (int j0 = it[lv]; j0 < sz[lv]; j0 += 32) {
-          const int j = j0 + lane;
-          int x = j < sz[lv] ? cs[lv][j] : 0;
-          bool act = j < sz[lv];
-          if (act && (unsigned)x >= (unsigned)n) {
-            atomicOr(status, kErrBadId);
-            act = false;
-          }
-          act = act && level_ok(sp, lv, x, map);
-          int len = 0;
-          const int32_t* base = cols;
-          const int32_t* tb = table;
-          int tlg = 0;
-          if (act) {
-            const int4 dx = __ldg(desc + x);
-            const int4 db = dx.y <= da.y ? dx : da, dt = dx.y <= da.y ? da : dx;
-            base = cols + db.x;
-            len = dt.y > 0 ? db.y : 0;
-            tb = table + desc_toff(dt);
-            tlg = desc_lg(dt);
-            if (rcut) len = lower_bound_key(base, len, rr == lv ? x : map[rr]);
-          }
-          const bool big = len > kLaneMax;
-          if (!big && len > 0) {
-            map[lv] = x;
-            unsigned long long c = 0;
-            for (int t = 0; t < len; ++t) {
-              const int z = base[t];
-              c += level_ok(sp, L, z, map) && probe_key<HIER>(z, tb, tlg, lg_max, bn, b, status);
-            }
-            hits += c;
-          }
-          for (unsigned bm = __ballot_sync(kFull, big); bm; bm &= bm - 1) {
-            const int f = __ffs(bm) - 1;
-            const int xb = __shfl_sync(kFull, x, f);
-            const int lb = __shfl_sync(kFull, len, f);
-            const int32_t* bb = cols + __shfl_sync(kFull, (int)(base - cols), f);
-            const int4 dx = __ldg(desc + xb);
-            const int4 dt = dx.y <= da.y ? da : dx;
-            map[lv] = xb;
-            for (int t = lane; t < lb; t += 32) {
-              const int z = bb[t];
-              hits += level_ok(sp, L, z, map) &&
-                      probe_key<HIER>(z, table + desc_toff(dt), desc_lg(dt), lg_max, bn, b, status);
-            }
-          }
-        }
-        --lv;
-        continue;
-      }
-      if (sorted && sp.fuse && lv == k - 2) {
-        // the last level probes nothing: every key x of C_lv that passes
-        // lv's check is m_lv for one lane, which counts the last level's
-        // keys for it at once (prefix below the restriction bound, less
-        // the earlier vertices found in the base), without building it
-        const int L = k - 1, rr = sp.restr[L], ru = sp.reuse[L];
-        const bool rcut = (sp.flags & RESET_PATTERN_RESTRICT) && rr >= 0;
-        const bool dist = (sp.flags & RESET_PATTERN_DISTINCT) && rr < 0;
-        for (int j = it[lv] + lane; j < sz[lv]; j += 32) {
-          const int x = cs[lv][j];
-          if ((unsigned)x >= (unsigned)n) {
-            atomicOr(status, kErrBadId);
+            if (lane == 0) hits += c2;
+            --lv;
             continue;
           }
-          if (!level_ok(sp, lv, x, map)) continue;
-          const int32_t* base;
-          int nbase;
-          if (ru >= 0) {
-            base = cs[ru];
-            nbase = sz[ru];
+          if (np == 0 && !last) {  // a view of the base
+            cs[lv] = src;
+            sz[lv] = ns;
           } else {
-            const int lj = sp.back[L][0];
-            const int4 dy = __ldg(desc + (lj == lv ? x : map[lj]));
-            base = cols + dy.x;
-            nbase = dy.y;
-          }
-          if (rcut) nbase = lower_bound_key(base, nbase, rr == lv ? x : map[rr]);
-          int c = nbase;
-          if (dist)
-            for (int i = 0; i <= lv; ++i) {
-              const int y = i == lv ? x : map[i];
-              bool seen = false;
-              for (int q = 0; q < i; ++q) seen |= map[q] == y;
-              if (seen) continue;
-              const int at = lower_bound_key(base, nbase, y);
-              if (at < nbase && base[at] == y) --c;
+            int32_t* dst = Sbase + (int64_t)(lv - 2) * cap;
+            const bool chk = last || sp.filt[lv];
+            int nw = 0;
+            for (int j0 = 0; j0 < ns; j0 += 32) {
+              const int j = j0 + lane;
+              bool in = false;
+              int x = 0;
+              if (j < ns) {
+                x = src[j];  // plain load: src may be this warp's scratch
+                in = !chk || level_ok(sp, lv, x, map);
+                for (int q = 0; in && q < np; ++q) in = holds(pbits[q], pd[q], x);
+              }
+              if (last) {
+                hits += in;
+              } else {
+                const unsigned msk = __ballot_sync(kFull, in);
+                if (in) {
+                  const int pos = nw + __popc(msk & lt);
+                  if (pos < cap) dst[pos] = x;
+                }
+                nw += __popc(msk);
+              }
             }
-          hits += c;
+            if (!last) {
+              if (nw > cap) {  // cannot happen: no set outgrows the longest row
+                if (lane == 0) atomicOr(status, kErrProbeLimit);
+                nw = cap;
+              }
+              __syncwarp();
+              cs[lv] = dst;
+              sz[lv] = nw;
+            }
+          }
+          if (last) {
+            --lv;
+            continue;
+          }
+          it[lv] = 0;
+          if (lv == 2) {
+            it[2] = (int)((int64_t)sz[2] * my_part / parts);
+            end2 = (int)((int64_t)sz[2] * (my_part + 1) / parts);
+          }
         }
-        --lv;
-        continue;
-      }
-      // the next key of C_lv that passes the level's check becomes m_lv
-      int x = -1;
-      while (it[lv] < sz[lv]) {
-        const int j = it[lv] + lane;
-        const int y = j < sz[lv] ? cs[lv][j] : 0;
-        const bool bad = j < sz[lv] && (unsigned)y >= (unsigned)n;
-        if (bad) atomicOr(status, kErrBadId);
-        const bool ok = j < sz[lv] && !bad && level_ok(sp, lv, y, map);
-        const unsigned msk = __ballot_sync(kFull, ok);
-        if (msk) {
-          const int f = __ffs(msk) - 1;
-          x = __shfl_sync(kFull, y, f);
-          it[lv] += f + 1;
-          break;
+        const int end = lv == 2 ? end2 : sz[lv];
+        if (sp.pair && lv == k - 2) {
+          // the last level is N(m_a) ∩ N(x) for the candidate x: short
+          // intersections run one candidate per lane, long ones afterwards
+          // by the warp
+          const int L = k - 1, rr = sp.restr[L];
+          const bool rcut = sorted && (sp.flags & RESET_PATTERN_RESTRICT) && rr >= 0;
+          const bool dist = (sp.flags & RESET_PATTERN_DISTINCT) && rr < 0;
+          // keys to be checked one by one: only where rows may be out of
+          // order or repeat keys
+          const bool chk = !sorted && ((sp.flags & RESET_PATTERN_RESTRICT) || dist);
+          const int ma = map[sp.pair_a];
+          const int4 da = __ldg(desc + ma);
+          const uint32_t* ba = br.of(ma);
+          unsigned in_a = 0;  // earlier vertices (each once) that N(m_a) holds
+          if (sorted && dist) {
+            bool in = false;
+            if (lane < lv) {
+              in = !(loop_free && map[lane] == ma);
+              for (int q = 0; q < lane; ++q) in = in && map[q] != map[lane];
+              in = in && da.y > 0 && holds(ba, da, map[lane]);
+            }
+            in_a = __ballot_sync(kFull, in);
+          }
+          for (int j0 = it[lv]; j0 < end; j0 += 32) {
+            const int j = j0 + lane;
+            int x = j < end ? cs[lv][j] : 0;
+            bool act = j < end;
+            if (act && (unsigned)x >= (unsigned)n) {
+              atomicOr(status, kErrBadId);
+              act = false;
+            }
+            act = act && level_ok(sp, lv, x, map);
+            int len = 0, bound = n;
+            bool a_base = false;  // the shorter row is m_a's
+            const uint32_t* bx = nullptr;
+            int4 dx = make_int4(0, 0, 0, 0);
+            if (act) {
+              dx = __ldg(desc + x);
+              a_base = dx.y > da.y;
+              len = min(dx.y, da.y);
+              bx = br.of(x);
+              if (rcut) {
+                bound = rr == lv ? x : map[rr];
+                len = lower_bound_key(cols + (a_base ? da.x : dx.x), len, bound);
+              }
+            }
+            const int32_t* base = cols + (a_base ? da.x : dx.x);
+            const int4 dt = a_base ? dx : da;
+            const uint32_t* bt = a_base ? bx : ba;
+            const bool big = len > kLaneMax;
+            if (!big && len > 0) {
+              unsigned long long c2 = 0;
+              if (chk) {
+                map[lv] = x;
+                for (int t = 0; t < len; ++t) {
+                  const int z = base[t];
+                  c2 += level_ok(sp, L, z, map) && holds(bt, dt, z);
+                }
+              } else {
+#pragma unroll 4
+                for (int t = 0; t < len; ++t) c2 += holds(bt, dt, base[t]);
+              }
+              hits += c2;
+            }
+            if (sorted && dist && len > 0) {
+              // less the earlier vertices in both rows
+              for (unsigned q = in_a; q; q &= q - 1) hits -= holds(bx, dx, map[__ffs(q) - 1]);
+              if (!loop_free && holds(bx, dx, x)) {
+                bool seen = false;
+                for (int q = 0; q < lv; ++q) seen |= map[q] == x;
+                if (!seen && holds(ba, da, x)) --hits;
+              }
+            }
+            for (unsigned bm = __ballot_sync(kFull, big); bm; bm &= bm - 1) {
+              const int g = __ffs(bm) - 1;
+              const int xb = __shfl_sync(kFull, x, g);
+              const int lb = __shfl_sync(kFull, len, g);
+              const int kb = __shfl_sync(kFull, bound, g);
+              const uint32_t* bxb = br.of(xb);
+              const int full = kb >> 5;  // whole words below the bound
+              // a word step is one AND + popcount on 128 words, a key step a
+              // lookup of 32 keys: about as many instructions
+              if (sorted && ba && bxb && full < 4 * lb) {
+                const int4* wa = reinterpret_cast<const int4*>(ba);
+                const int4* wx = reinterpret_cast<const int4*>(bxb);
+                unsigned t = 0;
+                for (int q = lane; 4 * q < full; q += 32) {
+                  const int4 p = __ldg(wa + q), r2 = __ldg(wx + q);
+                  unsigned w[4] = {(unsigned)(p.x & r2.x), (unsigned)(p.y & r2.y),
+                                   (unsigned)(p.z & r2.z), (unsigned)(p.w & r2.w)};
+#pragma unroll
+                  for (int i = 0; i < 4; ++i) t += 4 * q + i < full ? __popc(w[i]) : 0;
+                }
+                if (lane == 0 && (kb & 31))
+                  t += __popc(__ldg(ba + full) & __ldg(bxb + full) & ((1u << (kb & 31)) - 1));
+                hits += t;
+                continue;
+              }
+              const int4 dxb = __ldg(desc + xb);
+              const bool ab = dxb.y > da.y;
+              const int32_t* bb = cols + (ab ? da.x : dxb.x);
+              const int4 dtb = ab ? dxb : da;
+              const uint32_t* btb = ab ? bxb : ba;
+              if (chk) {
+                map[lv] = xb;
+                for (int t = lane; t < lb; t += 32) {
+                  const int z = bb[t];
+                  hits += level_ok(sp, L, z, map) && holds(btb, dtb, z);
+                }
+              } else {
+#pragma unroll 4
+                for (int t = lane; t < lb; t += 32) hits += holds(btb, dtb, bb[t]);
+              }
+            }
+          }
+          --lv;
+          continue;
         }
-        it[lv] += 32;
+        if (sorted && sp.fuse && lv == k - 2) {
+          // the last level looks up nothing: every key x of C_lv that passes
+          // lv's check is m_lv for one lane, which counts the last level's
+          // keys for it at once (prefix below the restriction bound, less
+          // the earlier vertices found in the base), without building it
+          const int L = k - 1, rr = sp.restr[L], ru = sp.reuse[L];
+          const bool rcut = (sp.flags & RESET_PATTERN_RESTRICT) && rr >= 0;
+          const bool dist = (sp.flags & RESET_PATTERN_DISTINCT) && rr < 0;
+          // the base: the same for every x, unless it is x's own row
+          const bool fixed = ru >= 0 || sp.back[L][0] != lv;
+          const int32_t* base = nullptr;
+          int nbase = 0, at_bound = 0, kept = 0;
+          if (fixed) {
+            if (ru >= 0) {
+              base = cs[ru];
+              nbase = sz[ru];
+            } else {
+              const int4 dy = __ldg(desc + map[sp.back[L][0]]);
+              base = cols + dy.x;
+              nbase = dy.y;
+            }
+            if (rcut && rr != lv) nbase = lower_bound_key(base, nbase, map[rr]);
+            if (dist) {  // (no bound then) the base's keys but the earlier vertices
+              bool in = false;
+              if (lane < lv) {
+                const int y = map[lane];
+                bool seen = false;
+                for (int q = 0; q < lane; ++q) seen |= map[q] == y;
+                const int at = lower_bound_key(base, nbase, y);
+                in = !seen && at < nbase && base[at] == y;
+              }
+              kept = nbase - __popc(__ballot_sync(kFull, in));
+            }
+          }
+          const bool same = fixed && base == cs[lv];  // x's index in the base is j, if below nbase
+          for (int j = it[lv] + lane; j < end; j += 32) {
+            const int x = cs[lv][j];
+            if ((unsigned)x >= (unsigned)n) {
+              atomicOr(status, kErrBadId);
+              continue;
+            }
+            if (!level_ok(sp, lv, x, map)) continue;
+            if (!fixed) {
+              const int4 dx = __ldg(desc + x);
+              base = cols + dx.x;
+              nbase = dx.y;
+              if (rcut && rr != lv) nbase = lower_bound_key(base, nbase, map[rr]);
+            }
+            int c2 = nbase;
+            if (rcut && rr == lv)
+              c2 = same ? min(j, nbase) : lower_bound_key(base, nbase, x);
+            if (dist && fixed) {
+              bool seen = false;
+              for (int q = 0; q < lv; ++q) seen |= map[q] == x;
+              at_bound = same ? j : lower_bound_key(base, nbase, x);
+              c2 = kept - (!seen && at_bound < nbase && (same || base[at_bound] == x));
+            } else if (dist) {
+              for (int i = 0; i <= lv; ++i) {
+                const int y = i == lv ? x : map[i];
+                bool seen = false;
+                for (int q = 0; q < i; ++q) seen |= map[q] == y;
+                if (seen) continue;
+                const int at = lower_bound_key(base, nbase, y);
+                if (at < nbase && base[at] == y) --c2;
+              }
+            }
+            hits += c2;
+          }
+          --lv;
+          continue;
+        }
+        // the next key of C_lv that passes the level's check becomes m_lv
+        int x = -1;
+        while (it[lv] < end) {
+          const int j = it[lv] + lane;
+          const int y = j < end ? cs[lv][j] : 0;
+          const bool bad = j < end && (unsigned)y >= (unsigned)n;
+          if (bad) atomicOr(status, kErrBadId);
+          const bool ok = j < end && !bad && level_ok(sp, lv, y, map);
+          const unsigned msk = __ballot_sync(kFull, ok);
+          if (msk) {
+            const int g = __ffs(msk) - 1;
+            x = __shfl_sync(kFull, y, g);
+            idx[lv] = it[lv] + g;
+            it[lv] += g + 1;
+            break;
+          }
+          it[lv] += 32;
+        }
+        if (x < 0) {
+          --lv;
+          continue;
+        }
+        map[lv] = x;
+        ++lv;
+        build = true;
       }
-      if (x < 0) {
-        --lv;
-        continue;
-      }
-      map[lv] = x;
-      ++lv;
-      build = true;
     }
   }
   hits = warp_sum_u64(hits);
@@ -517,35 +747,96 @@ extern "C" reset_status reset_pattern_count(const reset_table* t, const int32_t*
   const int32_t cap = stats.longest > 0 ? (int32_t)stats.longest : 1;
   const int sorted = stats.ascending() ? 1 : 0;
   const int64_t rows = pat.k > 3 ? pat.k - 3 : 1;
+  const int sms = sm_count();
   const void* kf = t->hier ? (const void*)pattern_kernel<true> : (const void*)pattern_kernel<false>;
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kf, kPtThreads, 0);
   if (per_sm < 1) per_sm = 1;
   const size_t per_block = sizeof(int32_t) * (size_t)cap * (size_t)rows * kPtWarps;
   const int64_t fit = std::max<int64_t>(1, (int64_t)(kPtScratchBudget / per_block));
-  const int64_t grid = std::min<int64_t>(std::min<int64_t>((int64_t)sm_count() * per_sm, fit),
-                                         (m + kPtWarps - 1) / kPtWarps);
-  int32_t* d_scr = nullptr;
-  unsigned long long* d_cur = nullptr;
-  RST_CUDA(scratch_malloc(reinterpret_cast<void**>(&d_scr), per_block * (size_t)grid, st));
-  cudaError_t e = scratch_malloc(reinterpret_cast<void**>(&d_cur), sizeof(unsigned long long), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d_cur, 0, sizeof(unsigned long long), st);
-  if (e == cudaSuccess) {
+  int64_t grid = std::min<int64_t>((int64_t)sms * per_sm, fit);
+  // bit rows: all vertices', or those of the longest rows that fit
+  BitRows br{nullptr, nullptr, ((int64_t)t->n + 127) / 128 * 4};
+  int64_t bit_rows = 0;
+  int bit_min = 0;
+  if (stats.outside == 0) {
+    const int64_t most = kBitBudget / (4 * br.words);
+    if (t->n <= most) {
+      bit_rows = t->n;
+    } else {
+      for (int i = 30; i >= 0 && (1 << i) >= kBitMinRow; --i) {
+        if (bit_rows + (int64_t)stats.lg_rows[i] > most) break;
+        bit_rows += (int64_t)stats.lg_rows[i];
+        bit_min = 1 << i;
+      }
+    }
+  }
+  // parts of long start edges: there are at most 2 * squares / part of them
+  int part = 0;
+  int64_t max_parts = 0;
+  if (pat.k > 3) {
+    const int least = pat.k > 4 ? kPartDeep : kPartFlat;
+    const unsigned long long by_count = 2 * stats.squares / (unsigned long long)kMaxParts;
+    part = (int)std::min<unsigned long long>(std::max<unsigned long long>(least, by_count), INT_MAX);
+    max_parts = (int64_t)(2 * stats.squares / part) + 1;
+  }
+  // up to 32 start edges at a time, fewer where that leaves warps idle; warps
+  // beyond the work items (parts, grabs of edges) have nothing to do
+  int lg_grab = 0;
+  while (lg_grab < 5 && (m >> (lg_grab + 1)) >= grid * kPtWarps * 8) ++lg_grab;
+  grid = std::min<int64_t>(grid, ((m >> lg_grab) + 1 + max_parts + kPtWarps - 1) / kPtWarps);
+  auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
+  const bool some = bit_rows > 0 && bit_rows < t->n;
+  const size_t sz_scr = al(per_block * (size_t)grid);
+  const size_t sz_bits = al(sizeof(uint32_t) * (size_t)(bit_rows * br.words));
+  const size_t sz_row = some ? al(sizeof(int32_t) * (size_t)t->n) : 0;
+  const size_t sz_list = al(sizeof(int4) * (size_t)max_parts);
+  char* base = nullptr;
+  RST_CUDA(scratch_malloc(reinterpret_cast<void**>(&base), sz_scr + sz_bits + sz_row + sz_list + 256,
+                          st));
+  int32_t* scr = reinterpret_cast<int32_t*>(base);
+  uint32_t* bits = reinterpret_cast<uint32_t*>(base + sz_scr);
+  int32_t* row = reinterpret_cast<int32_t*>(base + sz_scr + sz_bits);
+  int4* list = reinterpret_cast<int4*>(base + sz_scr + sz_bits + sz_row);
+  // [0..1] work cursors (u64), then the listed parts, self-loops, bit rows
+  auto* cursor = reinterpret_cast<unsigned long long*>(base + sz_scr + sz_bits + sz_row + sz_list);
+  int32_t* ctr = reinterpret_cast<int32_t*>(cursor + 2);
+  const int warp_grid = (int)std::min<int64_t>(((int64_t)t->n + 7) / 8, (int64_t)sms * 8);
+  cudaError_t e = cudaMemsetAsync(cursor, 0, 256, st);
+  if (e == cudaSuccess && bit_rows > 0) {
+    br.bits = bits;
+    e = cudaMemsetAsync(bits, 0, sizeof(uint32_t) * (size_t)(bit_rows * br.words), st);
+    if (e == cudaSuccess && some) {
+      br.row = row;
+      note_launch();
+      bit_assign_kernel<<<warp_grid, 256, 0, st>>>(t->d_desc, t->n, bit_min, row, ctr + 2);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) {
+      note_launch();
+      bit_fill_kernel<<<warp_grid, 256, 0, st>>>(t->d_desc, d_cols, t->n, br.row, br.words, bits,
+                                                 ctr + 1);
+      e = cudaGetLastError();
+    }
+  }
+  if (e == cudaSuccess && part > 0) {
     note_launch();
-    if (t->hier)
-      pattern_kernel<true><<<(int)grid, kPtThreads, 0, st>>>(
-          t->d_desc, d_off, d_cols, t->d_chunk_row, t->n, m, t->d_table, t->bucket_num,
-          t->bucket, t->lg_max, pat, sorted, d_scr, cap, reinterpret_cast<unsigned long long*>(d_count),
-          d_cur, t->d_status);
-    else
-      pattern_kernel<false><<<(int)grid, kPtThreads, 0, st>>>(
-          t->d_desc, d_off, d_cols, t->d_chunk_row, t->n, m, t->d_table, t->bucket_num,
-          t->bucket, t->lg_max, pat, sorted, d_scr, cap, reinterpret_cast<unsigned long long*>(d_count),
-          d_cur, t->d_status);
+    pattern_parts_kernel<<<warp_grid, 256, 0, st>>>(t->d_desc, d_cols, t->n, m, pat, part, list,
+                                                    ctr);
     e = cudaGetLastError();
   }
-  cudaFreeAsync(d_scr, st);
-  if (d_cur) cudaFreeAsync(d_cur, st);
+  if (e == cudaSuccess) {
+    note_launch();
+#define PT_LAUNCH(H)                                                                           \
+  pattern_kernel<H><<<(int)grid, kPtThreads, 0, st>>>(                                         \
+      t->d_desc, d_off, d_cols, t->d_chunk_row, t->n, m, t->d_table, t->bucket_num, t->bucket, \
+      t->lg_max, pat, sorted, br, ctr + 1, list, ctr, part, lg_grab, scr, cap,                 \
+      reinterpret_cast<unsigned long long*>(d_count), cursor, t->d_status)
+    if (t->hier) PT_LAUNCH(true); else PT_LAUNCH(false);
+#undef PT_LAUNCH
+    e = cudaGetLastError();
+  }
+  cudaFreeAsync(base, st);
   if (e != cudaSuccess) return cuda_fail(e, "pattern_kernel", __FILE__, __LINE__);
   return RESET_OK;
 }

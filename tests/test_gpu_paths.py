@@ -85,3 +85,52 @@ def _clique_multiset(rows, k):
             a, b = (v, u) if len(r) > len(rows[v]) else (u, v)
             total += below([x for x in rows[a].tolist() if x in sets[b]], k - 3)
     return total
+
+
+# -------------------------------------------------------------- patterns --
+
+def _patterns(R):
+    P = R.PatternSpec
+    out = dict(R.PATTERNS)
+    out["tail_bound"] = P(4, (0, 1, 3, 4), (0, 0, 1, 2), (-1, 0, -1, 2), None, 3)
+    out["tail_distinct"] = P(4, (0, 1, 3, 4), (0, 0, 1, 2), (-1, 0, -1, -1), None, 3)
+    out["pair_distinct"] = P(4, (0, 1, 2, 4), (0, 0, 1, 2), (-1, -1, -1, -1), None, 2)
+    out["pair_own_bound"] = P(4, (0, 1, 2, 4), (0, 0, 1, 2), (-1, -1, -1, 2), None, 1)
+    out["triangle_bound"] = P(3, (0, 1, 3), (0, 0, 1), (-1, 0, 1), None, 1)
+    return out
+
+
+def _oracle_pattern(oracle_mod, off, cols, p):
+    return oracle_mod.pattern_count(off, cols, p.k, p.flags, p.offsets, p.backward,
+                                    p.restriction, p.reuse)
+
+
+@pytest.mark.parametrize("n,density,loops", [(61, 0.3, True), (128, 0.2, False), (201, 0.35, True)])
+def test_patterns_on_digraphs(R, cuda, oracle_mod, n, density, loops):
+    """Rows that are not symmetric and may hold their own vertex; vertex
+    counts around whole words of the bit rows; first sets cut into parts."""
+    rng = np.random.default_rng(0x5EED7D00 + n)
+    rows = []
+    for u in range(n):
+        keep = np.flatnonzero(rng.random(n) < density * (2 if u % 9 == 0 else 0.5))
+        rows.append(keep if loops else keep[keep != u])
+    off, cols = csr(rows)
+    d_off, d_cols = dev(off, cuda), dev(cols, cuda)
+    t = R.Table(d_off, d_cols, hierarchical=bool(n % 2))
+    for name, p in _patterns(R).items():
+        assert R.pattern_count(t, d_off, d_cols, p) == _oracle_pattern(oracle_mod, off, cols, p), name
+    t.check()
+
+
+def test_patterns_with_bit_rows_for_hubs_only(R, cuda, oracle_mod):
+    """More vertices than a whole bit matrix takes: the long rows have bit
+    rows, the others are probed in their tables."""
+    off, cols = oracle_mod.rmat_graph(17, 1, 0x5EED7D17, oriented=False)
+    assert (np.diff(off) >= 64).any()
+    d_off, d_cols = dev(off, cuda), dev(cols, cuda)
+    t = R.Table(d_off, d_cols)
+    for name, p in _patterns(R).items():
+        if p.graph == "symmetric" and not name.startswith("pair") and name != "tail_distinct":
+            assert R.pattern_count(t, d_off, d_cols, p) == \
+                _oracle_pattern(oracle_mod, off, cols, p), name
+    t.check()
