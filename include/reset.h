@@ -140,13 +140,15 @@ reset_status reset_tc_count(const reset_table *t, const int32_t *d_off,
                             uint64_t *d_count, reset_stream_t stream);
 
 /* reset_tc_count with an explicit method (same count either way):
- *   0 = default (1, the faster on B200 as measured);
- *   1 = edge-flattened: 32 edges per warp; pairs with at least
+ *   0 = default: 3 from 2^19 edges on where d_cols is 16-byte aligned, else 1;
+ *   1 = edge-flattened: up to 32 edges per warp; pairs with at least
  *       warp_pair_min keys (reset_tuning, default 64) probed by the whole
  *       warp, smaller ones flattened across the lanes, both sides read from
  *       HBM (the reference's access pattern);
  *   2 = vertex-staged: each row staged once in shared memory (keys + hash
- *       set) and reused by all its out-edges. */
+ *       set) and reused by all its out-edges;
+ *   3 = owner-grouped: edges grouped by the set whose table they probe, each
+ *       such set staged in shared memory once (d_cols 16-byte aligned). */
 reset_status reset_tc_count_ex(const reset_table *t, const int32_t *d_off,
                                const int32_t *d_cols, int64_t m,
                                int32_t method, uint64_t *d_count,

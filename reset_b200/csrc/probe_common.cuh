@@ -326,19 +326,24 @@ __device__ __forceinline__ int warp_probe_pair_lean(const int32_t* __restrict__ 
 // then the loads of slots 0 and 1 of each home bucket (two independent
 // loads per probe: with load factor 0.2 and 5-slot buckets almost every
 // probe is settled by these two), and only then the rare longer walks.
+// Rows: how key j of the row that starts at a_j is read.
 // For every hit, on_hit(k) is called on the lane that probed, with k the
 // lane index of the owning pair; returns the number of hits of this lane.
 constexpr int kRounds = 4;
 
-template <bool HIER, class OnHit>
+struct PlainRows {
+  static __device__ __forceinline__ int key(const int32_t* keys, int start, int j) {
+    return __ldg(keys + start + j);
+  }
+};
+
+template <bool HIER, class Rows = PlainRows, class OnHit>
 __device__ __forceinline__ int flat_probe(const int32_t* __restrict__ keys,
-                                          int64_t n_keys,
                                           const int32_t* __restrict__ table,
                                           int s, int a_start, int64_t toff,
                                           int lg, int lg_max, int64_t bn,
                                           int b, int32_t* status,
                                           OnHit on_hit) {
-  (void)n_keys;
   const int lane = threadIdx.x & 31;
   int S, hits = 0;
   const int P = warp_excl_scan(s, &S);
@@ -362,7 +367,7 @@ __device__ __forceinline__ int flat_probe(const int32_t* __restrict__ keys,
       klg[r] = __shfl_sync(kFull, lg, k);
       tb[r] = table + __shfl_sync(kFull, toff, k);
       own[r] = k;
-      x[r] = act[r] ? __ldg(keys + ka + (f - kp)) : 0;
+      x[r] = act[r] ? Rows::key(keys, ka, f - kp) : 0;
     }
 #pragma unroll
     for (int r = 0; r < kRounds; ++r) {

@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(kOT, 2)
       const int2 e = gi < g1 ? __ldg(ent + gi) : make_int2(0, 0);
       C[lane] = 0;
       __syncwarp();
-      flat_probe<HIER>(elems, m, table, e.y, e.x, desc_toff(dw), desc_lg(dw), lg_max, bn, b,
+      flat_probe<HIER>(elems, table, e.y, e.x, desc_toff(dw), desc_lg(dw), lg_max, bn, b,
                        status, [&](int kk) { atomicAdd(C + kk, 1); });
       __syncwarp();
       if (gi < g1)
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(kOT, 2)
       const int2 e = f < TP ? __ldg(ent + gi) : make_int2(0, 0);
       C[lane] = 0;
       __syncwarp();
-      flat_probe<HIER>(elems, m, table, e.y, e.x, kt, klg, lg_max, bn, b, status,
+      flat_probe<HIER>(elems, table, e.y, e.x, kt, klg, lg_max, bn, b, status,
                        [&](int kk) { atomicAdd(C + kk, 1); });
       __syncwarp();
       if (f < TP) decide<FLOAT_RULE>(__ldg(pidx + gi), C[lane], e.y, kdl, num, den, thr,

@@ -167,7 +167,7 @@ __device__ __forceinline__ int global_batch(
   const bool sw = du4.y > dv.y;
   const int4 A = sw ? dv : du4;
   const int4 B = sw ? du4 : dv;
-  return flat_probe<HIER>(cols, n_cols, table, ok ? A.y : 0, A.x, desc_toff(B),
+  return flat_probe<HIER>(cols, table, ok ? A.y : 0, A.x, desc_toff(B),
                           desc_lg(B), lg_max, bn, b, status, [](int) {});
 }
 
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(kT, 2)
         const int a_start = sw ? dv.x : ksu;
         const int64_t t_off = sw ? kut : desc_toff(dv);
         const int t_lg = sw ? kulg : desc_lg(dv);
-        hits += flat_probe<HIER>(cols, n_cols, table, s, a_start, t_off, t_lg,
+        hits += flat_probe<HIER>(cols, table, s, a_start, t_off, t_lg,
                                  lg_max, bn, b, status, [](int) {});
       }
     }

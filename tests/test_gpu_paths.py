@@ -134,3 +134,73 @@ def test_patterns_with_bit_rows_for_hubs_only(R, cuda, oracle_mod):
             assert R.pattern_count(t, d_off, d_cols, p) == \
                 _oracle_pattern(oracle_mod, off, cols, p), name
     t.check()
+
+
+# ----------------------------------------------------- owner-grouped count --
+
+def _multiset_tc(off, cols):
+    """The reference's count: every key of the shorter row (ties: the edge's
+    source) looked up in the other row's set."""
+    rows = [cols[off[u]:off[u + 1]] for u in range(off.size - 1)]
+    sets = [np.unique(r) for r in rows]
+    total = 0
+    for u, r in enumerate(rows):
+        for v in r:
+            a, b = (v, u) if r.size > rows[v].size else (u, v)
+            total += int(np.isin(rows[a], sets[b]).sum())
+    return total
+
+
+@pytest.mark.parametrize("alpha,bucket", [(0.2, 5), (0.25, 1), (0.9, 2), (1.0, 1)])
+@pytest.mark.parametrize("kind", ["oriented", "symmetric", "repeated", "shuffled"])
+def test_owner_grouped_rows_of_every_kind(R, cuda, oracle_mod, kind, alpha, bucket):
+    """Groups of one to thousands of probers, rows of one chunk and less, rows
+    with repeated keys, tables at the highest load."""
+    off, cols = oracle_mod.rmat_graph(11, 16, 0x5EED7E00, oriented=kind != "symmetric")
+    rng = np.random.default_rng(0x5EED7E00)
+    if kind == "repeated":
+        rows = [np.concatenate([r, r[::3]]) for r in np.split(cols, off[1:-1])]
+        off, cols = csr(rows)
+    if kind == "shuffled":
+        for u in range(off.size - 1):
+            rng.shuffle(cols[off[u]:off[u + 1]])
+    want = _multiset_tc(off, cols)
+    d_off, d_cols = dev(off, cuda), dev(cols, cuda)
+    t = R.Table(d_off, d_cols, alpha=alpha, bucket=bucket, hash_order=True)
+    for c in (d_cols, t.hash_order):
+        for method in (0, 1, 3):
+            assert R.tc_count(t, d_off, c, method=method) == want, method
+    t.check()
+
+
+@pytest.mark.parametrize("d", [7, 8, 9, 255, 256, 257, 2040, 2041, 4095, 4096, 4097, 5000])
+def test_owner_grouped_set_sizes(R, cuda, d):
+    """Complete graphs on the last d of n vertices: sets around a warp's and a
+    CTA's staged table, and past both (probed in HBM)."""
+    n = d + 1
+    deg = np.arange(n - 1, -1, -1, dtype=np.int64)
+    deg[200:max(200, n - 200)] = 0  # the ends of the range are enough
+    off = np.zeros(n + 1, np.int64)
+    off[1:] = np.cumsum(deg)
+    cols = np.concatenate([np.arange(u + 1, n, dtype=np.int32) for u in range(n) if deg[u]])
+    d_off, d_cols = dev(off.astype(np.int32), cuda), dev(cols, cuda)
+    # sum over edges (u, v) of |N(u) n N(v)| = the keys above v, where v has a row
+    u_rows = np.flatnonzero(deg)
+    want = sum(int(deg[v]) * int((u_rows < v).sum()) for v in u_rows)
+    for bucket, alpha in ((5, 0.2), (1, 0.25)):
+        t = R.Table(d_off, d_cols, alpha=alpha, bucket=bucket, hierarchical=bucket == 1)
+        assert R.tc_count(t, d_off, d_cols, method=3) == want
+        t.check()
+        t.free()
+
+
+def test_owner_grouped_classes_and_single_chunk_rows(R, cuda):
+    """2^24 keys and more: rows in class order; long runs of rows of one chunk
+    between long ones (the rings that follow the rows fill with short rows)."""
+    off, cols = R.gen_rmat(21, 10, 0x5EED7E21)
+    assert cols.numel() >= 1 << 24
+    t = R.Table(off, cols, alpha=0.25, bucket=1)
+    want = R.tc_count(t, off, cols, method=1)
+    for _ in range(3):
+        assert R.tc_count(t, off, cols, method=3) == want
+    t.check()
