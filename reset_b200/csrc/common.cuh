@@ -119,6 +119,7 @@ struct reset_table {
   int64_t n_chunks = 0;
   const int32_t* build_off = nullptr;  // CSR offsets the table was built on
   int32_t* d_status = nullptr;   // device error bits
+  void* d_block = nullptr;       // the allocation that holds all but d_table
 };
 
 namespace rst {

@@ -10,11 +10,11 @@
 // of the input and equals the CPU restatement byte for byte.
 //
 // Layout of the work:
-//  * meta:   len[u] = calc_len(deg u), max_len, and the list of "big" sets
+//  * meta:   len[u] = calc_len(deg u), max_len, and the list of "long" sets
 //            whose table does not fit a shared-memory tile.
-//  * scan:   off[u] = sum_{w<u} len[w] (64-bit), off[n] = bucket_num.
-//  * layout: packed 16-byte per-set descriptors for the probe kernels, the
-//            row of every 32-edge chunk, and the first set of every tile.
+//  * layout: off[u] = sum_{w<u} len[w] (64-bit), off[n] = bucket_num; packed
+//            16-byte per-set descriptors for the probe kernels, the row of
+//            every 32-edge chunk, and the first set of every tile.
 //  * tile build: one CTA per tile of ~T consecutive buckets.  The tile's
 //            b slot planes live in shared memory; small sets (deg <= 8) are
 //            inserted by one thread each, larger ones by a warp that
@@ -24,13 +24,15 @@
 //            are then written to HBM with cp.async.bulk (the TMA engine's
 //            1-D bulk copy) -- every table byte is written exactly once and
 //            no separate memset pass runs.
-//  * big build: one CTA per big set, keys inserted straight into HBM.
+//  * long sets: all of them together, key- and bucket-parallel (see
+//            long_insert_kernel), straight in HBM.
 #include <cub/cub.cuh>
 
 #include <cstring>
 #include <mutex>
 
 #include "common.cuh"
+#include "probe_common.cuh"
 
 namespace rst {
 namespace {
@@ -43,8 +45,7 @@ constexpr bool kTileDynamic = true;  // warps take a tile's larger sets from a c
 constexpr int kThreadSetMax = 8;      // sets with deg <= this: thread per set
 constexpr int kTileSmemBudget = 72 * 1024;
 constexpr int kBigFillSmemMax = 64 * 1024;  // buckets whose fill bytes fit smem
-constexpr int kHugeKeys = 1 << 16;  // sets this long get the parallel build
-constexpr int kMaxHuge = 512;       // ... at most this many per table
+constexpr int kHugeKeys = 1 << 16;  // crowded sets this long are built by build_huge
 
 struct Geom {
   int R_max;  // buckets per shared-memory tile (stride of a slot plane)
@@ -91,77 +92,139 @@ __device__ __forceinline__ void bulk_wait_all() {
 
 // ------------------------------------------------------------ meta pass --
 
-__global__ void meta_kernel(const int32_t* __restrict__ off, int32_t n,
-                            float alpha, int b, int LT,
-                            int32_t* __restrict__ len,
-                            int64_t* __restrict__ len64,
-                            int32_t* __restrict__ info,  // [0]=max_len [1]=big [2]=huge
-                            int32_t* __restrict__ big_list,
-                            int32_t* __restrict__ huge_list,
-                            int32_t* __restrict__ status) {
+// What the host reads back to size the table.
+struct BuildInfo {
+  int32_t max_len;
+  int32_t n_long;   // sets whose table does not fit a tile
+  int32_t n_huge;   // ... of kHugeKeys keys or more
+  int32_t n_crowded;  // ... of those, left to build_huge (after long_insert)
+  unsigned long long long_keys, long_buckets;
+  int64_t bucket_num;
+};
+
+// Sets [bid * per, (bid + 1) * per) of block bid.
+__global__ void __launch_bounds__(kThreads)
+    meta_kernel(const int32_t* __restrict__ off, int32_t n, int64_t per, float alpha, int b,
+                int LT, int32_t* __restrict__ len, int64_t* __restrict__ blk_sum,
+                int32_t* __restrict__ long_list, int64_t long_cap, BuildInfo* __restrict__ info,
+                int32_t* __restrict__ status) {
+  __shared__ int64_t s_sum[kWarps];
+  const int64_t u1 = min((int64_t)n, (blockIdx.x + 1) * per);
   int mx = 0;
-  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n;
-       u += (int64_t)gridDim.x * blockDim.x) {
+  int64_t sum = 0;
+  for (int64_t u = blockIdx.x * per + threadIdx.x; u < u1; u += kThreads) {
     int d = off[u + 1] - off[u];
     if (d < 0) {
       atomicOr(status, kErrTableFull);
       d = 0;
     }
-    int l = calc_len(d, alpha, b);
+    const int l = calc_len(d, alpha, b);
     len[u] = l;
-    len64[u] = l;
+    sum += l;
     mx = max(mx, l);
     if (l > LT) {
-      // sets of kHugeKeys or more keys (up to kMaxHuge of them) get the
-      // parallel build; the rest of the long sets one warp each
-      int slot = d >= kHugeKeys ? atomicAdd(&info[2], 1) : kMaxHuge;
-      if (slot < kMaxHuge)
-        huge_list[slot] = (int32_t)u;
-      else
-        big_list[atomicAdd(&info[1], 1)] = (int32_t)u;
+      const int at = atomicAdd(&info->n_long, 1);
+      if (at < long_cap) long_list[at] = (int32_t)u;
+      if (d >= kHugeKeys) atomicAdd(&info->n_huge, 1);
+      atomicAdd(&info->long_keys, (unsigned long long)d);
+      atomicAdd(&info->long_buckets, (unsigned long long)l);
     }
   }
   mx = __reduce_max_sync(kFull, mx);
-  if ((threadIdx.x & 31) == 0 && mx > 0) atomicMax(&info[0], mx);
+  sum = (int64_t)warp_sum_u64((unsigned long long)sum);
+  if ((threadIdx.x & 31) == 0) {
+    s_sum[threadIdx.x >> 5] = sum;
+    if (mx > 0) atomicMax(&info->max_len, mx);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kWarps; ++w) sum += s_sum[w];
+    blk_sum[blockIdx.x] = sum;
+  }
 }
 
-__global__ void finalize_kernel(const int32_t* __restrict__ len,
-                                int64_t* __restrict__ off64, int32_t n,
-                                int64_t* __restrict__ out_bucket_num) {
-  int64_t bn = n > 0 ? off64[n - 1] + len[n - 1] : 0;
-  off64[n] = bn;
-  *out_bucket_num = bn;
+// v (rows that start in 32-edge chunk c, or the first set of tile c) written
+// to out[c0 .. c1) by every lane of the warp: short runs by their own lane,
+// long ones (a hub's row, a large table) by all lanes.
+__device__ __forceinline__ void fill_runs(int32_t* __restrict__ out, int64_t c0, int64_t c1,
+                                          int32_t v) {
+  const int lane = threadIdx.x & 31;
+  const bool wide = c1 - c0 > 8;
+  if (!wide)
+    for (int64_t c = c0; c < c1; ++c) out[c] = v;
+  for (unsigned m = __ballot_sync(kFull, wide); m; m &= m - 1) {
+    const int k = __ffs(m) - 1;
+    const int64_t a = __shfl_sync(kFull, c0, k), z = __shfl_sync(kFull, c1, k);
+    const int32_t x = __shfl_sync(kFull, v, k);
+    for (int64_t c = a + lane; c < z; c += 32) out[c] = x;
+  }
 }
 
-// Per-set descriptors, 32-edge chunk rows and the first set of every tile.
-__global__ void layout_kernel(const int32_t* __restrict__ off,
-                              const int64_t* __restrict__ off64,
-                              const int32_t* __restrict__ len, int32_t n,
-                              int4* __restrict__ desc,
-                              int32_t* __restrict__ chunk_row,
-                              int32_t* __restrict__ tile_first, int T,
-                              int32_t n_tiles) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    int u = (int)i;
-    int s = off[u], e = off[u + 1];
-    if (chunk_row)
-      for (int64_t c = ((int64_t)s + 31) >> 5; c * 32 < e; ++c)
-        chunk_row[c] = u;
-    if (!off64) continue;
-    int64_t toff = off64[u];
-    int lg = 31 - __clz(len[u]);
-    if (desc)
+// The row of every 32-edge chunk of a CSR.
+__global__ void __launch_bounds__(kThreads)
+    chunk_rows_kernel(const int32_t* __restrict__ off, int32_t n, int64_t n_chunks,
+                      int32_t* __restrict__ chunk_row) {
+  for (int64_t base = (int64_t)blockIdx.x * kThreads; base < n;
+       base += (int64_t)gridDim.x * kThreads) {
+    const int64_t u = base + threadIdx.x;
+    const bool in = u < n;
+    const int s = in ? off[u] : 0, e = in ? off[u + 1] : 0;
+    fill_runs(chunk_row, ((int64_t)s + 31) >> 5, in ? min(((int64_t)e + 31) >> 5, n_chunks) : 0,
+              (int32_t)u);
+  }
+}
+
+// Offsets, descriptors, chunk rows and the first set of every tile, over
+// meta_kernel's blocks of sets.
+__global__ void __launch_bounds__(kThreads)
+    layout_kernel(const int32_t* __restrict__ off, const int32_t* __restrict__ len, int32_t n,
+                  int64_t per, const int64_t* __restrict__ blk_sum, int64_t* __restrict__ off64,
+                  int4* __restrict__ desc, int64_t n_chunks, int32_t* __restrict__ chunk_row,
+                  int32_t* __restrict__ tile_first, int64_t tile_cap, int T,
+                  BuildInfo* __restrict__ info) {
+  using Reduce = cub::BlockReduce<int64_t, kThreads>;
+  using Scan = cub::BlockScan<int64_t, kThreads>;
+  __shared__ union {
+    typename Reduce::TempStorage reduce;
+    typename Scan::TempStorage scan;
+  } tmp;
+  __shared__ int64_t s_carry;
+  int64_t part = 0;
+  for (int i = threadIdx.x; i < (int)blockIdx.x; i += kThreads) part += blk_sum[i];
+  part = Reduce(tmp.reduce).Sum(part);
+  if (threadIdx.x == 0) s_carry = part;
+  __syncthreads();
+  int64_t carry = s_carry;
+  const int64_t u1 = min((int64_t)n, (blockIdx.x + 1) * per);
+  for (int64_t base = blockIdx.x * per; base < u1; base += kThreads) {
+    const int64_t u = base + threadIdx.x;
+    const bool in = u < u1;
+    const int l = in ? len[u] : 0;
+    int64_t toff, total;
+    __syncthreads();  // tmp is used again
+    Scan(tmp.scan).ExclusiveSum((int64_t)l, toff, total);
+    toff += carry;
+    carry += total;
+    const int s = in ? off[u] : 0, e = in ? off[u + 1] : 0;
+    if (in) {
+      const int lg = 31 - __clz(l);
+      off64[u] = toff;
       desc[u] = make_int4(s, e - s, (int)(uint32_t)toff,
                           (int)(((toff >> 32) & 0xFFFFFF) | ((int64_t)lg << 24)));
-    if (tile_first) {
-      // tiles whose first set is u: (tile(off64[u-1]), tile(off64[u])]
-      int64_t cu = toff / T;
-      int64_t cp = u > 0 ? off64[u - 1] / T : -1;
-      for (int64_t c = cp + 1; c <= cu && c < n_tiles; ++c) tile_first[c] = u;
-      if (u == n - 1)
-        for (int64_t c = cu + 1; c <= n_tiles; ++c) tile_first[c] = n;
+      if (u == n - 1) {
+        off64[n] = toff + l;
+        info->bucket_num = toff + l;
+        const int64_t end = (toff + l + T - 1) / T;
+        if (end < tile_cap) tile_first[end] = n;
+      }
     }
+    fill_runs(chunk_row, ((int64_t)s + 31) >> 5, in ? min(((int64_t)e + 31) >> 5, n_chunks) : 0,
+              (int32_t)u);
+    // tile c's first set is the first one at or after bucket c * T: the one
+    // after the set that bucket c * T lies in, beyond its first bucket
+    fill_runs(tile_first, in ? toff / T + 1 : 0, in ? min((toff + l) / T + 1, tile_cap) : 0,
+              (int32_t)u + 1);
+    if (in && u == 0) tile_first[0] = 0;
   }
 }
 
@@ -426,31 +489,45 @@ __global__ void __launch_bounds__(kTileThreads)
     // are consecutive in the tile and their rows consecutive in the CSR, so
     // the rows in bucket order are the tile's non-empty slots in (bucket,
     // slot) order, compacted into hash_out[off[u] .. off[r]): each warp
-    // counts a contiguous span of slots, then writes its keys after the
-    // spans before it.
+    // counts a contiguous span of buckets, then writes its keys after the
+    // spans before it.  A lane takes a bucket, not a slot: with 5 slots to a
+    // bucket most are empty (R-MAT scale 22, build with rows: 3.24 -> 2.33 ms).
     if (hash_out) {
-      const int total = R * b;
-      const int span = (((total + kTileWarps - 1) / kTileWarps) + 31) & ~31;
-      const int i_lo = min(total, warp * span), i_hi = min(total, i_lo + span);
-      auto slot = [&](int i) {
-        return b == 1 ? S[i] : S[(i % b) * R_max + i / b];
+      const int span = (((R + kTileWarps - 1) / kTileWarps) + 31) & ~31;
+      const int h_lo = min(R, warp * span), h_hi = min(R, h_lo + span);
+      auto keys_of = [&](int h) {  // a bucket's keys (its slots fill in order)
+        int f = 0;
+        if (h < h_hi)
+          while (f < b && S[f * R_max + h] != -1) ++f;
+        return f;
       };
       int c = 0;
-      for (int i0 = i_lo; i0 < i_hi; i0 += 32) {
-        const int i = i0 + lane;
-        c += __popc(__ballot_sync(kFull, i < i_hi && slot(i) != -1));
-      }
+      for (int h = h_lo + lane; h < h_hi; h += 32) c += b == 1 ? S[h] != -1 : keys_of(h);
+      c = __reduce_add_sync(kFull, c);
       if (lane == 0) s_span[warp] = c;
       __syncthreads();
       int w = off[u];
       for (int k = 0; k < warp; ++k) w += s_span[k];
       const unsigned lt = lanemask_lt();
-      for (int i0 = i_lo; i0 < i_hi; i0 += 32) {
-        const int i = i0 + lane;
-        const int v = i < i_hi ? slot(i) : -1;
-        const unsigned msk = __ballot_sync(kFull, v != -1);
-        if (v != -1) hash_out[w + __popc(msk & lt)] = v;
-        w += __popc(msk);
+      if (b == 1) {
+        for (int h0 = h_lo; h0 < h_hi; h0 += 32) {
+          const int h = h0 + lane, v = h < h_hi ? S[h] : -1;
+          const unsigned m = __ballot_sync(kFull, v != -1);
+          if (v != -1) hash_out[w + __popc(m & lt)] = v;
+          w += __popc(m);
+        }
+      } else for (int h0 = h_lo; h0 < h_hi; h0 += 32) {
+        const int h = h0 + lane, f = keys_of(h);
+        // keys before this bucket's: at most b ballots, usually one or two
+        int before = 0, all = 0;
+        for (int k = 0; k < b; ++k) {
+          const unsigned m = __ballot_sync(kFull, f > k);
+          if (!m) break;
+          before += __popc(m & lt);
+          all += __popc(m);
+        }
+        for (int k = 0; k < f; ++k) hash_out[w + before + k] = S[k * R_max + h];
+        w += all;
       }
     }
     if (tid == 0) bulk_wait_read_all();
@@ -460,24 +537,217 @@ __global__ void __launch_bounds__(kTileThreads)
   if (tid == 0) bulk_wait_all();
 }
 
-// ------------------------------------------------------------ big build --
+// ------------------------------------------------------------ long sets --
+//
+// Sets whose table does not fit a tile, all of them together, with exactly
+// the slots of sequential CSR-order insertion.  Which slots are occupied does
+// not depend on the insertion order, only which key lies where, so:
+//  1. long_insert: every key, in parallel, puts its INDEX in the row into the
+//     first free slot at or after its home bucket (a compare-and-swap on the
+//     slots themselves).  The occupied slots are then the final ones.
+//  2. long_fix: a run is a maximal stretch of full buckets and the bucket
+//     after it.  A key never leaves its home's run, so the run's slots hold
+//     exactly the indices of the run's keys: one thread per run sorts them
+//     and replays the sequential rule, writing the keys.
+// Runs are a few buckets long at the loads in use.  A set with a walk of
+// kWalkMax buckets or a run of more than kRunMax keys is "crowded" (a key
+// repeated many times, a full table): one warp inserts it sequentially, or
+// build_huge builds it if it is long.
+// Bound by the latency of the scattered slot accesses.  Index of 2M documents
+// and 100k terms (8M postings, ~100 long sets), build with rows, b = 5 / b = 1:
+// one warp per set, and 20 launches per set of 2^16 keys, 7.9 / 31 ms; all
+// sets together 0.57 / 1.07 ms; 20M documents, 1M terms 36.7 / 59 -> 4.5 / 8.2.
+constexpr int kKeyItem = 2048;     // keys per CTA of long_insert
+constexpr int kBucketItem = 2048;  // buckets per CTA of long_fix / long_rows
+constexpr int kWalkMax = 256;
+constexpr int kRunMax = 96;
+
+struct LongSet {
+  int32_t u, rs, d, lg;
+  int64_t toff;
+  int32_t key_item, bucket_item;  // its first items
+};
+
+// The long sets' descriptors and the prefix sums of their items (one block).
+__global__ void __launch_bounds__(1024)
+    long_plan_kernel(const int32_t* __restrict__ off, const int32_t* __restrict__ len,
+                     const int64_t* __restrict__ off64, const int32_t* __restrict__ list, int n,
+                     LongSet* __restrict__ sets, int32_t* __restrict__ crowded) {
+  using Scan = cub::BlockScan<int, 1024>;
+  __shared__ typename Scan::TempStorage tmp;
+  int keys = 0, buckets = 0;  // items before this round
+  for (int base = 0; base < n; base += 1024) {
+    const int i = base + threadIdx.x;
+    LongSet s{};
+    int ki = 0, bi = 0;
+    if (i < n) {
+      s.u = list[i];
+      s.rs = off[s.u];
+      s.d = off[s.u + 1] - s.rs;
+      const int l = len[s.u];
+      s.lg = 31 - __clz(l);
+      s.toff = off64[s.u];
+      ki = (s.d + kKeyItem - 1) / kKeyItem;
+      bi = (l + kBucketItem - 1) / kBucketItem;
+      crowded[i] = 0;
+    }
+    int total;
+    __syncthreads();
+    Scan(tmp).ExclusiveSum(ki, s.key_item, total);
+    s.key_item += keys;
+    keys += total;
+    __syncthreads();
+    Scan(tmp).ExclusiveSum(bi, s.bucket_item, total);
+    s.bucket_item += buckets;
+    buckets += total;
+    if (i < n) sets[i] = s;
+  }
+  if (threadIdx.x == 0) {
+    LongSet end{};
+    end.key_item = keys;
+    end.bucket_item = buckets;
+    sets[n] = end;
+  }
+}
+
+// The set whose items hold `item` (-1: past the last), found by thread 0.
+template <int32_t LongSet::*FIRST>
+__device__ __forceinline__ int long_set_of(const LongSet* __restrict__ sets, int n, int item) {
+  __shared__ int s_i;
+  if (threadIdx.x == 0) {
+    int lo = 0, hi = n;  // largest i with first item <= item
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (sets[mid].*FIRST <= item) lo = mid; else hi = mid - 1;
+    }
+    s_i = lo < n ? lo : -1;
+  }
+  __syncthreads();
+  return s_i;
+}
+
+__global__ void __launch_bounds__(kThreads)
+    long_clear_kernel(const LongSet* __restrict__ sets, int n, int64_t bucket_num, int b,
+                      int32_t* __restrict__ table) {
+  const int i = long_set_of<&LongSet::bucket_item>(sets, n, blockIdx.x);
+  if (i < 0) return;
+  const LongSet s = sets[i];
+  const int h0 = ((int)blockIdx.x - s.bucket_item) * kBucketItem;
+  const int q = min(kBucketItem, (1 << s.lg) - h0) >> 2;
+  const int4 neg = make_int4(-1, -1, -1, -1);
+  for (int k = 0; k < b; ++k) {
+    int4* P = reinterpret_cast<int4*>(table + s.toff + h0 + (int64_t)k * bucket_num);
+    for (int j = threadIdx.x; j < q; j += kThreads) P[j] = neg;
+  }
+}
 
 template <bool HIER>
 __global__ void __launch_bounds__(kThreads)
-    big_build_kernel(const int32_t* __restrict__ off,
-                     const int32_t* __restrict__ elems,
-                     const int32_t* __restrict__ len,
-                     const int64_t* __restrict__ off64,
-                     const int32_t* __restrict__ big_list, int64_t bucket_num,
-                     int b, int lg_max, int32_t* __restrict__ table,
-                     int32_t* __restrict__ hash_out,
-                     int32_t* __restrict__ status) {
+    long_insert_kernel(const int32_t* __restrict__ elems, const LongSet* __restrict__ sets, int n,
+                       int64_t bucket_num, int b, int lg_max, int32_t* __restrict__ table,
+                       int32_t* __restrict__ crowded) {
+  const int i = long_set_of<&LongSet::key_item>(sets, n, blockIdx.x);
+  if (i < 0) return;
+  const LongSet s = sets[i];
+  const int j0 = ((int)blockIdx.x - s.key_item) * kKeyItem;
+  int32_t* G = table + s.toff;
+  const int lmask = (1 << s.lg) - 1;
+  constexpr int kPer = kKeyItem / kThreads;
+  int h[kPer];
+#pragma unroll
+  for (int r = 0; r < kPer; ++r) {
+    const int j = j0 + r * kThreads + threadIdx.x;
+    h[r] = j < s.d ? home_bucket<HIER>(__ldg(elems + s.rs + j), s.lg, lg_max) : -1;
+  }
+#pragma unroll
+  for (int r = 0; r < kPer; ++r) {
+    if (h[r] < 0) continue;
+    const int j = j0 + r * kThreads + threadIdx.x;
+    int hh = h[r], k = 0, walked = 0;
+    while (atomicCAS(G + hh + (int64_t)k * bucket_num, -1, j) != -1) {
+      if (++k < b) continue;
+      k = 0;
+      hh = (hh + 1) & lmask;
+      if (++walked == kWalkMax || *(volatile int32_t*)(crowded + i)) {
+        crowded[i] = 1;  // (the key is left out: the set is built again)
+        break;
+      }
+    }
+  }
+}
+
+// blk_cnt (optional): occupied slots of every bucket item.
+template <bool HIER>
+__global__ void __launch_bounds__(kThreads)
+    long_fix_kernel(const int32_t* __restrict__ elems, const LongSet* __restrict__ sets, int n,
+                    int64_t bucket_num, int b, int lg_max, int32_t* __restrict__ table,
+                    int32_t* __restrict__ crowded) {
+  const int i = long_set_of<&LongSet::bucket_item>(sets, n, blockIdx.x);
+  if (i < 0) return;
+  const LongSet s = sets[i];
+  if (crowded[i]) return;
+  int32_t* G = table + s.toff;
+  const int lmask = (1 << s.lg) - 1;
+  const int h0 = ((int)blockIdx.x - s.bucket_item) * kBucketItem;
+  const int h1 = min(h0 + kBucketItem, lmask + 1);
+  const int64_t last = (int64_t)(b - 1) * bucket_num;  // a bucket's last slot
+  for (int h = h0 + threadIdx.x; h < h1; h += kThreads) {
+    // an occupied slot holds an index or, once its run is done, a key (>= 0)
+    if (__ldcg(G + h) == -1 || __ldcg(G + ((h - 1) & lmask) + last) != -1) continue;
+    int idx[kRunMax];
+    int t = 0;
+    bool fits = true;
+    for (int e = h;; e = (e + 1) & lmask) {  // the run's indices, in order
+      bool full = true;
+      for (int k = 0; k < b; ++k) {
+        const int v = __ldcg(G + e + (int64_t)k * bucket_num);
+        if (v == -1) {
+          full = false;
+          break;
+        }
+        if (t == kRunMax) {
+          fits = false;
+          break;
+        }
+        int p = t++;
+        for (; p > 0 && idx[p - 1] > v; --p) idx[p] = idx[p - 1];
+        idx[p] = v;
+      }
+      if (!full || !fits) break;
+    }
+    if (!fits) {
+      crowded[i] = 1;
+      continue;
+    }
+    unsigned char fill[kRunMax];  // keys placed per bucket of the run
+    for (int j = 0; j < t; ++j) fill[j] = 0;
+    for (int j = 0; j < t; ++j) {
+      const int x = __ldg(elems + s.rs + idx[j]);
+      int p = (home_bucket<HIER>(x, s.lg, lg_max) - h) & lmask;
+      while (fill[p] == b) ++p;
+      G[((h + p) & lmask) + (int64_t)fill[p] * bucket_num] = x;
+      ++fill[p];
+    }
+  }
+}
+
+// Crowded sets, sequentially, a CTA each (those of kHugeKeys keys or more are
+// listed for build_huge).
+template <bool HIER>
+__global__ void __launch_bounds__(kThreads)
+    long_crowded_kernel(const int32_t* __restrict__ elems, const LongSet* __restrict__ sets,
+                        const int32_t* __restrict__ crowded, int64_t bucket_num, int b, int lg_max,
+                        int32_t* __restrict__ table, LongSet* __restrict__ huge,
+                        BuildInfo* __restrict__ info, int32_t* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char fill[];
-  const int u = big_list[blockIdx.x];
-  const int l = len[u];
-  const int lg = 31 - __clz(l);
-  const int64_t toff = off64[u];
-  int32_t* G = table + toff;
+  if (!crowded[blockIdx.x]) return;
+  const LongSet s = sets[blockIdx.x];
+  if (s.d >= kHugeKeys) {
+    if (threadIdx.x == 0) huge[atomicAdd(&info->n_crowded, 1)] = s;
+    return;
+  }
+  const int l = 1 << s.lg;
+  int32_t* G = table + s.toff;
   const int tid = threadIdx.x;
   {
     const int4 neg = make_int4(-1, -1, -1, -1);
@@ -491,26 +761,73 @@ __global__ void __launch_bounds__(kThreads)
     }
   }
   __syncthreads();
-  const int rs = off[u], d = off[u + 1] - rs;
   if (tid < 32) {
     if (l <= kBigFillSmemMax)
-      insert_set_warp<HIER>(elems + rs, d, lg, lg_max, b,
+      insert_set_warp<HIER>(elems + s.rs, s.d, s.lg, lg_max, b,
                             GlobalSlotsSmemFill{G, bucket_num, fill}, status);
     else
-      insert_set_warp<HIER>(elems + rs, d, lg, lg_max, b,
+      insert_set_warp<HIER>(elems + s.rs, s.d, s.lg, lg_max, b,
                             GlobalSlotsScan{G, bucket_num, b}, status);
   }
+}
+
+// The long sets' rows in bucket order: a set's non-empty slots in (bucket,
+// slot) order, compacted.  long_count: per bucket item, then a scan over all
+// items; long_rows writes.
+__global__ void __launch_bounds__(kThreads)
+    long_count_kernel(const LongSet* __restrict__ sets, int n, int64_t bucket_num, int b,
+                      const int32_t* __restrict__ table, int32_t* __restrict__ blk_cnt) {
+  __shared__ int s_c[kWarps];
+  const int i = long_set_of<&LongSet::bucket_item>(sets, n, blockIdx.x);
+  int c = 0;
+  if (i >= 0) {
+    const LongSet s = sets[i];
+    const int h0 = ((int)blockIdx.x - s.bucket_item) * kBucketItem;
+    const int h1 = min(h0 + kBucketItem, 1 << s.lg);
+    for (int k = 0; k < b; ++k) {
+      const int32_t* P = table + s.toff + (int64_t)k * bucket_num;
+      for (int h = h0 + threadIdx.x; h < h1; h += kThreads) c += P[h] != -1;
+    }
+  }
+  c = __reduce_add_sync(kFull, c);
+  if ((threadIdx.x & 31) == 0) s_c[threadIdx.x >> 5] = c;
   __syncthreads();
-  if (hash_out && tid < 32 && d > 0)
-    extract_set_warp(l, b, hash_out + rs, [&](int bb, int k) {
-      return __ldcg(G + bb + (int64_t)k * bucket_num);
-    });
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kWarps; ++w) c += s_c[w];
+    blk_cnt[blockIdx.x] = c;
+  }
+}
+
+__global__ void __launch_bounds__(kThreads)
+    long_rows_kernel(const LongSet* __restrict__ sets, int n, int64_t bucket_num, int b,
+                     const int32_t* __restrict__ table, const int32_t* __restrict__ blk_off,
+                     int32_t* __restrict__ hash_out) {
+  using Scan = cub::BlockScan<int, kThreads>;
+  __shared__ typename Scan::TempStorage tmp;
+  const int i = long_set_of<&LongSet::bucket_item>(sets, n, blockIdx.x);
+  if (i < 0) return;
+  const LongSet s = sets[i];
+  const int h0 = ((int)blockIdx.x - s.bucket_item) * kBucketItem;
+  const int h1 = min(h0 + kBucketItem, 1 << s.lg);
+  int32_t* out = hash_out + s.rs + (blk_off[blockIdx.x] - blk_off[s.bucket_item]);
+  for (int hb = h0; hb < h1; hb += kThreads) {
+    const int h = hb + threadIdx.x;
+    const int32_t* P = table + s.toff + h;
+    int f = 0;
+    if (h < h1)
+      while (f < b && P[(int64_t)f * bucket_num] != -1) ++f;
+    int at, total;
+    __syncthreads();
+    Scan(tmp).ExclusiveSum(f, at, total);
+    for (int k = 0; k < f; ++k) out[at + k] = P[(int64_t)k * bucket_num];
+    out += total;
+  }
 }
 
 // ----------------------------------------------------------- huge build --
 //
-// One set of d >= kHugeKeys keys, built in parallel with exactly the slots
-// of sequential CSR-order insertion:
+// One set of d >= kHugeKeys keys that long_insert_kernel found too crowded,
+// built in parallel with exactly the slots of sequential CSR-order insertion:
 //  1. home bucket of every key, keys per home bucket (cnt);
 //  2. the final fills: in linear probing they do not depend on the
 //     insertion order -- the keys carried from bucket h to h+1 are
@@ -624,82 +941,6 @@ __global__ void huge_place_kernel(const int32_t* __restrict__ keys,
   }
 }
 
-// A huge set's rows in bucket order: its non-empty slots in (bucket, slot)
-// order, compacted.  Block k covers indices [k*kHugeChunk, (k+1)*kHugeChunk)
-// of the l*b (bucket, slot) pairs, each warp a contiguous span of them.
-constexpr int kHugeChunk = 8192;
-
-__device__ __forceinline__ int32_t huge_slot(const int32_t* G, int64_t bn, int b, int64_t i) {
-  return b == 1 ? G[i] : G[i / b + (i % b) * bn];
-}
-
-__device__ __forceinline__ int huge_warp_count(const int32_t* G, int64_t bn, int b,
-                                               int64_t lo, int64_t hi) {
-  const int lane = threadIdx.x & 31;
-  int c = 0;
-  for (int64_t i0 = lo; i0 < hi; i0 += 32) {
-    const int64_t i = i0 + lane;
-    c += __popc(__ballot_sync(kFull, i < hi && huge_slot(G, bn, b, i) != -1));
-  }
-  return c;
-}
-
-__global__ void __launch_bounds__(kThreads)
-    huge_count_kernel(const int32_t* __restrict__ G, int64_t bn, int b, int64_t total,
-                      int32_t* __restrict__ blk_cnt) {
-  __shared__ int s_c[kWarps];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t base = (int64_t)blockIdx.x * kHugeChunk;
-  const int span = kHugeChunk / kWarps;
-  const int64_t lo = min(total, base + (int64_t)warp * span), hi = min(total, lo + span);
-  const int c = huge_warp_count(G, bn, b, lo, hi);
-  if (lane == 0) s_c[warp] = c;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int t = 0;
-    for (int w = 0; w < kWarps; ++w) t += s_c[w];
-    blk_cnt[blockIdx.x] = t;
-  }
-}
-
-__global__ void __launch_bounds__(kThreads)
-    huge_write_kernel(const int32_t* __restrict__ G, int64_t bn, int b, int64_t total,
-                      const int32_t* __restrict__ blk_off, int32_t* __restrict__ out) {
-  __shared__ int s_c[kWarps];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t base = (int64_t)blockIdx.x * kHugeChunk;
-  const int span = kHugeChunk / kWarps;
-  const int64_t lo = min(total, base + (int64_t)warp * span), hi = min(total, lo + span);
-  const int c = huge_warp_count(G, bn, b, lo, hi);
-  if (lane == 0) s_c[warp] = c;
-  __syncthreads();
-  int64_t w = blk_off[blockIdx.x];
-  for (int k = 0; k < warp; ++k) w += s_c[k];
-  const unsigned lt = lanemask_lt();
-  for (int64_t i0 = lo; i0 < hi; i0 += 32) {
-    const int64_t i = i0 + lane;
-    const int32_t v = i < hi ? huge_slot(G, bn, b, i) : -1;
-    const unsigned msk = __ballot_sync(kFull, v != -1);
-    if (v != -1) out[w + __popc(msk & lt)] = v;
-    w += __popc(msk);
-  }
-}
-
-// (row start, keys, table length, table offset) of each huge set.
-__global__ void huge_info_kernel(const int32_t* __restrict__ off,
-                                 const int32_t* __restrict__ len,
-                                 const int64_t* __restrict__ off64,
-                                 const int32_t* __restrict__ huge_list, int nh,
-                                 int64_t* __restrict__ out) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nh) return;
-  const int u = huge_list[k];
-  out[4 * k + 0] = off[u];
-  out[4 * k + 1] = (int64_t)off[u + 1] - off[u];
-  out[4 * k + 2] = len[u];
-  out[4 * k + 3] = off64[u];
-}
-
 // ------------------------------------------------- standalone extraction --
 
 __global__ void __launch_bounds__(kThreads)
@@ -735,8 +976,8 @@ reset_status make_chunk_rows(const int32_t* d_off, int32_t n, int64_t m,
   RST_CUDA(scratch_malloc(reinterpret_cast<void**>(d_rows_out),
                            sizeof(int32_t) * (nc > 0 ? nc : 1), st));
   RST_CUDA(cudaMemsetAsync(*d_rows_out, 0, sizeof(int32_t) * (nc > 0 ? nc : 1), st));
-  note_launch(); layout_kernel<<<grid_for(n, 256), 256, 0, st>>>(
-      d_off, nullptr, nullptr, n, nullptr, *d_rows_out, nullptr, 1, 0);
+  note_launch(); chunk_rows_kernel<<<grid_for(n, kThreads), kThreads, 0, st>>>(d_off, n, nc,
+                                                                             *d_rows_out);
   RST_CUDA(cudaGetLastError());
   return RESET_OK;
 }
@@ -818,10 +1059,8 @@ namespace {
 void destroy(reset_table* t) {
   if (!t) return;
   // stream-ordered frees into the table pool (callers synchronise first)
-  void* ptrs[] = {t->d_table, t->d_len, t->d_off64, t->d_desc, t->d_chunk_row,
-                  t->d_status};
-  for (void* p : ptrs)
-    if (p) cudaFreeAsync(p, 0);
+  if (t->d_table) cudaFreeAsync(t->d_table, 0);
+  if (t->d_block) cudaFreeAsync(t->d_block, 0);
   delete t;
 }
 
@@ -830,7 +1069,7 @@ void destroy(reset_table* t) {
 // from the table pool, stream-ordered; no host synchronisation.
 template <bool HIER>
 reset_status build_huge(const reset_table* t, const int32_t* d_elems, int64_t rs, int64_t d,
-                        int64_t l, int64_t toff, int32_t* d_hash_out, cudaStream_t st) {
+                        int64_t l, int64_t toff, cudaStream_t st) {
   const int b = t->bucket;
   const int64_t bn = t->bucket_num;
   const int lg = 63 - __builtin_clzll((unsigned long long)l);
@@ -839,11 +1078,9 @@ reset_status build_huge(const reset_table* t, const int32_t* d_elems, int64_t rs
     RST_CUDA(cudaMemsetAsync(G + (int64_t)k * bn, 0xFF, sizeof(int32_t) * (size_t)l, st));
   if (d <= 0) return RESET_OK;
   const int di = (int)d, li = (int)l;
-  const int64_t total = l * b;
-  const int64_t nblk = (total + kHugeChunk - 1) / kHugeChunk;
   const int32_t* keys = d_elems + rs;
   // CUB temporary sizes
-  size_t tb[6] = {0, 0, 0, 0, 0, 0};
+  size_t tb[5] = {0, 0, 0, 0, 0};
   CarryFn* nf = nullptr;
   int32_t* ni = nullptr;
   RST_CUDA(cub::DeviceScan::InclusiveScan(nullptr, tb[0], nf, nf, ComposeCarry(), li, st));
@@ -852,14 +1089,12 @@ reset_status build_huge(const reset_table* t, const int32_t* d_elems, int64_t rs
                                            std::max(lg, 1), st));
   RST_CUDA(cub::DeviceRunLengthEncode::Encode(nullptr, tb[3], ni, ni, ni, ni, di, st));
   RST_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb[4], ni, ni, di, st));
-  RST_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb[5], ni, ni, (int)nblk, st));
   size_t tmp = 0;
   for (size_t x : tb) tmp = std::max(tmp, x);
   // one scratch block: 8 arrays of d ints, 5 of l ints, l carry functions
   auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
   const size_t sd = al(4 * (size_t)d), sl = al(4 * (size_t)l);
-  const size_t bytes = 8 * sd + 5 * sl + al(sizeof(CarryFn) * (size_t)l) +
-                       2 * al(4 * (size_t)(nblk + 1)) + al(16) + al(tmp);
+  const size_t bytes = 8 * sd + 5 * sl + al(sizeof(CarryFn) * (size_t)l) + al(16) + al(tmp);
   char* base = nullptr;
   RST_CUDA(scratch_malloc(reinterpret_cast<void**>(&base), bytes, st));
   char* q = base;
@@ -882,8 +1117,6 @@ reset_status build_huge(const reset_table* t, const int32_t* d_elems, int64_t rs
   int32_t* fill = reinterpret_cast<int32_t*>(carve(sl));
   int32_t* nxt = reinterpret_cast<int32_t*>(carve(sl));
   CarryFn* fn = reinterpret_cast<CarryFn*>(carve(al(sizeof(CarryFn) * (size_t)l)));
-  int32_t* blk = reinterpret_cast<int32_t*>(carve(al(4 * (size_t)(nblk + 1))));
-  int32_t* blk_off = reinterpret_cast<int32_t*>(carve(al(4 * (size_t)(nblk + 1))));
   int32_t* n_runs = reinterpret_cast<int32_t*>(carve(al(16)));
   void* ctmp = carve(al(tmp));
 
@@ -916,16 +1149,6 @@ reset_status build_huge(const reset_table* t, const int32_t* d_elems, int64_t rs
     huge_place_kernel<<<grid_for(d, kThreads), kThreads, 0, st>>>(
         keys, home, idx_s, run_len, run_off, n_runs, l, b, bn, fill, nxt, G, t->d_status);
     RST_CUDA(cudaGetLastError());
-    if (d_hash_out) {
-      note_launch();
-      huge_count_kernel<<<(unsigned)nblk, kThreads, 0, st>>>(G, bn, b, total, blk);
-      x = tmp;
-      RST_CUDA(cub::DeviceScan::ExclusiveSum(ctmp, x, blk, blk_off, (int)nblk, st));
-      note_launch();
-      huge_write_kernel<<<(unsigned)nblk, kThreads, 0, st>>>(G, bn, b, total, blk_off,
-                                                             d_hash_out + rs);
-      RST_CUDA(cudaGetLastError());
-    }
     return RESET_OK;
   };
   rs_out = run();
@@ -934,10 +1157,10 @@ reset_status build_huge(const reset_table* t, const int32_t* d_elems, int64_t rs
 }
 
 template <bool HIER>
-reset_status launch_builds(const reset_table* t, const int32_t* d_off,
-                           const int32_t* d_elems, const int32_t* d_tile_first,
-                           int32_t n_tiles, const int32_t* d_big, int32_t n_big,
-                           const Geom& g, int32_t* d_hash_out, cudaStream_t st) {
+reset_status launch_builds(const reset_table* t, const int32_t* d_off, const int32_t* d_elems,
+                           const int32_t* d_tile_first, int32_t n_tiles, const Geom& g,
+                           const int32_t* d_long, BuildInfo* d_info, const BuildInfo& info,
+                           int32_t* d_hash_out, cudaStream_t st) {
   if (n_tiles > 0) {
     RST_CUDA(cudaFuncSetAttribute(tile_build_kernel<HIER>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -948,17 +1171,69 @@ reset_status launch_builds(const reset_table* t, const int32_t* d_off,
         t->d_status);
     RST_CUDA(cudaGetLastError());
   }
-  if (n_big > 0) {
-    size_t sm = kBigFillSmemMax;
-    RST_CUDA(cudaFuncSetAttribute(big_build_kernel<HIER>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sm));
-    note_launch(); big_build_kernel<HIER><<<n_big, kThreads, sm, st>>>(
-        d_off, d_elems, t->d_len, t->d_off64, d_big, t->bucket_num, t->bucket,
-        t->lg_max, t->d_table, d_hash_out, t->d_status);
+  if (info.n_long == 0) return RESET_OK;
+  // at most one partly filled item per set
+  const int n = info.n_long, b = t->bucket;
+  const int64_t bn = t->bucket_num;
+  const int64_t key_items = (int64_t)(info.long_keys / kKeyItem) + n;
+  const int64_t bucket_items = (int64_t)(info.long_buckets / kBucketItem) + n;
+  if (bucket_items > INT32_MAX) return arg_fail("too many buckets in long sets");
+  size_t scan_bytes = 0;
+  if (d_hash_out)
+    RST_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (int32_t*)nullptr,
+                                           (int32_t*)nullptr, (int)bucket_items, st));
+  auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
+  const size_t sz_sets = al(sizeof(LongSet) * ((size_t)n + 1)), sz_flag = al(4 * (size_t)n);
+  const size_t sz_blk = d_hash_out ? al(4 * (size_t)bucket_items) : 0;
+  char* base = nullptr;
+  RST_CUDA(scratch_malloc(reinterpret_cast<void**>(&base),
+                          2 * sz_sets + sz_flag + 2 * sz_blk + al(scan_bytes), st));
+  LongSet* sets = reinterpret_cast<LongSet*>(base);
+  LongSet* huge = reinterpret_cast<LongSet*>(base + sz_sets);
+  int32_t* crowded = reinterpret_cast<int32_t*>(base + 2 * sz_sets);
+  int32_t* blk = reinterpret_cast<int32_t*>(base + 2 * sz_sets + sz_flag);
+  int32_t* blk_off = reinterpret_cast<int32_t*>(base + 2 * sz_sets + sz_flag + sz_blk);
+  void* scan_tmp = base + 2 * sz_sets + sz_flag + 2 * sz_blk;
+  auto run = [&]() -> reset_status {
+    const int fill_smem = kBigFillSmemMax;
+    RST_CUDA(cudaFuncSetAttribute(long_crowded_kernel<HIER>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, fill_smem));
+    note_launch(5);
+    long_plan_kernel<<<1, 1024, 0, st>>>(d_off, t->d_len, t->d_off64, d_long, n, sets, crowded);
+    long_clear_kernel<<<(unsigned)bucket_items, kThreads, 0, st>>>(sets, n, bn, b, t->d_table);
+    long_insert_kernel<HIER><<<(unsigned)key_items, kThreads, 0, st>>>(
+        d_elems, sets, n, bn, b, t->lg_max, t->d_table, crowded);
+    long_fix_kernel<HIER><<<(unsigned)bucket_items, kThreads, 0, st>>>(
+        d_elems, sets, n, bn, b, t->lg_max, t->d_table, crowded);
+    long_crowded_kernel<HIER><<<n, kThreads, fill_smem, st>>>(
+        d_elems, sets, crowded, bn, b, t->lg_max, t->d_table, huge, d_info, t->d_status);
     RST_CUDA(cudaGetLastError());
-  }
-  return RESET_OK;
+    if (info.n_huge > 0) {  // one more sync, only for tables that have such sets
+      int32_t nc = 0;
+      RST_CUDA(cudaMemcpyAsync(&nc, &d_info->n_crowded, sizeof(nc), cudaMemcpyDeviceToHost, st));
+      RST_CUDA(cudaStreamSynchronize(st));
+      for (int i = 0; i < nc; ++i) {
+        LongSet s;
+        RST_CUDA(cudaMemcpyAsync(&s, huge + i, sizeof(s), cudaMemcpyDeviceToHost, st));
+        RST_CUDA(cudaStreamSynchronize(st));
+        RST_CHECK(build_huge<HIER>(t, d_elems, s.rs, s.d, (int64_t)1 << s.lg, s.toff, st));
+      }
+    }
+    if (d_hash_out) {
+      note_launch(2);
+      long_count_kernel<<<(unsigned)bucket_items, kThreads, 0, st>>>(sets, n, bn, b, t->d_table,
+                                                                     blk);
+      size_t x = scan_bytes;
+      RST_CUDA(cub::DeviceScan::ExclusiveSum(scan_tmp, x, blk, blk_off, (int)bucket_items, st));
+      long_rows_kernel<<<(unsigned)bucket_items, kThreads, 0, st>>>(sets, n, bn, b, t->d_table,
+                                                                    blk_off, d_hash_out);
+      RST_CUDA(cudaGetLastError());
+    }
+    return RESET_OK;
+  };
+  const reset_status rs = run();
+  cudaFreeAsync(base, st);
+  return rs;
 }
 
 }  // namespace
@@ -993,23 +1268,10 @@ reset_status reset_table_build(const int32_t* d_off, const int32_t* d_elems,
   t->build_off = d_off;
   cudaGetDevice(&t->device);
 
-  int32_t* d_info = nullptr;
-  int32_t* d_big = nullptr;
-  int32_t* d_huge = nullptr;
-  int64_t* d_huge_info = nullptr;
-  int32_t* d_tile_first = nullptr;
-  int64_t* d_bn = nullptr;
-  void* d_tmp = nullptr;
-  reset_status rs = RESET_OK;
+  char* scratch = nullptr;
   auto fail = [&](reset_status s) {
     cudaStreamSynchronize(st);
-    if (d_info) cudaFreeAsync(d_info, st);
-    if (d_big) cudaFreeAsync(d_big, st);
-    if (d_huge) cudaFreeAsync(d_huge, st);
-    if (d_huge_info) cudaFreeAsync(d_huge_info, st);
-    if (d_tile_first) cudaFreeAsync(d_tile_first, st);
-    if (d_bn) cudaFreeAsync(d_bn, st);
-    if (d_tmp) cudaFreeAsync(d_tmp, st);
+    if (scratch) cudaFreeAsync(scratch, st);
     cudaStreamSynchronize(st);
     destroy(t);
     return s;
@@ -1020,97 +1282,86 @@ reset_status reset_table_build(const int32_t* d_off, const int32_t* d_elems,
     if (_e != cudaSuccess) return fail(cuda_fail(_e, #call, __FILE__, __LINE__)); \
   } while (0)
 
-  cudaMemPool_t pool;
-  {
-    reset_status ps = table_pool(&pool);
-    if (ps != RESET_OK) return fail(ps);
-  }
-#define POOL_ALLOC(ptr, bytes) \
-  BUILD_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&(ptr)), (bytes), pool, st))
-  POOL_ALLOC(t->d_status, sizeof(int32_t));
-  BUILD_CUDA(cudaMemsetAsync(t->d_status, 0, sizeof(int32_t), st));
-  POOL_ALLOC(t->d_len, sizeof(int32_t) * (n > 0 ? n : 1));
-  POOL_ALLOC(t->d_off64, sizeof(int64_t) * (n + 1));
-  POOL_ALLOC(d_info, sizeof(int32_t) * 4);
-  POOL_ALLOC(d_bn, sizeof(int64_t));
-  BUILD_CUDA(cudaMemsetAsync(d_info, 0, sizeof(int32_t) * 4, st));
-  POOL_ALLOC(d_big, sizeof(int32_t) * (n > 0 ? n : 1));
-  POOL_ALLOC(d_huge, sizeof(int32_t) * kMaxHuge);
+  // what the table keeps but its slots, in one allocation
+  auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
+  const size_t n1 = n > 0 ? n : 1;
+  t->n_chunks = (m + 31) / 32;
+  const size_t sz_len = al(sizeof(int32_t) * n1), sz_off = al(sizeof(int64_t) * ((size_t)n + 1));
+  const size_t sz_desc = al(sizeof(int4) * n1);
+  const size_t sz_rows = al(sizeof(int32_t) * (t->n_chunks > 0 ? t->n_chunks : 1));
+  BUILD_CUDA(scratch_malloc(&t->d_block, 256 + sz_len + sz_off + sz_desc + sz_rows, st));
+  char* q = static_cast<char*>(t->d_block);
+  t->d_status = reinterpret_cast<int32_t*>(q); q += 256;
+  t->d_len = reinterpret_cast<int32_t*>(q); q += sz_len;
+  t->d_off64 = reinterpret_cast<int64_t*>(q); q += sz_off;
+  t->d_desc = reinterpret_cast<int4*>(q); q += sz_desc;
+  t->d_chunk_row = reinterpret_cast<int32_t*>(q);
 
-  if (n > 0) {
-    note_launch(); meta_kernel<<<grid_for(n, 256), 256, 0, st>>>(d_off, n, p.alpha, p.bucket,
-                                                   g.LT, t->d_len, t->d_off64,
-                                                   d_info, d_big, d_huge, t->d_status);
-    BUILD_CUDA(cudaGetLastError());
-    size_t tmp_bytes = 0;
-    BUILD_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, t->d_off64,
-                                             t->d_off64, n, st));
-    POOL_ALLOC(d_tmp, tmp_bytes);
-    BUILD_CUDA(cub::DeviceScan::ExclusiveSum(d_tmp, tmp_bytes, t->d_off64,
-                                             t->d_off64, n, st));
-  }
-  note_launch(); finalize_kernel<<<1, 1, 0, st>>>(t->d_len, t->d_off64, n, d_bn);
-  BUILD_CUDA(cudaGetLastError());
-  int32_t info[4];
-  int64_t bn = 0;
-  BUILD_CUDA(cudaMemcpyAsync(info, d_info, sizeof(info), cudaMemcpyDeviceToHost, st));
-  BUILD_CUDA(cudaMemcpyAsync(&bn, d_bn, sizeof(bn), cudaMemcpyDeviceToHost, st));
-  BUILD_CUDA(cudaStreamSynchronize(st));
-  t->bucket_num = bn;
-  t->max_len = n > 0 ? info[0] : 8;
-  t->lg_max = 31 - __builtin_clz((unsigned)t->max_len);
-  const int32_t n_big = info[1];
-  const int n_huge = std::min(info[2], kMaxHuge);
-  if (bn >= ((int64_t)1 << 56)) return fail(arg_fail("table too large"));
-  // huge sets: their rows and table places on the host (one more sync,
-  // only for tables that have such sets)
-  int64_t huge[4 * kMaxHuge];
-  if (n_huge > 0) {
-    POOL_ALLOC(d_huge_info, sizeof(int64_t) * 4 * kMaxHuge);
-    note_launch(); huge_info_kernel<<<1, kMaxHuge, 0, st>>>(d_off, t->d_len, t->d_off64,
-                                                            d_huge, n_huge, d_huge_info);
-    BUILD_CUDA(cudaGetLastError());
-    BUILD_CUDA(cudaMemcpyAsync(huge, d_huge_info, sizeof(int64_t) * 4 * n_huge,
-                               cudaMemcpyDeviceToHost, st));
+  // scratch: what the host reads back, the blocks' sums, the long sets (each
+  // has LT buckets' keys at the least) and the tiles' first sets (len is at
+  // most 8 or twice the buckets its keys need at the load factor)
+  const int64_t blocks = n > 0 ? std::min<int64_t>((n + 4 * kThreads - 1) / (4 * kThreads),
+                                                   (int64_t)sm_count() * 4) : 0;
+  const int64_t per = blocks > 0 ? (n + blocks - 1) / blocks : 0;
+  const double long_least = std::max(1.0, (double)p.alpha * p.bucket * g.LT * 0.99);
+  int64_t long_cap = std::min<int64_t>(n, (int64_t)((double)m / long_least) + 1);
+  const int64_t bn_cap = 8 * (int64_t)n +
+                         (int64_t)(2.02 * (double)m / ((double)p.alpha * p.bucket)) + 16;
+  int64_t tile_cap = bn_cap / g.T + 3;
+  const size_t sz_sum = al(sizeof(int64_t) * (blocks > 0 ? blocks : 1));
+  BuildInfo info{};
+  BuildInfo* d_info = nullptr;
+  int32_t *d_long = nullptr, *d_tile_first = nullptr;
+  BUILD_CUDA(cudaMemsetAsync(t->d_status, 0, sizeof(int32_t), st));
+  if (n == 0) {
+    BUILD_CUDA(cudaMemsetAsync(t->d_off64, 0, sizeof(int64_t), st));
     BUILD_CUDA(cudaStreamSynchronize(st));
   }
-
-  size_t tbytes = sizeof(int32_t) * (size_t)bn * p.bucket;
-  POOL_ALLOC(t->d_table, tbytes > 0 ? tbytes : 16);
-  POOL_ALLOC(t->d_desc, sizeof(int4) * (n > 0 ? n : 1));
-  t->n_chunks = (m + 31) / 32;
-  POOL_ALLOC(t->d_chunk_row, sizeof(int32_t) * (t->n_chunks > 0 ? t->n_chunks : 1));
+  while (n > 0) {
+    const size_t sz_long = al(sizeof(int32_t) * (size_t)(long_cap > 0 ? long_cap : 1));
+    BUILD_CUDA(scratch_malloc(reinterpret_cast<void**>(&scratch),
+                              256 + sz_sum + sz_long + al(sizeof(int32_t) * (size_t)tile_cap), st));
+    d_info = reinterpret_cast<BuildInfo*>(scratch);
+    int64_t* d_sum = reinterpret_cast<int64_t*>(scratch + 256);
+    d_long = reinterpret_cast<int32_t*>(scratch + 256 + sz_sum);
+    d_tile_first = reinterpret_cast<int32_t*>(scratch + 256 + sz_sum + sz_long);
+    BUILD_CUDA(cudaMemsetAsync(d_info, 0, sizeof(BuildInfo), st));
+    note_launch(2);
+    meta_kernel<<<(int)blocks, kThreads, 0, st>>>(d_off, n, per, p.alpha, p.bucket, g.LT, t->d_len,
+                                                  d_sum, d_long, long_cap, d_info, t->d_status);
+    layout_kernel<<<(int)blocks, kThreads, 0, st>>>(d_off, t->d_len, n, per, d_sum, t->d_off64,
+                                                    t->d_desc, t->n_chunks, t->d_chunk_row,
+                                                    d_tile_first, tile_cap, g.T, d_info);
+    BUILD_CUDA(cudaGetLastError());
+    BUILD_CUDA(cudaMemcpyAsync(&info, d_info, sizeof(info), cudaMemcpyDeviceToHost, st));
+    BUILD_CUDA(cudaStreamSynchronize(st));
+    const int64_t tiles = (info.bucket_num + g.T - 1) / g.T + 1;
+    if (info.n_long <= long_cap && tiles <= tile_cap) break;
+    // offsets that descend (an error that reset_table_check reports) can make
+    // more of them than m keys do: once more, with room for all
+    long_cap = n;
+    tile_cap = tiles;
+    cudaFreeAsync(scratch, st);
+    scratch = nullptr;
+  }
+  const int64_t bn = info.bucket_num;
+  t->bucket_num = bn;
+  t->max_len = n > 0 ? info.max_len : 8;
+  t->lg_max = 31 - __builtin_clz((unsigned)t->max_len);
+  if (bn >= ((int64_t)1 << 56)) return fail(arg_fail("table too large"));
   const int64_t n_tiles64 = (bn + g.T - 1) / g.T;
   if (n_tiles64 > INT32_MAX) return fail(arg_fail("too many tiles"));
-  const int32_t n_tiles = (int32_t)n_tiles64;
-  POOL_ALLOC(d_tile_first, sizeof(int32_t) * (n_tiles + 1));
+  size_t tbytes = sizeof(int32_t) * (size_t)bn * p.bucket;
+  BUILD_CUDA(scratch_malloc(reinterpret_cast<void**>(&t->d_table), tbytes > 0 ? tbytes : 16, st));
   if (n > 0) {
-    note_launch(); layout_kernel<<<grid_for(n, 256), 256, 0, st>>>(
-        d_off, t->d_off64, t->d_len, n, t->d_desc, t->d_chunk_row,
-        d_tile_first, g.T, n_tiles);
-    BUILD_CUDA(cudaGetLastError());
-    if (t->hier)
-      rs = launch_builds<true>(t, d_off, d_elems, d_tile_first, n_tiles, d_big,
-                               n_big, g, d_hash_out, st);
-    else
-      rs = launch_builds<false>(t, d_off, d_elems, d_tile_first, n_tiles,
-                                d_big, n_big, g, d_hash_out, st);
-    if (rs != RESET_OK) return fail(rs);
-    for (int k = 0; k < n_huge && rs == RESET_OK; ++k) {
-      const int64_t* h = huge + 4 * k;
-      rs = t->hier ? build_huge<true>(t, d_elems, h[0], h[1], h[2], h[3], d_hash_out, st)
-                   : build_huge<false>(t, d_elems, h[0], h[1], h[2], h[3], d_hash_out, st);
-    }
+    const reset_status rs =
+        t->hier ? launch_builds<true>(t, d_off, d_elems, d_tile_first, (int32_t)n_tiles64, g,
+                                      d_long, d_info, info, d_hash_out, st)
+                : launch_builds<false>(t, d_off, d_elems, d_tile_first, (int32_t)n_tiles64, g,
+                                       d_long, d_info, info, d_hash_out, st);
     if (rs != RESET_OK) return fail(rs);
   }
-  cudaFreeAsync(d_info, st);
-  cudaFreeAsync(d_big, st);
-  cudaFreeAsync(d_huge, st);
-  if (d_huge_info) cudaFreeAsync(d_huge_info, st);
-  cudaFreeAsync(d_tile_first, st);
-  cudaFreeAsync(d_bn, st);
-  if (d_tmp) cudaFreeAsync(d_tmp, st);
-#undef POOL_ALLOC
+  if (scratch) cudaFreeAsync(scratch, st);
 #undef BUILD_CUDA
   *out = t;
   return RESET_OK;
@@ -1143,10 +1394,8 @@ reset_status reset_table_free(reset_table* t) {
 reset_status reset_table_free_async(reset_table* t, reset_stream_t stream) {
   if (!t) return RESET_OK;
   cudaStream_t st = as_stream(stream);
-  void* ptrs[] = {t->d_table, t->d_len, t->d_off64, t->d_desc, t->d_chunk_row,
-                  t->d_status};
   cudaError_t e = cudaSuccess;
-  for (void* p : ptrs)
+  for (void* p : {static_cast<void*>(t->d_table), t->d_block})
     if (p) {
       cudaError_t e2 = cudaFreeAsync(p, st);
       if (e == cudaSuccess) e = e2;

@@ -204,3 +204,57 @@ def test_owner_grouped_classes_and_single_chunk_rows(R, cuda):
     for _ in range(3):
         assert R.tc_count(t, off, cols, method=3) == want
     t.check()
+
+
+# ------------------------------------------------------------ table build --
+
+def _check_build(R, cuda, oracle_mod, rows, alpha, bucket, hier):
+    off, elems = csr(rows)
+    d_off, d_el = dev(off, cuda), dev(elems, cuda)
+    t = R.Table(d_off, d_el, alpha=alpha, bucket=bucket, hierarchical=hier, hash_order=True)
+    t.check()
+    want = oracle_mod.Table(off, elems, alpha=alpha, bucket=bucket, hier=hier)
+    slots, length, offsets = (x.cpu().numpy() for x in t.tensors())
+    assert np.array_equal(length, want.len) and np.array_equal(offsets, want.off64)
+    assert np.array_equal(slots, want.table)
+    assert np.array_equal(t.hash_order.cpu().numpy(), want.hash_order())
+
+
+@pytest.mark.parametrize("alpha,bucket", [(0.2, 5), (0.25, 1), (1.0, 1), (0.9, 2), (0.3, 16)])
+@pytest.mark.parametrize("hier", [True, False])
+def test_long_sets_runs_and_crowding(R, cuda, oracle_mod, alpha, bucket, hier):
+    """Sets past a tile: lengths around the items of 2048 keys and buckets, a
+    key repeated 95, 96, 97 and 3000 times (runs at and past their limit), keys
+    of the last buckets (a run that wraps), short sets between them."""
+    rng = np.random.default_rng(0x5EED7F00 + bucket)
+    rows = [np.arange(5)]
+    for i, d in enumerate((4095, 4096, 4097, 6143, 9000, 20011)):
+        x = rng.choice(1 << 24, d, replace=False)
+        if i:
+            rep = (95, 96, 97, 3000, 1)[i - 1]
+            x[rng.choice(d, rep, replace=False)] = x[0]
+        x[-40:] = (1 << 24) - 1 - np.arange(40)
+        rows += [x, rng.choice(1 << 24, 3 * i, replace=False), np.zeros(0, np.int64)]
+    _check_build(R, cuda, oracle_mod, rows, alpha, bucket, hier)
+
+
+def test_chunk_rows_of_long_rows(R, cuda, oracle_mod):
+    """Chunk rows and tile starts of rows that span many chunks and tiles
+    (written by a whole warp), beside empty ones."""
+    rng = np.random.default_rng(0x5EED7F77)
+    n = 100000
+    sizes = [0, 1, 33, 0, 0, 300, 50000, 31, 32, 70000, 0, 2]
+    rows = [np.sort(rng.choice(n, d, replace=False)) for d in sizes]
+    rows += [np.zeros(0, np.int64)] * (n - len(rows))
+    rows[n - 1] = np.arange(1, 40)  # edges into the long rows
+    off, cols = csr(rows)
+    want = oracle_mod.tc_merge(off, cols)
+    assert want > 0
+    d_off, d_cols = dev(off, cuda), dev(cols, cuda)
+    for bucket in (1, 5):
+        t = R.Table(d_off, d_cols, bucket=bucket)
+        copy = d_off.clone()  # other offsets: chunk rows found again
+        for o in (d_off, copy):
+            for method in (1, 3):
+                assert R.tc_count(t, o, d_cols, method=method) == want
+        t.check()
