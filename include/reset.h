@@ -366,8 +366,9 @@ reset_status reset_pattern_count(const reset_table *t, const int32_t *d_off,
 reset_status reset_pattern_named(const char *name, reset_pattern *out, int32_t *oriented);
 
 /* |A ∩ B| counted with A's multiplicity for one pair of device arrays
- * (keys >= 0).  Builds B's table with `params` and probes A.  *d_count
- * (device i64) is overwritten.  Replaces make_hashtable_kernel +
+ * (keys >= 0).  `params` is checked as for a table; the count does not depend
+ * on it (B's keys go into a hash set of their own).  Does not synchronise.
+ * *d_count (device i64) is overwritten.  Replaces make_hashtable_kernel +
  * intersection_kernel (set_size/intersection.cu:128-181). */
 reset_status reset_intersect_count(const int32_t *d_a, int64_t na,
                                    const int32_t *d_b, int64_t nb,

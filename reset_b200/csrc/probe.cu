@@ -18,6 +18,7 @@
 // they need; the grid is persistent and walks 32-pair chunks grid-stride.
 #include <cub/cub.cuh>
 
+#include <algorithm>
 #include <climits>
 
 #include "common.cuh"
@@ -110,7 +111,7 @@ __global__ void __launch_bounds__(kThreads, 4)
                const int32_t* __restrict__ elems, int64_t n_elems,
                const int32_t* __restrict__ pa, const int32_t* __restrict__ pb,
                int64_t np, const int64_t* __restrict__ np_dev,
-               unsigned long long* __restrict__ cursor,
+               unsigned long long* __restrict__ cursor, int lg_grab,
                const int32_t* __restrict__ table, int64_t bn, int b,
                int lg_max, int num, int den, float thr, int warp_pair_min,
                uint8_t* __restrict__ flags, int32_t* __restrict__ inter,
@@ -119,7 +120,8 @@ __global__ void __launch_bounds__(kThreads, 4)
   __shared__ int s_qx[kWarps][32 * ROUNDS], s_qh[kWarps][32 * ROUNDS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (np_dev) np = *np_dev;  // pair count set on the device (captured graphs)
-  const int64_t n_chunks = (np + 31) >> 5;
+  const int grab = 1 << lg_grab;  // pairs a warp takes at a time, at most 32
+  const int64_t n_chunks = (np + grab - 1) >> lg_grab;
   const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t it = 0;; ++it) {
@@ -132,8 +134,8 @@ __global__ void __launch_bounds__(kThreads, 4)
       c = gw + it * nw;
     }
     if (c >= n_chunks) break;
-    const int64_t p = c * 32 + lane;
-    const bool valid = p < np;
+    const int64_t p = (c << lg_grab) + lane;
+    const bool valid = lane < grab && p < np;
     int a = valid ? __ldg(pa + p) : 0;
     int q = valid ? __ldg(pb + p) : 0;
     bool ok = valid;
@@ -209,18 +211,85 @@ __global__ void __launch_bounds__(kThreads, 4)
 }
 
 // ----------------------------------------------------------- raw pair ----
+//
+// |A ∩ B| with A's multiplicity needs membership in B only, so B goes into a
+// hash set of its own (linear probing, at most half full) and not into the
+// reference's table: the order of insertion does not matter, no size has to
+// be read back, and nothing can fail on the device.  Up to kPairSmem keys of B
+// every CTA builds the set in its shared memory and looks up its share of A:
+// one launch.  Larger sets lie in HBM (L2): one launch to insert, one to look
+// up (at 16384 keys 46 us a call against 73 in every CTA's shared memory).
+// Latency-bound.  A call through Python, us, by a table build / now: 1000 x
+// 1500 keys 140 / 41, 300 x 100000 353 / 58, 2^20 x 2^20 1162 / 79.
+constexpr int kPairThreads = 512;
+constexpr int kPairSmem = 4096;  // keys (a set of up to 64 KB)
+
+struct PairSet {  // 1 << lg slots at S, -1 = empty
+  int32_t* S;
+  int lg;
+  __device__ __forceinline__ unsigned home(int x) const {
+    return ((unsigned)x * 0x9E3779B1u) >> (32 - lg);
+  }
+  __device__ __forceinline__ void insert(int x) const {
+    for (unsigned h = home(x);; h = (h + 1) & ((1u << lg) - 1u)) {
+      const int old = atomicCAS(S + h, -1, x);
+      if (old == -1 || old == x) return;
+    }
+  }
+  __device__ __forceinline__ bool holds(int x) const {
+    for (unsigned h = home(x);; h = (h + 1) & ((1u << lg) - 1u)) {
+      const int s = S[h];
+      if (s == x) return true;
+      if (s == -1) return false;
+    }
+  }
+};
+
+__global__ void __launch_bounds__(kPairThreads)
+    pair_smem_kernel(const int32_t* __restrict__ a, int64_t na, const int32_t* __restrict__ b,
+                     int nb, int lg, unsigned long long* __restrict__ count) {
+  extern __shared__ __align__(16) int32_t pair_sm[];
+  __shared__ unsigned long long s_sum[kPairThreads / 32];
+  const PairSet set{pair_sm, lg};
+  const int tid = threadIdx.x;
+  for (int i = tid; i < (1 << lg) / 4; i += kPairThreads)
+    reinterpret_cast<int4*>(pair_sm)[i] = make_int4(-1, -1, -1, -1);
+  __syncthreads();
+  for (int i = tid; i < nb; i += kPairThreads) set.insert(__ldg(b + i));
+  __syncthreads();
+  unsigned long long hits = 0;
+  const int64_t step = (int64_t)gridDim.x * kPairThreads;
+#pragma unroll 4
+  for (int64_t i = (int64_t)blockIdx.x * kPairThreads + tid; i < na; i += step)
+    hits += set.holds(__ldg(a + i));
+  hits = warp_sum_u64(hits);
+  if ((tid & 31) == 0) s_sum[tid >> 5] = hits;
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 1; w < kPairThreads / 32; ++w) hits += s_sum[w];
+    if (gridDim.x == 1) *count = hits;  // (else zeroed before the launch)
+    else if (hits) atomicAdd(count, hits);
+  }
+}
 
 __global__ void __launch_bounds__(kThreads)
-    pair_probe_kernel(const int32_t* __restrict__ a, int64_t na,
-                      const int32_t* __restrict__ table, int lg, int64_t bn,
-                      int b, unsigned long long* __restrict__ count,
-                      int32_t* __restrict__ status) {
+    pair_insert_kernel(const int32_t* __restrict__ b, int64_t nb, int32_t* __restrict__ slots,
+                       int lg) {
+  const PairSet set{slots, lg};
+  for (int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x; i < nb;
+       i += (int64_t)gridDim.x * kThreads)
+    set.insert(__ldg(b + i));
+}
+
+__global__ void __launch_bounds__(kThreads)
+    pair_lookup_kernel(const int32_t* __restrict__ a, int64_t na, int32_t* __restrict__ slots,
+                       int lg, unsigned long long* __restrict__ count) {
+  const PairSet set{slots, lg};
   unsigned long long hits = 0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < na;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    // set_size/intersection.cu:169: d_hash(key, len) = key & (len-1)
-    hits += probe_key<false>(__ldg(a + i), table, lg, lg, bn, b, status);
-  }
+#pragma unroll 4
+  for (int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x; i < na;
+       i += (int64_t)gridDim.x * kThreads)
+    hits += set.holds(__ldg(a + i));
   hits = warp_sum_u64(hits);
   if ((threadIdx.x & 31) == 0 && hits) atomicAdd(count, hits);
 }
@@ -511,7 +580,7 @@ reset_status sss_launch_persistent(const reset_table* t, const int32_t* elems,
                                  persistent_grid((const void*)sss_kernel<H, false, R, LN, E>)); \
     note_launch();                                                             \
     sss_kernel<H, false, R, LN, E><<<(int)g, kThreads, 0, st>>>(               \
-        t->d_desc, t->n, elems, t->m, pa, pb, capacity, np_dev, cursor,        \
+        t->d_desc, t->n, elems, t->m, pa, pb, capacity, np_dev, cursor, 5,     \
         t->d_table, t->bucket_num, t->bucket, t->lg_max, num, den, 0.f, wpm,   \
         flags, E ? nullptr : inter, t->d_status);                              \
   } while (0)
@@ -667,10 +736,13 @@ static reset_status sss_common(const reset_table* t, const int32_t* d_off,
                      d_flags, d_inter, st);
 #define SSS_LAUNCH(H, F, R, LN, ...)                                         \
   do {                                                                       \
-    const int64_t g = clamp_grid(((np + 31) / 32 + kWarps - 1) / kWarps,     \
-                                 persistent_grid((const void*)sss_kernel<H, F, R, LN, ##__VA_ARGS__>)); \
+    const int most = persistent_grid((const void*)sss_kernel<H, F, R, LN, ##__VA_ARGS__>); \
+    /* 32 pairs at a time, fewer where that leaves warps idle */             \
+    int lg_grab = 5;                                                         \
+    while (lg_grab > 0 && (np >> lg_grab) < (int64_t)most * kWarps) --lg_grab; \
+    const int64_t g = clamp_grid(((np >> lg_grab) + kWarps) / kWarps, most); \
     note_launch(); sss_kernel<H, F, R, LN, ##__VA_ARGS__><<<(int)g, kThreads, 0, st>>>( \
-        ds.desc, t->n, d_elems, t->m, d_pa, d_pb, np, nullptr, nullptr,      \
+        ds.desc, t->n, d_elems, t->m, d_pa, d_pb, np, nullptr, nullptr, lg_grab, \
         t->d_table, t->bucket_num, t->bucket, t->lg_max, num, den, thr,       \
         tun.warp_pair_min, d_flags, d_inter, t->d_status);                    \
   } while (0)
@@ -719,31 +791,55 @@ reset_status reset_intersect_count(const int32_t* d_a, int64_t na,
   if (!d_count) return arg_fail("NULL count");
   if (na < 0 || nb < 0 || nb > INT32_MAX) return arg_fail("sizes out of range");
   if ((na > 0 && !d_a) || (nb > 0 && !d_b)) return arg_fail("NULL set");
+  reset_params p;
+  reset_params_default(&p);
+  if (params) p = *params;
+  if (na > 0 && nb > 0) {  // what a table with these parameters refuses
+    if (!(p.alpha > 0.f && p.alpha <= 1.f)) return arg_fail("alpha must be in (0, 1]");
+    if (p.bucket < 1 || p.bucket > 16) return arg_fail("bucket must be in 1..16");
+    // (lengths of 2^31 buckets wrap around to 8, calculate_length)
+    const float q = (float)nb / p.alpha;
+    if ((q >= 2147483648.f ? INT32_MAX : (int)q) / p.bucket >= (1 << 30) && nb > 8 * p.bucket) {
+      set_error("a set did not fit its table (or a CSR row had negative length)");
+      return RESET_ERR_TABLE_FULL;
+    }
+  }
   cudaStream_t st = as_stream(stream);
+  unsigned long long* count = reinterpret_cast<unsigned long long*>(d_count);
+  int lg = 6;
+  while (((int64_t)1 << lg) < 2 * nb) ++lg;
+  if (na > 0 && nb > 0 && nb <= kPairSmem) {
+    ++lg;  // (at most a quarter full)
+    const int smem = (int)sizeof(int32_t) << lg;
+    RST_CUDA(cudaFuncSetAttribute(pair_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  smem));
+    // a CTA looks up about as many keys as it inserts
+    const int64_t share = std::max<int64_t>(4 * kPairThreads, nb);
+    const int grid = (int)clamp_grid((na + share - 1) / share, sm_count());
+    if (grid > 1) RST_CUDA(cudaMemsetAsync(d_count, 0, sizeof(int64_t), st));
+    note_launch();
+    pair_smem_kernel<<<grid, kPairThreads, smem, st>>>(d_a, na, d_b, (int)nb, lg, count);
+    RST_CUDA(cudaGetLastError());
+    return RESET_OK;
+  }
   RST_CUDA(cudaMemsetAsync(d_count, 0, sizeof(int64_t), st));
   if (na == 0 || nb == 0) return RESET_OK;
-  int32_t* d_offb = nullptr;
-  RST_CUDA(scratch_malloc(reinterpret_cast<void**>(&d_offb), 2 * sizeof(int32_t), st));
-  const int32_t h_offb[2] = {0, (int32_t)nb};
-  RST_CUDA(cudaMemcpyAsync(d_offb, h_offb, sizeof(h_offb), cudaMemcpyHostToDevice, st));
-  reset_table* t = nullptr;
-  reset_status s = reset_table_build(d_offb, d_b, 1, nb, params, 0, nullptr, &t, stream);
-  if (s != RESET_OK) {
-    cudaFreeAsync(d_offb, st);
-    return s;
+  int32_t* slots = nullptr;
+  const size_t bytes = sizeof(int32_t) << lg;
+  RST_CUDA(scratch_malloc(reinterpret_cast<void**>(&slots), bytes, st));
+  cudaError_t e = cudaMemsetAsync(slots, 0xFF, bytes, st);
+  if (e == cudaSuccess) {
+    const int cap = sm_count() * 8;
+    note_launch(2);
+    pair_insert_kernel<<<(int)clamp_grid((nb + kThreads - 1) / kThreads, cap), kThreads, 0, st>>>(
+        d_b, nb, slots, lg);
+    pair_lookup_kernel<<<(int)clamp_grid((na + kThreads - 1) / kThreads, cap), kThreads, 0, st>>>(
+        d_a, na, slots, lg, count);
+    e = cudaGetLastError();
   }
-  const int lg = t->lg_max;
-  const int64_t g = clamp_grid((na + kThreads - 1) / kThreads,
-                               persistent_grid((const void*)pair_probe_kernel));
-  note_launch(); pair_probe_kernel<<<(int)g, kThreads, 0, st>>>(
-      d_a, na, t->d_table, lg, t->bucket_num, t->bucket,
-      reinterpret_cast<unsigned long long*>(d_count), t->d_status);
-  cudaError_t e = cudaGetLastError();
-  reset_status cs = reset_table_check(t, stream);  // synchronises `stream`
-  cudaFree(d_offb);
-  reset_table_free(t);
-  if (e != cudaSuccess) return cuda_fail(e, "pair_probe_kernel", __FILE__, __LINE__);
-  return cs;
+  cudaFreeAsync(slots, st);
+  if (e != cudaSuccess) return cuda_fail(e, "raw pair kernels", __FILE__, __LINE__);
+  return RESET_OK;
 }
 
 reset_status reset_ir(const reset_table* t, const int32_t* d_toff,

@@ -258,3 +258,33 @@ def test_chunk_rows_of_long_rows(R, cuda, oracle_mod):
             for method in (1, 3):
                 assert R.tc_count(t, o, d_cols, method=method) == want
         t.check()
+
+
+# -------------------------------------------------------------- raw pair --
+
+@pytest.mark.parametrize("nb", [0, 1, 2, 31, 33, 511, 4095, 4096, 4097, 8193, 70001])
+@pytest.mark.parametrize("na", [0, 1, 513, 20011])
+def test_raw_pair_sizes(R, cuda, na, nb):
+    """Around the largest set held in shared memory; both unsorted, with
+    repeats; keys at the ends of the range."""
+    rng = np.random.default_rng(na * 7 + nb)
+    hi = max(4, (na + nb) // 2)
+    a = rng.integers(0, hi, na).astype(np.int32)
+    b = rng.integers(0, hi, nb).astype(np.int32)
+    ends = np.array([0, 2**31 - 1, 2**31 - 2, 1 << 30], np.int32)
+    a[: min(na, 4)] = ends[: min(na, 4)]
+    b[max(nb - 3, 0):] = ends[:nb][-3:][: len(b[max(nb - 3, 0):])]
+    assert R.intersect_count(dev(a, cuda), dev(b, cuda)) == int(np.isin(a, b).sum())
+
+
+@pytest.mark.parametrize("pairs", [1, 33, 300, 4800, 40000])
+def test_pairs_per_warp(R, cuda, pairs):
+    """Few pairs are spread over the warps, one to a warp at the fewest."""
+    rng = np.random.default_rng(pairs)
+    rows = [np.sort(rng.choice(900, rng.integers(0, 200), replace=False)) for _ in range(400)]
+    off, cols = csr(rows)
+    t = R.Table(dev(off, cuda), dev(cols, cuda))
+    pa, pb = (rng.integers(0, 400, pairs).astype(np.int32) for _ in range(2))
+    _, inter = R.sss(t, dev(off, cuda), dev(cols, cuda), dev(pa, cuda), dev(pb, cuda), 1, 10)
+    want = [len(np.intersect1d(rows[u], rows[v])) for u, v in zip(pa, pb)]
+    assert inter.cpu().tolist() == want
