@@ -288,3 +288,41 @@ def test_pairs_per_warp(R, cuda, pairs):
     _, inter = R.sss(t, dev(off, cuda), dev(cols, cuda), dev(pa, cuda), dev(pb, cuda), 1, 10)
     want = [len(np.intersect1d(rows[u], rows[v])) for u, v in zip(pa, pb)]
     assert inter.cpu().tolist() == want
+
+
+# -------------------------------------------------------- decisions only --
+
+@pytest.mark.parametrize("num,den", [(1, 20), (1, 2), (7, 10), (19, 20), (1, 1)])
+@pytest.mark.parametrize("kind", ["ascending", "shuffled", "repeated"])
+def test_decisions_only_like_full(R, cuda, kind, num, den):
+    """Runs of pairs of every length with the same first set, sets of up to
+    more keys than the run's bitmap takes, equal, near and unlike ones, against
+    the decisions of full intersections."""
+    rng = np.random.default_rng(num * 31 + den)
+    rows = []
+    for size in [0, 1, 2, 7, 8, 31, 33, 100, 257, 1000, 4096, 4097, 5000]:
+        base = np.sort(rng.choice(20000, size, replace=False))
+        rows.append(base)
+        for keep in [1.0, 0.97, 0.8, 0.6, 0.1]:
+            r = base[rng.random(size) < keep]
+            rows.append(np.unique(np.concatenate([r, rng.choice(20000, size - len(r))])))
+    if kind == "shuffled":
+        rows = [rng.permutation(r) for r in rows]
+    if kind == "repeated":
+        rows = [np.sort(np.concatenate([r, r[: len(r) // 3]])) if i % 3 else r
+                for i, r in enumerate(rows)]
+    n = len(rows)
+    pa, pb = [], []
+    for u in range(n):  # runs of 1, 2, 3, ... and all of them
+        for v in [*rng.integers(0, n, u % 37), *range(u - u % 6, u + 6 - u % 6)]:
+            pa.append(u)
+            pb.append(v)
+    off, cols = csr(rows)
+    d_off, d_cols = dev(off, cuda), dev(cols, cuda)
+    t = R.Table(d_off, d_cols)
+    pa, pb = dev(np.array(pa, np.int32), cuda), dev(np.array(pb, np.int32), cuda)
+    for x, y in [(pa, pb), (pb, pa)]:
+        full, _ = R.sss(t, d_off, d_cols, x, y, num, den)
+        dec, none = R.sss(t, d_off, d_cols, x, y, num, den, with_inter=False)
+        assert none is None and 0 < int(full.sum()) < full.numel()
+        assert cuda.equal(full, dec)
