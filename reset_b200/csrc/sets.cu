@@ -16,7 +16,10 @@
 // pairs (a < b), sorted.
 #include <cub/cub.cuh>
 
+#include <algorithm>
+#include <climits>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -149,7 +152,6 @@ __global__ void split_keys_kernel(const uint64_t* __restrict__ keys, int64_t m,
 // ---- prefix filtering -----------------------------------------------------
 
 constexpr int kFreqBits = 19;
-constexpr int kSizeBits = 15;
 
 __global__ void token_freq_kernel(const int32_t* __restrict__ tokens, int64_t m,
                                   int32_t* __restrict__ freq) {
@@ -158,67 +160,166 @@ __global__ void token_freq_kernel(const int32_t* __restrict__ tokens, int64_t m,
     atomicAdd(&freq[tokens[j]], 1);
 }
 
-// (set | min(freq, cap) | token): sorting it orders each set's tokens by
-// (frequency, id) -- one global order, the same for every set.
-__global__ void canon_keys_kernel(const int32_t* __restrict__ off, int32_t n,
-                                  const int32_t* __restrict__ tokens,
-                                  const int32_t* __restrict__ freq, int ulog,
-                                  uint64_t* __restrict__ keys) {
-  const int cap = (1 << kFreqBits) - 1;
-  for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < n;
-       i += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-    const int lane = threadIdx.x & 31;
-    for (int j = off[i] + lane; j < off[i + 1]; j += 32) {
-      const int t = tokens[j];
-      const uint64_t f = (uint64_t)min(freq[t], cap);
-      keys[j] = ((uint64_t)i << (kFreqBits + ulog)) | (f << ulog) | (uint64_t)t;
-    }
-  }
-}
-
+// Prefix lengths, and the largest set.
 __global__ void prefix_len_kernel(const int32_t* __restrict__ off, int32_t n,
-                                  int num, int den, int64_t* __restrict__ plen) {
+                                  int num, int den, int64_t* __restrict__ plen,
+                                  int64_t* __restrict__ largest) {
+  int mx = 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t sz = off[i + 1] - off[i];
     // |x| - ceil(t|x|) + 1, t = num/den; empty sets have no prefix
     const int64_t need = (num * sz + den - 1) / den;
     plen[i] = sz > 0 ? sz - need + 1 : 0;
+    mx = max(mx, (int)sz);
   }
+  mx = __reduce_max_sync(kFull, mx);
+  if ((threadIdx.x & 31) == 0)
+    atomicMax(reinterpret_cast<unsigned long long*>(largest), (unsigned long long)mx);
 }
 
-// Prefix entries (token | size | set) of every set.
-__global__ void prefix_entries_kernel(const int32_t* __restrict__ off, int32_t n,
-                                      const uint64_t* __restrict__ canon,
-                                      const int64_t* __restrict__ pre_off, int ulog,
-                                      uint64_t* __restrict__ entries) {
-  const uint64_t tmask = (1ull << ulog) - 1;
+// The p-th smallest (frequency, token) of a set of n keys read by a warp
+// through each(f): f(frequency, token) for every key of this lane.  Found by
+// bits, the frequency's first: a count of the set's keys per bit, in
+// registers, where sorting all sets' keys took eight radix passes over the
+// collection, 128 B of HBM per key.  *equal: how many keys equal to it belong
+// to the p smallest.  Bound by instructions; 50 M tokens in 400,000 sets:
+// 5.0 ms for keys and sort, 1.44 this way.
+template <class Each>
+__device__ __forceinline__ void select_key(int p, int fbits, int ulog, Each each, int* f_out,
+                                           int* t_out, int* equal) {
+  auto count = [&](auto test) {
+    int c = 0;
+    each([&](int f, int t) { c += test(f, t); });
+    return __reduce_add_sync(kFull, c);
+  };
+  int F = 0;  // largest value with fewer than p keys below it
+  for (int bit = fbits - 1; bit >= 0; --bit) {
+    const int cand = F | 1 << bit;
+    if (count([&](int f, int) { return f < cand; }) < p) F = cand;
+  }
+  p -= count([&](int f, int) { return f < F; });
+  *f_out = F;
+  *t_out = INT_MAX;
+  *equal = p;
+  if (count([&](int f, int) { return f == F; }) == p) return;  // all of that frequency
+  int T = 0;
+  for (int bit = ulog - 1; bit >= 0; --bit) {
+    const int cand = T | 1 << bit;
+    if (count([&](int f, int t) { return f == F && t < cand; }) < p) T = cand;
+  }
+  *equal = p - count([&](int f, int t) { return f == F && t < T; });
+  *t_out = T;
+}
+
+// Entries (token | size | set) of every set's prefix: its p smallest tokens by
+// (min(frequency, cap), token) -- one global order, the same for every set --
+// in no particular order.  A warp per set; fbuf (m ints) holds the
+// frequencies of sets too large for registers.
+__global__ void __launch_bounds__(256)
+    prefix_entries_kernel(const int32_t* __restrict__ off, int32_t n,
+                          const int32_t* __restrict__ tokens, const int32_t* __restrict__ freq,
+                          const int64_t* __restrict__ pre_off, int ulog, int size_bits,
+                          int32_t* __restrict__ fbuf, uint64_t* __restrict__ entries) {
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = lanemask_lt();
+  const int cap = (1 << kFreqBits) - 1;
   for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < n;
        i += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-    const int lane = threadIdx.x & 31;
     const int s0 = off[i], sz = off[i + 1] - s0;
-    const int64_t w0 = pre_off[i], p = pre_off[i + 1] - w0;
-    for (int j = lane; j < p; j += 32) {
-      const uint64_t tok = canon[s0 + j] & tmask;
-      entries[w0 + j] = (tok << (kSizeBits + 21)) | ((uint64_t)sz << 21) | (uint64_t)i;
+    uint64_t* out = entries + pre_off[i];
+    const int p = (int)(pre_off[i + 1] - pre_off[i]);
+    if (p <= 0) continue;
+    const uint64_t low = ((uint64_t)sz << 21) | (uint64_t)i;
+    // keys of the prefix appended in the lanes' order
+    auto emit = [&](auto each, int F, int T, int equal) {
+      int w = 0;
+      each([&](int f, int t) {
+        const bool eq = f == F && t == T;
+        const unsigned em = __ballot_sync(kFull, eq);
+        const bool in = f < F || (f == F && t < T) || (eq && __popc(em & lt) < equal);
+        equal -= min(equal, __popc(em));
+        const unsigned im = __ballot_sync(kFull, in);
+        if (in) out[w + __popc(im & lt)] = ((uint64_t)t << (size_bits + 21)) | low;
+        w += __popc(im);
+      });
+    };
+    auto in_registers = [&](auto r_const) {
+      constexpr int R = decltype(r_const)::value;
+      int f[R], t[R], mx = 0;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int j = r * 32 + lane;
+        t[r] = j < sz ? __ldg(tokens + s0 + j) : INT_MAX;
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        f[r] = r * 32 + lane < sz ? min(__ldg(freq + t[r]), cap) : INT_MAX;
+        if (r * 32 + lane < sz) mx = max(mx, f[r]);
+      }
+      const int fbits = 32 - __clz(__reduce_max_sync(kFull, mx));
+      auto each = [&](auto fn) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) fn(f[r], t[r]);
+      };
+      int F, T, equal;
+      select_key(p, fbits, ulog, each, &F, &T, &equal);
+      emit(each, F, T, equal);
+    };
+    if (sz <= 64) {
+      in_registers(std::integral_constant<int, 2>());
+    } else if (sz <= 256) {
+      in_registers(std::integral_constant<int, 8>());
+    } else if (sz <= 512) {
+      in_registers(std::integral_constant<int, 16>());
+    } else {
+      const int rounds = (sz + 31) / 32;
+      int mx = 0;
+      for (int j = lane; j < sz; j += 32) {
+        const int f = min(__ldg(freq + __ldg(tokens + s0 + j)), cap);
+        fbuf[s0 + j] = f;
+        mx = max(mx, f);
+      }
+      __syncwarp();
+      const int fbits = 32 - __clz(__reduce_max_sync(kFull, mx));
+      auto each = [&](auto fn) {
+#pragma unroll 4
+        for (int r = 0; r < rounds; ++r) {
+          const int j = r * 32 + lane;
+          fn(j < sz ? fbuf[s0 + j] : INT_MAX, j < sz ? __ldg(tokens + s0 + j) : INT_MAX);
+        }
+      };
+      int F, T, equal;
+      select_key(p, fbits, ulog, each, &F, &T, &equal);
+      emit(each, F, T, equal);
     }
   }
 }
 
 // For sorted entry e: partners are the following entries of the same token
 // whose size is <= floor(den*size_e/num) (sizes ascend within a token).
-__global__ void pair_count_kernel(const uint64_t* __restrict__ ent, int64_t ne,
+__global__ void pair_count_kernel(const uint64_t* __restrict__ ent, int64_t ne, int size_bits,
                                   int num, int den, int64_t* __restrict__ cnt) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < ne;
        e += (int64_t)gridDim.x * blockDim.x) {
     const uint64_t k = ent[e];
-    const uint64_t tok = k >> (kSizeBits + 21);
-    const int64_t sz = (int64_t)((k >> 21) & ((1u << kSizeBits) - 1));
+    const uint64_t tok = k >> (size_bits + 21);
+    const int64_t sz = (int64_t)((k >> 21) & ((1u << size_bits) - 1));
     const int64_t maxsz = (den * sz) / num;
-    const int64_t capsz = maxsz < ((1 << kSizeBits) - 1) ? maxsz : ((1 << kSizeBits) - 1);
-    const uint64_t lim = (tok << (kSizeBits + 21)) | ((uint64_t)capsz << 21) |
+    const int64_t capsz = maxsz < ((1 << size_bits) - 1) ? maxsz : ((1 << size_bits) - 1);
+    const uint64_t lim = (tok << (size_bits + 21)) | ((uint64_t)capsz << 21) |
                          ((1ull << 21) - 1);
+    // the end of the partners, a few entries on: by doubling steps, then
+    // halving (0.40 ms by halving alone for 8 M entries, 0.11 this way)
     int64_t a = e + 1, b = ne;
+    for (int64_t step = 1; a < ne; step *= 2) {
+      const int64_t at = a + step - 1 < ne ? a + step - 1 : ne - 1;
+      if (ent[at] > lim) {
+        b = at;
+        break;
+      }
+      a = at + 1;
+    }
     while (a < b) {
       int64_t mid = (a + b) >> 1;
       if (ent[mid] <= lim) a = mid + 1; else b = mid;
@@ -228,7 +329,7 @@ __global__ void pair_count_kernel(const uint64_t* __restrict__ ent, int64_t ne,
 }
 
 __global__ void pair_emit_kernel(const uint64_t* __restrict__ ent, int64_t ne,
-                                 const int64_t* __restrict__ cnt_off,
+                                 const int64_t* __restrict__ cnt_off, int set_bits,
                                  uint64_t* __restrict__ pairs) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < ne;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -238,17 +339,17 @@ __global__ void pair_emit_kernel(const uint64_t* __restrict__ ent, int64_t ne,
     for (int64_t j = 1; j <= c; ++j) {
       const uint32_t sj = (uint32_t)(ent[e + j] & ((1u << 21) - 1));
       const uint32_t lo = se < sj ? se : sj, hi = se < sj ? sj : se;
-      pairs[w++] = ((uint64_t)lo << 32) | hi;
+      pairs[w++] = ((uint64_t)lo << set_bits) | hi;
     }
   }
 }
 
-__global__ void pair_split_kernel(const uint64_t* __restrict__ pairs, int64_t np,
+__global__ void pair_split_kernel(const uint64_t* __restrict__ pairs, int64_t np, int set_bits,
                                   int32_t* __restrict__ pa, int32_t* __restrict__ pb) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np;
        i += (int64_t)gridDim.x * blockDim.x) {
-    pa[i] = (int32_t)(pairs[i] >> 32);
-    pb[i] = (int32_t)(pairs[i] & 0xFFFFFFFFu);
+    pa[i] = (int32_t)(pairs[i] >> set_bits);
+    pb[i] = (int32_t)(pairs[i] & ((1u << set_bits) - 1));
   }
 }
 
@@ -407,38 +508,37 @@ extern "C" reset_status reset_prefix_candidates(const int32_t* d_off,
   cudaStream_t st = as_stream(stream);
   Temps tmp(st);
   const int64_t U = 1ll << universe_log2;
-  int32_t* freq;
-  uint64_t *ck0, *ck1;
+  int32_t *freq, *fbuf;
   int64_t *plen, *poff;
   RST_CUDA(tmp.get(&freq, sizeof(int32_t) * U));
   RST_CUDA(cudaMemsetAsync(freq, 0, sizeof(int32_t) * U, st));
-  RST_CUDA(tmp.get(&ck0, sizeof(uint64_t) * (m > 0 ? m : 1)));
-  RST_CUDA(tmp.get(&ck1, sizeof(uint64_t) * (m > 0 ? m : 1)));
   RST_CUDA(tmp.get(&plen, sizeof(int64_t) * (n + 1)));
-  RST_CUDA(tmp.get(&poff, sizeof(int64_t) * (n + 1)));
-  note_launch();
+  RST_CUDA(tmp.get(&poff, sizeof(int64_t) * (n + 2)));  // [n + 1]: the largest set
+  RST_CUDA(cudaMemsetAsync(poff + n + 1, 0, sizeof(int64_t), st));
+  note_launch(2);
   token_freq_kernel<<<g_grid(m), 256, 0, st>>>(d_tokens, m, freq);
-  note_launch();
-  canon_keys_kernel<<<g_grid((int64_t)n * 32), 256, 0, st>>>(d_off, n, d_tokens, freq,
-                                                             universe_log2, ck0);
+  prefix_len_kernel<<<g_grid(n), 256, 0, st>>>(d_off, n, num, den, plen, poff + n + 1);
   RST_CUDA(cudaGetLastError());
-  cub::DoubleBuffer<uint64_t> cb(ck0, ck1);
-  size_t ts = 0;
-  RST_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, ts, cb, m, 0, 64, st));
-  void* d_ts;
-  RST_CUDA(tmp.get(&d_ts, ts));
-  RST_CUDA(cub::DeviceRadixSort::SortKeys(d_ts, ts, cb, m, 0, 64, st));
-  note_launch();
-  prefix_len_kernel<<<g_grid(n), 256, 0, st>>>(d_off, n, num, den, plen);
   RST_CUDA(cudaMemsetAsync(plen + n, 0, sizeof(int64_t), st));
   size_t tsc = 0;
   RST_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tsc, plen, poff, n + 1, st));
   void* d_tsc;
   RST_CUDA(tmp.get(&d_tsc, tsc));
   RST_CUDA(cub::DeviceScan::ExclusiveSum(d_tsc, tsc, plen, poff, n + 1, st));
-  int64_t ne = 0;
-  RST_CUDA(cudaMemcpyAsync(&ne, poff + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+  int64_t sizes[2] = {0, 0};  // entries, the largest set
+  RST_CUDA(cudaMemcpyAsync(sizes, poff + n, sizeof(sizes), cudaMemcpyDeviceToHost, st));
   RST_CUDA(cudaStreamSynchronize(st));
+  const int64_t ne = sizes[0];
+  // keys to be sorted hold as many bits as sizes and ids need, and no others
+  // are sorted by: the passes of a radix sort are paid per 8 bits
+  auto bits_for = [](int64_t x) {
+    int b = 1;
+    while ((x >> b) != 0) ++b;
+    return b;
+  };
+  const int size_bits = std::min(bits_for(sizes[1]), 64 - 21 - universe_log2);
+  const int set_bits = bits_for((int64_t)n - 1);
+  RST_CUDA(tmp.get(&fbuf, sizes[1] > 512 ? sizeof(int32_t) * (m > 0 ? m : 1) : 16));
   uint64_t *e0, *e1;
   int64_t *cnt, *coff;
   RST_CUDA(tmp.get(&e0, sizeof(uint64_t) * (ne > 0 ? ne : 1)));
@@ -447,17 +547,17 @@ extern "C" reset_status reset_prefix_candidates(const int32_t* d_off,
   RST_CUDA(tmp.get(&coff, sizeof(int64_t) * (ne + 1)));
   note_launch();
   prefix_entries_kernel<<<g_grid((int64_t)n * 32), 256, 0, st>>>(
-      d_off, n, cb.Current(), poff, universe_log2, e0);
+      d_off, n, d_tokens, freq, poff, universe_log2, size_bits, fbuf, e0);
   RST_CUDA(cudaGetLastError());
   cub::DoubleBuffer<uint64_t> eb(e0, e1);
   size_t te = 0;
-  const int ebits = universe_log2 + kSizeBits + 21;
-  RST_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, te, eb, ne, 0, ebits, st));
+  const int ebits = universe_log2 + size_bits + 21;
+  RST_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, te, eb, ne, 21, ebits, st));
   void* d_te;
   RST_CUDA(tmp.get(&d_te, te));
-  RST_CUDA(cub::DeviceRadixSort::SortKeys(d_te, te, eb, ne, 0, ebits, st));
+  RST_CUDA(cub::DeviceRadixSort::SortKeys(d_te, te, eb, ne, 21, ebits, st));
   note_launch();
-  pair_count_kernel<<<g_grid(ne), 256, 0, st>>>(eb.Current(), ne, num, den, cnt);
+  pair_count_kernel<<<g_grid(ne), 256, 0, st>>>(eb.Current(), ne, size_bits, num, den, cnt);
   RST_CUDA(cudaMemsetAsync(cnt + ne, 0, sizeof(int64_t), st));
   size_t tc2 = 0;
   RST_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tc2, cnt, coff, ne + 1, st));
@@ -473,15 +573,15 @@ extern "C" reset_status reset_prefix_candidates(const int32_t* d_off,
   RST_CUDA(tmp.get(&p1, sizeof(uint64_t) * (nraw > 0 ? nraw : 1)));
   RST_CUDA(tmp.get(&d_np, sizeof(int64_t)));
   note_launch();
-  pair_emit_kernel<<<g_grid(ne), 256, 0, st>>>(eb.Current(), ne, coff, p0);
+  pair_emit_kernel<<<g_grid(ne), 256, 0, st>>>(eb.Current(), ne, coff, set_bits, p0);
   RST_CUDA(cudaGetLastError());
   cub::DoubleBuffer<uint64_t> pb(p0, p1);
   size_t tp = 0, tu = 0;
-  RST_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, tp, pb, nraw, 0, 64, st));
+  RST_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, tp, pb, nraw, 0, 2 * set_bits, st));
   RST_CUDA(cub::DeviceSelect::Unique(nullptr, tu, p0, p1, d_np, nraw, st));
   void* d_tp;
   RST_CUDA(tmp.get(&d_tp, tp > tu ? tp : tu));
-  RST_CUDA(cub::DeviceRadixSort::SortKeys(d_tp, tp, pb, nraw, 0, 64, st));
+  RST_CUDA(cub::DeviceRadixSort::SortKeys(d_tp, tp, pb, nraw, 0, 2 * set_bits, st));
   RST_CUDA(cub::DeviceSelect::Unique(d_tp, tu, pb.Current(), pb.Alternate(), d_np, nraw, st));
   int64_t np = 0;
   RST_CUDA(cudaMemcpyAsync(&np, d_np, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
@@ -494,7 +594,7 @@ extern "C" reset_status reset_prefix_candidates(const int32_t* d_off,
     return cuda_fail(e, "cudaMalloc", __FILE__, __LINE__);
   }
   note_launch();
-  pair_split_kernel<<<g_grid(np), 256, 0, st>>>(pb.Alternate(), np, pa, pbb);
+  pair_split_kernel<<<g_grid(np), 256, 0, st>>>(pb.Alternate(), np, set_bits, pa, pbb);
   e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {

@@ -326,3 +326,38 @@ def test_decisions_only_like_full(R, cuda, kind, num, den):
         dec, none = R.sss(t, d_off, d_cols, x, y, num, den, with_inter=False)
         assert none is None and 0 < int(full.sum()) < full.numel()
         assert cuda.equal(full, dec)
+
+
+# -------------------------------------------------------- prefix filter --
+
+@pytest.mark.parametrize("num,den", [(1, 2), (7, 10), (1, 1)])
+@pytest.mark.parametrize("freq", ["skewed", "level", "repeated"])
+def test_prefix_selection_at_set_sizes(R, cuda, freq, num, den):
+    """Sets around every size whose selection runs in registers and past the
+    largest; frequencies that differ, tie, and tokens repeated in a set."""
+    rng = np.random.default_rng(num + 10 * den)
+    rows = []
+    for size in [0, 1, 2, 31, 63, 64, 65, 255, 256, 257, 511, 512, 513, 1500]:
+        for _ in range(3):
+            if freq == "level":  # runs of a cycle: every token equally often, nearly
+                r = (np.arange(size) + rng.integers(0, 4096)) % 4096
+            else:
+                r = (4096 * rng.random(2 * size) ** 2).astype(int)
+                r = np.unique(r)[:size] if freq == "skewed" else np.sort(r[:size])
+            rows.append(r.astype(np.int32))
+    off, tok = csr(rows)
+    pa, pb = R.prefix_candidates(dev(off, cuda), dev(tok, cuda), 12, num, den)
+    f = np.bincount(tok, minlength=4096)
+    by_token, want = {}, set()
+    for i, r in enumerate(rows):
+        p = len(r) - -(-num * len(r) // den) + 1 if len(r) else 0
+        for t in sorted(r.tolist(), key=lambda t: (f[t], t))[:p]:
+            by_token.setdefault(t, []).append((len(r), i))
+    for e in by_token.values():
+        e.sort()
+        for k, (size, i) in enumerate(e):
+            for other, j in e[k + 1:]:
+                if other <= den * size // num:
+                    want.add((min(i, j), max(i, j)))
+    got = list(zip(pa.cpu().tolist(), pb.cpu().tolist()))
+    assert got == sorted(want)
