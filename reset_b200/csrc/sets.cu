@@ -152,12 +152,35 @@ __global__ void split_keys_kernel(const uint64_t* __restrict__ keys, int64_t m,
 // ---- prefix filtering -----------------------------------------------------
 
 constexpr int kFreqBits = 19;
+constexpr int kInShared = 1024;  // keys of a set whose frequencies a warp holds in shared memory
 
-__global__ void token_freq_kernel(const int32_t* __restrict__ tokens, int64_t m,
-                                  int32_t* __restrict__ freq) {
+// Counts of the tokens.  Few tokens are in many sets and their counters are
+// where the atomics of all blocks queue (0.57 ms for 50 M tokens, the most
+// frequent in 300,000 sets): a block counts the tokens that come first to a
+// slot of its cache in shared memory, which the frequent ones do.
+constexpr int kFreqCache = 4096;
+
+__global__ void __launch_bounds__(256)
+    token_freq_kernel(const int32_t* __restrict__ tokens, int64_t m, int32_t* __restrict__ freq) {
+  __shared__ int s_tok[kFreqCache], s_cnt[kFreqCache];
+  for (int i = threadIdx.x; i < kFreqCache; i += blockDim.x) {
+    s_tok[i] = -1;
+    s_cnt[i] = 0;
+  }
+  __syncthreads();
+#pragma unroll 4
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < m;
-       j += (int64_t)gridDim.x * blockDim.x)
-    atomicAdd(&freq[tokens[j]], 1);
+       j += (int64_t)gridDim.x * blockDim.x) {
+    const int t = __ldg(tokens + j);
+    const int h = ((unsigned)t * 0x9E3779B1u) >> 20;
+    int at = s_tok[h];
+    if (at == -1) at = atomicCAS(&s_tok[h], -1, t);
+    if (at == -1 || at == t) atomicAdd(&s_cnt[h], 1);
+    else atomicAdd(&freq[t], 1);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kFreqCache; i += blockDim.x)
+    if (s_cnt[i]) atomicAdd(&freq[s_tok[i]], s_cnt[i]);
 }
 
 // Prefix lengths, and the largest set.
@@ -178,120 +201,144 @@ __global__ void prefix_len_kernel(const int32_t* __restrict__ off, int32_t n,
     atomicMax(reinterpret_cast<unsigned long long*>(largest), (unsigned long long)mx);
 }
 
-// The p-th smallest (frequency, token) of a set of n keys read by a warp
-// through each(f): f(frequency, token) for every key of this lane.  Found by
-// bits, the frequency's first: a count of the set's keys per bit, in
-// registers, where sorting all sets' keys took eight radix passes over the
-// collection, 128 B of HBM per key.  *equal: how many keys equal to it belong
-// to the p smallest.  Bound by instructions; 50 M tokens in 400,000 sets:
-// 5.0 ms for keys and sort, 1.44 this way.
-template <class Each>
-__device__ __forceinline__ void select_key(int p, int fbits, int ulog, Each each, int* f_out,
-                                           int* t_out, int* equal) {
-  auto count = [&](auto test) {
-    int c = 0;
-    each([&](int f, int t) { c += test(f, t); });
-    return __reduce_add_sync(kFull, c);
-  };
-  int F = 0;  // largest value with fewer than p keys below it
-  for (int bit = fbits - 1; bit >= 0; --bit) {
-    const int cand = F | 1 << bit;
-    if (count([&](int f, int) { return f < cand; }) < p) F = cand;
-  }
-  p -= count([&](int f, int) { return f < F; });
-  *f_out = F;
-  *t_out = INT_MAX;
-  *equal = p;
-  if (count([&](int f, int) { return f == F; }) == p) return;  // all of that frequency
-  int T = 0;
-  for (int bit = ulog - 1; bit >= 0; --bit) {
-    const int cand = T | 1 << bit;
-    if (count([&](int f, int t) { return f == F && t < cand; }) < p) T = cand;
-  }
-  *equal = p - count([&](int f, int t) { return f == F && t < T; });
-  *t_out = T;
+// How many of this warp's keys pass each of three tests, by each(fn): fn(j, f)
+// for every key of the lane, index and frequency (j past the set and f =
+// INT_MAX in a last, partial row).
+template <class Each, class T0, class T1, class T2>
+__device__ __forceinline__ int3 count_keys(Each each, T0 t0, T1 t1, T2 t2) {
+  int c0 = 0, c1 = 0, c2 = 0;
+  each([&](int j, int f) {
+    c0 += t0(j, f);
+    c1 += t1(j, f);
+    c2 += t2(j, f);
+  });
+  return make_int3(__reduce_add_sync(kFull, c0), __reduce_add_sync(kFull, c1),
+                   __reduce_add_sync(kFull, c2));
 }
 
 // Entries (token | size | set) of every set's prefix: its p smallest tokens by
 // (min(frequency, cap), token) -- one global order, the same for every set --
-// in no particular order.  A warp per set; fbuf (m ints) holds the
-// frequencies of sets too large for registers.
+// in no particular order.  A warp per set finds the p-th by counting: the
+// frequency (mostly a small one: its magnitude, then two bits at a time); of
+// the tokens with that frequency the first ones, which in an ascending row
+// are the smallest, else the token in the same way.  The frequencies of up to
+// kInShared keys lie in shared memory, those of larger sets in fbuf (m ints).
+// Bound by the latency of the frequencies' random reads and by instructions.
+// 50 M tokens in 400,000 sets: 5.0 ms by sorting all sets' keys (eight radix
+// passes, 128 B of HBM per key), 1.74 with the keys in registers and a code
+// path per size (past the instruction cache), 1.02 this way.
 __global__ void __launch_bounds__(256)
     prefix_entries_kernel(const int32_t* __restrict__ off, int32_t n,
                           const int32_t* __restrict__ tokens, const int32_t* __restrict__ freq,
                           const int64_t* __restrict__ pre_off, int ulog, int size_bits,
-                          int32_t* __restrict__ fbuf, uint64_t* __restrict__ entries) {
-  const int lane = threadIdx.x & 31;
+                          int32_t* __restrict__ fbuf, uint64_t* __restrict__ entries,
+                          unsigned long long* __restrict__ cursor) {
+  __shared__ __align__(16) int s_freq[8][kInShared];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned lt = lanemask_lt();
   const int cap = (1 << kFreqBits) - 1;
-  for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < n;
-       i += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+  const auto none = [](int, int) { return 0; };
+  // sets differ in size: each warp takes the next one, asked for a set ahead
+  auto ask = [&] { return lane == 0 ? atomicAdd(cursor, 1ull) : 0ull; };
+  unsigned long long next = ask();
+  for (;;) {
+    const int64_t i = (int64_t)__shfl_sync(kFull, next, 0);
+    if (i >= n) break;
+    next = ask();
     const int s0 = off[i], sz = off[i + 1] - s0;
     uint64_t* out = entries + pre_off[i];
-    const int p = (int)(pre_off[i + 1] - pre_off[i]);
+    int p = (int)(pre_off[i + 1] - pre_off[i]);
     if (p <= 0) continue;
     const uint64_t low = ((uint64_t)sz << 21) | (uint64_t)i;
-    // keys of the prefix appended in the lanes' order
-    auto emit = [&](auto each, int F, int T, int equal) {
+    auto token = [&](int j) { return __ldg(tokens + s0 + j); };
+    auto select = [&](const int* fr, bool ascends, auto each) {
+      // F: largest value with fewer than p keys below it
+      int3 c = count_keys(each, [](int, int f) { return f < 1 << 4; },
+                          [](int, int f) { return f < 1 << 8; },
+                          [](int, int f) { return f < 1 << 12; });
+      int F = 0;
+      for (int bit = c.x >= p ? 4 : c.y >= p ? 8 : c.z >= p ? 12 : (kFreqBits + 1) / 2 * 2;
+           bit;) {
+        bit -= 2;
+        c = count_keys(each, [&](int, int f) { return f < (F | 1 << bit); },
+                       [&](int, int f) { return f < (F | 2 << bit); },
+                       [&](int, int f) { return f < (F | 3 << bit); });
+        F |= ((c.x < p) + (c.y < p) + (c.z < p)) << bit;
+      }
+      c = count_keys(each, [&](int, int f) { return f < F; }, [&](int, int f) { return f == F; },
+                     none);
+      p -= c.x;
+      ascends = ascends || c.y == p;  // (all of them)
+      int T = 0;
+      if (!ascends) {
+        for (int bit = (ulog + 1) / 2 * 2; bit;) {
+          bit -= 2;
+          auto below = [&](int digit) {
+            return [&, digit](int j, int f) { return f == F && token(j) < (T | digit << bit); };
+          };
+          c = count_keys(each, below(1), below(2), below(3));
+          T |= ((c.x < p) + (c.y < p) + (c.z < p)) << bit;
+        }
+        p -= count_keys(each, [&](int j, int f) { return f == F && token(j) < T; }, none, none).x;
+      }
       int w = 0;
-      each([&](int f, int t) {
-        const bool eq = f == F && t == T;
-        const unsigned em = __ballot_sync(kFull, eq);
-        const bool in = f < F || (f == F && t < T) || (eq && __popc(em & lt) < equal);
-        equal -= min(equal, __popc(em));
+      for (int j = lane; j - lane < sz; j += 32) {  // p: of those that tie still to take
+        const int f = j < sz ? fr[j] : INT_MAX;
+        const int t = f <= F ? token(j) : 0;
+        const bool tie = f == F && (ascends || t == T);
+        const unsigned tm = __ballot_sync(kFull, tie);
+        const bool in = f < F || (f == F && (tie ? __popc(tm & lt) < p : !ascends && t < T));
+        p -= min(p, __popc(tm));
         const unsigned im = __ballot_sync(kFull, in);
         if (in) out[w + __popc(im & lt)] = ((uint64_t)t << (size_bits + 21)) | low;
         w += __popc(im);
-      });
+      }
     };
-    auto in_registers = [&](auto r_const) {
-      constexpr int R = decltype(r_const)::value;
-      int f[R], t[R], mx = 0;
+    bool ascends = true;
+    auto fill = [&](int* fr) {
+      constexpr int R = 8;  // rows of 32 keys in flight
+      for (int base = 0; base < sz; base += 32 * R) {
+        int t[R], f[R];
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int j = r * 32 + lane;
-        t[r] = j < sz ? __ldg(tokens + s0 + j) : INT_MAX;
-      }
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        f[r] = r * 32 + lane < sz ? min(__ldg(freq + t[r]), cap) : INT_MAX;
-        if (r * 32 + lane < sz) mx = max(mx, f[r]);
-      }
-      const int fbits = 32 - __clz(__reduce_max_sync(kFull, mx));
-      auto each = [&](auto fn) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) fn(f[r], t[r]);
-      };
-      int F, T, equal;
-      select_key(p, fbits, ulog, each, &F, &T, &equal);
-      emit(each, F, T, equal);
-    };
-    if (sz <= 64) {
-      in_registers(std::integral_constant<int, 2>());
-    } else if (sz <= 256) {
-      in_registers(std::integral_constant<int, 8>());
-    } else if (sz <= 512) {
-      in_registers(std::integral_constant<int, 16>());
-    } else {
-      const int rounds = (sz + 31) / 32;
-      int mx = 0;
-      for (int j = lane; j < sz; j += 32) {
-        const int f = min(__ldg(freq + __ldg(tokens + s0 + j)), cap);
-        fbuf[s0 + j] = f;
-        mx = max(mx, f);
-      }
-      __syncwarp();
-      const int fbits = 32 - __clz(__reduce_max_sync(kFull, mx));
-      auto each = [&](auto fn) {
-#pragma unroll 4
-        for (int r = 0; r < rounds; ++r) {
-          const int j = r * 32 + lane;
-          fn(j < sz ? fbuf[s0 + j] : INT_MAX, j < sz ? __ldg(tokens + s0 + j) : INT_MAX);
+        for (int r = 0; r < R; ++r) {
+          const int j = base + r * 32 + lane;
+          t[r] = token(min(j, sz - 1));
+          f[r] = token(max(min(j, sz - 1) - 1, 0));  // the one before
         }
-      };
-      int F, T, equal;
-      select_key(p, fbits, ulog, each, &F, &T, &equal);
-      emit(each, F, T, equal);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          ascends &= f[r] <= t[r];
+          f[r] = base + r * 32 < sz ? __ldg(freq + t[r]) : 0;
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const int j = base + r * 32 + lane;
+          if (j < sz) fr[j] = min(f[r], cap);
+        }
+      }
+    };
+    if (sz <= kInShared) {
+      int* fr = s_freq[warp];
+      fill(fr);
+      for (int j = sz + lane; j < (sz + 127) / 128 * 128; j += 32) fr[j] = INT_MAX;
+      __syncwarp();
+      select(fr, __all_sync(kFull, ascends), [&](auto fn) {
+        for (int j = lane * 4; j - lane * 4 < sz; j += 128) {
+          const int4 v = *reinterpret_cast<const int4*>(fr + j);
+          fn(j, v.x);
+          fn(j + 1, v.y);
+          fn(j + 2, v.z);
+          fn(j + 3, v.w);
+        }
+      });
+      __syncwarp();
+    } else {
+      int* fr = fbuf + s0;
+      fill(fr);
+      __syncwarp();
+      select(fr, __all_sync(kFull, ascends), [&](auto fn) {
+        for (int j = lane; j - lane < sz; j += 32) fn(j, j < sz ? fr[j] : INT_MAX);
+      });
     }
   }
 }
@@ -513,8 +560,8 @@ extern "C" reset_status reset_prefix_candidates(const int32_t* d_off,
   RST_CUDA(tmp.get(&freq, sizeof(int32_t) * U));
   RST_CUDA(cudaMemsetAsync(freq, 0, sizeof(int32_t) * U, st));
   RST_CUDA(tmp.get(&plen, sizeof(int64_t) * (n + 1)));
-  RST_CUDA(tmp.get(&poff, sizeof(int64_t) * (n + 2)));  // [n + 1]: the largest set
-  RST_CUDA(cudaMemsetAsync(poff + n + 1, 0, sizeof(int64_t), st));
+  RST_CUDA(tmp.get(&poff, sizeof(int64_t) * (n + 3)));  // then the largest set, a cursor
+  RST_CUDA(cudaMemsetAsync(poff + n + 1, 0, 2 * sizeof(int64_t), st));
   note_launch(2);
   token_freq_kernel<<<g_grid(m), 256, 0, st>>>(d_tokens, m, freq);
   prefix_len_kernel<<<g_grid(n), 256, 0, st>>>(d_off, n, num, den, plen, poff + n + 1);
@@ -538,7 +585,7 @@ extern "C" reset_status reset_prefix_candidates(const int32_t* d_off,
   };
   const int size_bits = std::min(bits_for(sizes[1]), 64 - 21 - universe_log2);
   const int set_bits = bits_for((int64_t)n - 1);
-  RST_CUDA(tmp.get(&fbuf, sizes[1] > 512 ? sizeof(int32_t) * (m > 0 ? m : 1) : 16));
+  RST_CUDA(tmp.get(&fbuf, sizes[1] > kInShared ? sizeof(int32_t) * (m > 0 ? m : 1) : 16));
   uint64_t *e0, *e1;
   int64_t *cnt, *coff;
   RST_CUDA(tmp.get(&e0, sizeof(uint64_t) * (ne > 0 ? ne : 1)));
@@ -546,8 +593,9 @@ extern "C" reset_status reset_prefix_candidates(const int32_t* d_off,
   RST_CUDA(tmp.get(&cnt, sizeof(int64_t) * (ne + 1)));
   RST_CUDA(tmp.get(&coff, sizeof(int64_t) * (ne + 1)));
   note_launch();
-  prefix_entries_kernel<<<g_grid((int64_t)n * 32), 256, 0, st>>>(
-      d_off, n, d_tokens, freq, poff, universe_log2, size_bits, fbuf, e0);
+  prefix_entries_kernel<<<std::min((n + 7) / 8, sm_count() * 6), 256, 0, st>>>(
+      d_off, n, d_tokens, freq, poff, universe_log2, size_bits, fbuf, e0,
+      reinterpret_cast<unsigned long long*>(poff + n + 2));
   RST_CUDA(cudaGetLastError());
   cub::DoubleBuffer<uint64_t> eb(e0, e1);
   size_t te = 0;

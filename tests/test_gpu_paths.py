@@ -331,19 +331,21 @@ def test_decisions_only_like_full(R, cuda, kind, num, den):
 # -------------------------------------------------------- prefix filter --
 
 @pytest.mark.parametrize("num,den", [(1, 2), (7, 10), (1, 1)])
-@pytest.mark.parametrize("freq", ["skewed", "level", "repeated"])
+@pytest.mark.parametrize("freq", ["skewed", "level", "repeated", "shuffled"])
 def test_prefix_selection_at_set_sizes(R, cuda, freq, num, den):
-    """Sets around every size whose selection runs in registers and past the
-    largest; frequencies that differ, tie, and tokens repeated in a set."""
+    """Sets around the sizes of a row of lanes, of vectors and of the shared
+    buffer and past it; frequencies that differ and tie, tokens repeated in a
+    set, rows that do not ascend ("level": all tie and the row wraps)."""
     rng = np.random.default_rng(num + 10 * den)
     rows = []
-    for size in [0, 1, 2, 31, 63, 64, 65, 255, 256, 257, 511, 512, 513, 1500]:
+    for size in [0, 1, 2, 31, 63, 64, 65, 255, 256, 257, 511, 512, 513, 1023, 1024, 1025, 1500]:
         for _ in range(3):
             if freq == "level":  # runs of a cycle: every token equally often, nearly
                 r = (np.arange(size) + rng.integers(0, 4096)) % 4096
             else:
                 r = (4096 * rng.random(2 * size) ** 2).astype(int)
-                r = np.unique(r)[:size] if freq == "skewed" else np.sort(r[:size])
+                r = np.sort(r[:size]) if freq == "repeated" else np.unique(r)[:size]
+                r = rng.permutation(r) if freq == "shuffled" else r
             rows.append(r.astype(np.int32))
     off, tok = csr(rows)
     pa, pb = R.prefix_candidates(dev(off, cuda), dev(tok, cuda), 12, num, den)
