@@ -268,6 +268,18 @@ reset_status reset_prefix_candidates(const int32_t *d_off, const int32_t *d_toke
                                      int32_t **d_pb_out, int64_t *np_out,
                                      reset_stream_t stream);
 
+/* The same with the outputs in the caller's device memory: alloc(bytes, ctx)
+ * is called on the calling thread, twice, when the number of pairs is known,
+ * and returns memory that `stream` may write at once, or NULL
+ * (RESET_ERR_CUDA).  What it returned stays the caller's, on errors too. */
+typedef void *(*reset_alloc_fn)(int64_t bytes, void *ctx);
+reset_status reset_prefix_candidates_alloc(const int32_t *d_off, const int32_t *d_tokens,
+                                           int32_t n, int64_t m, int32_t universe_log2,
+                                           int32_t num, int32_t den, reset_alloc_fn alloc,
+                                           void *ctx, int32_t **d_pa_out,
+                                           int32_t **d_pb_out, int64_t *np_out,
+                                           reset_stream_t stream);
+
 /* Conjunctive retrieval.  The table is built over the inverted index
  * (d_toff[nterms+1], d_docs).  Query q is the term list
  * d_query[d_qoff[q] .. d_qoff[q+1]); its result is the posting list of its

@@ -88,6 +88,7 @@ class ServerCounters(C.Structure):
 P = C.c_void_p
 I32 = C.c_int32
 I64 = C.c_int64
+AllocFn = C.CFUNCTYPE(C.c_void_p, C.c_int64, C.c_void_p)
 
 # name -> (restype, argtypes); every symbol include/reset.h declares.
 SIGNATURES = {
@@ -129,6 +130,8 @@ SIGNATURES = {
                                    C.POINTER(P), C.POINTER(P), C.POINTER(I64), P]),
     "reset_prefix_candidates": (I32, [P, P, I32, I64, I32, I32, I32, C.POINTER(P),
                                       C.POINTER(P), C.POINTER(I64), P]),
+    "reset_prefix_candidates_alloc": (I32, [P, P, I32, I64, I32, I32, I32, AllocFn, P,
+                                            C.POINTER(P), C.POINTER(P), C.POINTER(I64), P]),
     "reset_gen_inverted_index": (I32, [I32, I32, C.c_double, I64, C.c_uint64,
                                        C.POINTER(P), C.POINTER(P), C.POINTER(I64), P]),
     "reset_server_config_default": (None, [C.POINTER(ServerConfig)]),

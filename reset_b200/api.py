@@ -12,7 +12,7 @@ from typing import NamedTuple, Optional, Tuple
 
 import torch
 
-from ._lib import Params, Pattern, TableView, Tuning, check, load
+from ._lib import AllocFn, Params, Pattern, TableView, Tuning, check, load
 
 
 def _lib():
@@ -467,17 +467,26 @@ def prefix_candidates(off: torch.Tensor, tokens: torch.Tensor, universe_log2: in
     """Prefix-filter candidate pairs (a < b, sorted) -> (pa, pb) int32."""
     _need(off, torch.int32, "off")
     _need(tokens, torch.int32, "tokens")
-    L = _lib()
+    current = torch.cuda.current_stream()
+    outs, failed = [], []
+
+    @AllocFn
+    def alloc(nbytes, _):
+        try:
+            outs.append(torch.empty(nbytes // 4, dtype=torch.int32, device=off.device))
+            if stream is not None and stream != current:
+                current.synchronize()  # the memory may be in use there still
+            return outs[-1].data_ptr()
+        except Exception as e:  # raised below: nothing passes through the library
+            failed.append(e)
+            return None
+
     pa, pb, npr = C.c_void_p(), C.c_void_p(), C.c_int64()
-    check(L.reset_prefix_candidates(_ptr(off), _ptr(tokens), off.numel() - 1,
-                                    tokens.numel(), universe_log2, num, den,
-                                    C.byref(pa), C.byref(pb), C.byref(npr),
-                                    _stream(stream)))
-    try:
-        a = _view(pa.value, npr.value, torch.int32).clone()
-        b = _view(pb.value, npr.value, torch.int32).clone()
-        torch.cuda.current_stream().synchronize()
-    finally:
-        L.reset_free(pa)
-        L.reset_free(pb)
+    status = _lib().reset_prefix_candidates_alloc(
+        _ptr(off), _ptr(tokens), off.numel() - 1, tokens.numel(), universe_log2, num, den,
+        alloc, None, C.byref(pa), C.byref(pb), C.byref(npr), _stream(stream))
+    if failed:
+        raise failed[0]
+    check(status)
+    a, b = (t[:npr.value] for t in outs)
     return a, b

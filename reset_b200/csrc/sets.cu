@@ -539,15 +539,19 @@ extern "C" reset_status reset_gen_token_sets(int32_t n, int32_t universe_log2,
   return RESET_OK;
 }
 
-extern "C" reset_status reset_prefix_candidates(const int32_t* d_off,
-                                                const int32_t* d_tokens,
-                                                int32_t n, int64_t m,
-                                                int32_t universe_log2,
-                                                int32_t num, int32_t den,
-                                                int32_t** d_pa_out,
-                                                int32_t** d_pb_out,
-                                                int64_t* np_out,
-                                                reset_stream_t stream) {
+// The outputs' memory comes from the caller: cudaMalloc and cudaFree of two
+// arrays of 21 MB took 1.7 of 6.5 ms of a call.
+extern "C" reset_status reset_prefix_candidates_alloc(const int32_t* d_off,
+                                                      const int32_t* d_tokens,
+                                                      int32_t n, int64_t m,
+                                                      int32_t universe_log2,
+                                                      int32_t num, int32_t den,
+                                                      reset_alloc_fn alloc, void* ctx,
+                                                      int32_t** d_pa_out,
+                                                      int32_t** d_pb_out,
+                                                      int64_t* np_out,
+                                                      reset_stream_t stream) {
+  if (!alloc) return arg_fail("NULL alloc");
   if (!d_pa_out || !d_pb_out || !np_out) return arg_fail("NULL output");
   if (n < 1 || n >= (1 << 21)) return arg_fail("n must be in 1..2^21-1");
   if (universe_log2 < 4 || universe_log2 > 24) return arg_fail("universe_log2 in 4..24");
@@ -634,26 +638,46 @@ extern "C" reset_status reset_prefix_candidates(const int32_t* d_off,
   int64_t np = 0;
   RST_CUDA(cudaMemcpyAsync(&np, d_np, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   RST_CUDA(cudaStreamSynchronize(st));
-  int32_t *pa = nullptr, *pbb = nullptr;
-  RST_CUDA(cudaMalloc(&pa, sizeof(int32_t) * (np > 0 ? np : 1)));
-  cudaError_t e = cudaMalloc(&pbb, sizeof(int32_t) * (np > 0 ? np : 1));
-  if (e != cudaSuccess) {
-    cudaFree(pa);
-    return cuda_fail(e, "cudaMalloc", __FILE__, __LINE__);
-  }
+  const int64_t bytes = (int64_t)sizeof(int32_t) * (np > 0 ? np : 1);
+  auto* pa = static_cast<int32_t*>(alloc(bytes, ctx));
+  auto* pbb = pa ? static_cast<int32_t*>(alloc(bytes, ctx)) : nullptr;
+  if (!pbb) return cuda_fail(cudaErrorMemoryAllocation, "alloc", __FILE__, __LINE__);
   note_launch();
   pair_split_kernel<<<g_grid(np), 256, 0, st>>>(pb.Alternate(), np, set_bits, pa, pbb);
-  e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) {
-    cudaFree(pa);
-    cudaFree(pbb);
-    return cuda_fail(e, "candidate split", __FILE__, __LINE__);
-  }
+  RST_CUDA(cudaGetLastError());
+  RST_CUDA(cudaStreamSynchronize(st));
   *d_pa_out = pa;
   *d_pb_out = pbb;
   *np_out = np;
   return RESET_OK;
+}
+
+extern "C" reset_status reset_prefix_candidates(const int32_t* d_off,
+                                                const int32_t* d_tokens,
+                                                int32_t n, int64_t m,
+                                                int32_t universe_log2,
+                                                int32_t num, int32_t den,
+                                                int32_t** d_pa_out,
+                                                int32_t** d_pb_out,
+                                                int64_t* np_out,
+                                                reset_stream_t stream) {
+  struct Got {
+    void* p[2];
+    int n;
+    cudaError_t err;
+  } got{{nullptr, nullptr}, 0, cudaSuccess};
+  const reset_status rc = reset_prefix_candidates_alloc(
+      d_off, d_tokens, n, m, universe_log2, num, den,
+      [](int64_t bytes, void* ctx) -> void* {
+        auto* g = static_cast<Got*>(ctx);
+        void* q = nullptr;
+        g->err = cudaMalloc(&q, (size_t)bytes);
+        return g->err == cudaSuccess ? g->p[g->n++] = q : nullptr;
+      },
+      &got, d_pa_out, d_pb_out, np_out, stream);
+  if (rc != RESET_OK)
+    for (int k = 0; k < got.n; ++k) cudaFree(got.p[k]);
+  return got.err == cudaSuccess ? rc : cuda_fail(got.err, "cudaMalloc", __FILE__, __LINE__);
 }
 
 extern "C" reset_status reset_gen_inverted_index(int32_t nterms, int32_t ndocs,

@@ -363,3 +363,29 @@ def test_prefix_selection_at_set_sizes(R, cuda, freq, num, den):
                     want.add((min(i, j), max(i, j)))
     got = list(zip(pa.cpu().tolist(), pb.cpu().tolist()))
     assert got == sorted(want)
+
+
+def test_prefix_outputs_in_either_memory(R, cuda, libreset):
+    """Pairs in memory of the library's and of the caller's; memory refused."""
+    import ctypes as C
+    from reset_b200._lib import AllocFn
+    off, tok = R.gen_token_sets(3000, 12, size_lo=4, size_hi=60, seed=3)
+    pa, pb = R.prefix_candidates(off, tok, 12)
+    args = (C.c_void_p(off.data_ptr()), C.c_void_p(tok.data_ptr()), off.numel() - 1, tok.numel(),
+            12, 7, 10)
+    p, q, k = C.c_void_p(), C.c_void_p(), C.c_int64()
+    outs = (C.byref(p), C.byref(q), C.byref(k), C.c_void_p(0))
+    cuda.cuda.synchronize()
+    assert libreset.reset_prefix_candidates(*args, *outs) == 0 and k.value == pa.numel() > 0
+    assert cuda.equal(R._view(p.value, k.value, cuda.int32), pa)
+    assert cuda.equal(R._view(q.value, k.value, cuda.int32), pb)
+    libreset.reset_free(p)
+    libreset.reset_free(q)
+    calls = []
+    for _ in range(2):  # none, then the first alone
+        mem = cuda.empty(pa.numel(), dtype=cuda.int32, device="cuda")
+        fn = AllocFn(lambda n, _: calls.append(n) or (mem.data_ptr() if len(calls) == 2 else None))
+        assert libreset.reset_prefix_candidates_alloc(*args, fn, None, *outs) != 0
+    assert calls == [4 * pa.numel()] * 3
+    a2, b2 = R.prefix_candidates(off, tok, 12, stream=cuda.cuda.Stream())
+    assert cuda.equal(a2, pa) and cuda.equal(b2, pb)
