@@ -389,3 +389,53 @@ def test_prefix_outputs_in_either_memory(R, cuda, libreset):
     assert calls == [4 * pa.numel()] * 3
     a2, b2 = R.prefix_candidates(off, tok, 12, stream=cuda.cuda.Stream())
     assert cuda.equal(a2, pa) and cuda.equal(b2, pb)
+
+
+# -------------------------------------------------------------- retrieval --
+
+@pytest.mark.parametrize("hier,bucket", [(True, 5), (False, 1)])
+@pytest.mark.parametrize("ascending", [True, False])
+def test_retrieval_list_and_query_sizes(R, cuda, hier, bucket, ascending):
+    """Lists around a row of lanes, the keys of a warp's step and a slice;
+    queries of one term up to more than a warp's lanes hold."""
+    rng = np.random.default_rng(bucket)
+    dfs = [0, 1, 31, 32, 33, 255, 256, 257, 511, 512, 513, 1024, 1025, 2900, 2999, 3000]
+    rows = [rng.choice(3000, d, replace=False) for d in dfs]
+    rows = [np.sort(r) if ascending else r for r in rows]
+    off, docs = csr(rows)
+    d_off, d_docs = dev(off, cuda), dev(docs, cuda)
+    t = R.Table(d_off, d_docs, hierarchical=hier, bucket=bucket)
+    queries = [[]]
+    for first in range(len(rows)):
+        for more in [0, 1, 2, 5]:
+            queries.append([first, *rng.integers(0, len(rows), more)])
+        for more in [31, 32, 33, 40]:  # long ones that leave something over
+            queries.append([first, *rng.integers(13, len(rows), more)])
+    qoff, query = csr(queries)
+    roff, res, cnt = R.ir(t, d_off, d_docs, dev(query, cuda), dev(qoff, cuda))
+    roff, res, cnt = (x.cpu().numpy() for x in (roff, res, cnt))
+    for q, terms in enumerate(queries):
+        want = rows[terms[0]] if terms else np.empty(0, int)
+        for term in terms[1:]:
+            want = want[np.isin(want, rows[term])]
+        got = res[roff[q]:roff[q + 1]]
+        assert cnt[q] == len(want) and np.array_equal(got[: len(want)], want)
+        assert (got[len(want):] == -1).all()
+
+
+def test_retrieval_of_many_slices(R, cuda):
+    """More slices than one block's share of the scan, the last one partial."""
+    n = 3 * 16384 * 512 // 2 + 77
+    rows = [cuda.arange(0, n, dtype=cuda.int32), cuda.arange(0, n, 3, dtype=cuda.int32),
+            cuda.arange(0, n, 1000, dtype=cuda.int32)]
+    off = cuda.tensor(np.cumsum([0] + [r.numel() for r in rows]), dtype=cuda.int32)
+    rows = [r.cuda() for r in rows]
+    off, docs = off.cuda(), cuda.cat(rows)
+    t = R.Table(off, docs)
+    query = cuda.tensor([0, 1, 0, 1, 0, 2, 0, 2], dtype=cuda.int32).cuda()
+    qoff = cuda.tensor([0, 2, 3, 5, 7, 8], dtype=cuda.int32).cuda()
+    roff, res, cnt = R.ir(t, off, docs, query, qoff)
+    for q, want in enumerate([rows[1], rows[0], rows[1], rows[2], rows[2]]):
+        got = res[int(roff[q]):int(roff[q + 1])]
+        assert int(cnt[q]) == want.numel() and cuda.equal(got[: want.numel()], want)
+        assert bool((got[want.numel():] == -1).all())
