@@ -37,13 +37,15 @@
 // candidate just picked (N(m_a) ∩ N(x)) is not entered either: such
 // intersections of at most kLaneMax keys run one candidate per lane, longer
 // ones by the whole warp, as AND + popcount over the two bit rows where that
-// is less work than looking up the shorter row's keys.  A reusing
+// is less work than looking up the shorter row's keys; without a bound, on up
+// to 8192 vertices, the sizes of all such intersections are computed first
+// (codegree_kernel) and a candidate costs a load.  A reusing
 // k-clique chain without checks (SMOG's Q0, Q3, Q5, Q7) runs the k-clique
 // count (clique.cu).
 //
 // Bound by instruction issue and, on small graphs, by the longest part.
 // Against one edge per warp with every lookup a hash probe (R-MAT, ms):
-// Q6 scale 8 / 11: 3.2 / 116 -> 0.26 / 3.6; Q4 scale 8 / 13: 0.57 / 19.8 ->
+// Q6 scale 8 / 11: 3.2 / 116 -> 0.16 / 0.79; Q4 scale 8 / 13: 0.57 / 19.8 ->
 // 0.15 / 4.8; Q8 scale 13: 20.6 -> 3.7; Q1 scale 8 / 14: 0.16 / 16.3 ->
 // 0.12 / 6.5; Q2 scale 14: 11.9 -> 3.1.
 //
@@ -171,28 +173,96 @@ __device__ __forceinline__ int first_set(const PatternDev& p, int du, int dv) {
   return s;
 }
 
-// Start edges with a first set above `part` keys, as (u, v, i, parts).
+// Start edges with a first set above `part` keys, as (u, v, i, parts), and
+// the sum of these sets' squares.
 __global__ void pattern_parts_kernel(const int4* __restrict__ desc,
                                      const int32_t* __restrict__ cols, int32_t n, int64_t m,
                                      const PatternDev pat, int part, int4* __restrict__ list,
-                                     int32_t* __restrict__ n_list) {
+                                     int32_t* __restrict__ n_list,
+                                     unsigned long long* __restrict__ squares) {
   const int lane = threadIdx.x & 31;
+  unsigned long long sum = 0;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t u = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; u < n; u += nw) {
     const int4 du = __ldg(desc + u);
     if (du.y <= part) continue;
     const int d = (int)min((int64_t)du.y, m - du.x);
-    for (int j = lane; j < d; j += 32) {
-      const int v = __ldg(cols + du.x + j);
+    for (int j = lane; j - lane < d; j += 32) {
+      const int v = j < d ? __ldg(cols + du.x + j) : -1;
       const int map[2] = {(int)u, v};
-      if ((unsigned)v >= (unsigned)n || !level_ok(pat, 1, v, map)) continue;
-      const int s = first_set(pat, du.y, __ldg(&desc[v].y));
-      if (s <= part) continue;
-      const int np = (s + part - 1) / part;
-      const int at = atomicAdd(n_list, np);
+      int s = 0;
+      if ((unsigned)v < (unsigned)n && level_ok(pat, 1, v, map))
+        s = first_set(pat, du.y, __ldg(&desc[v].y));
+      const int np = s > part ? (s + part - 1) / part : 0;
+      int total;
+      const int before = warp_excl_scan(np, &total);
+      if (total == 0) continue;
+      int at = lane == 0 ? atomicAdd(n_list, total) : 0;
+      at = __shfl_sync(kFull, at, 0) + before;
       for (int i = 0; i < np; ++i) list[at + i] = make_int4((int)u, v, i, np);
+      if (np) sum += (unsigned long long)s * s;
     }
   }
+  sum = warp_sum_u64(sum);
+  if (lane == 0 && sum) atomicAdd(squares, sum);
+}
+
+// Co-degrees |N(a) ∩ N(x)| of all pairs of vertices, from the bit rows: where
+// the paired last level has no bound, its count for a candidate x is one of
+// them, less the earlier vertices, and a visit costs a load where it took the
+// AND of two bit rows by the whole warp.  The matrix takes n^3 / 64 word
+// steps, a walk visits some part of the sum of the squared first sets: the
+// matrix is filled (and used) where that sum times kCoVisits reaches n^3, on
+// the device, since the sum is found there.  Popcounts bound
+// the matrix (n = 2048: 44 us).  Q6 on R-MAT graphs, ms a call, by ANDs / by
+// co-degrees: scale 11 3.41 / 0.79, scale 13 62.8 / 6.9 (268 MB of matrix);
+// scale 8, whose matrix is nothing, 0.26 / 0.16.
+constexpr unsigned long long kCoVisits = 1024;
+constexpr int kCoTile = 64;  // vertices on a side of a block's tile
+constexpr int kCoWords = 32;
+
+__device__ __forceinline__ bool co_used(const unsigned long long* squares, int64_t n) {
+  return *squares * kCoVisits >= (unsigned long long)(n * n * n);
+}
+
+__global__ void __launch_bounds__(256)
+    codegree_kernel(const uint32_t* __restrict__ bits, int32_t n, int words,
+                    const unsigned long long* __restrict__ squares, int32_t* __restrict__ co) {
+  if (!co_used(squares, n)) return;
+  const int i0 = blockIdx.y * kCoTile, j0 = blockIdx.x * kCoTile;
+  if (i0 > j0) return;  // the tile below the diagonal is written with its mirror
+  __shared__ uint32_t sa[kCoTile][kCoWords + 1], sb[kCoTile][kCoWords + 1];
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  int acc[4][4] = {};
+  for (int w0 = 0; w0 < words; w0 += kCoWords) {
+    __syncthreads();
+    for (int t = threadIdx.x; t < kCoTile * kCoWords; t += 256) {
+      const int r = t / kCoWords, w = t % kCoWords;
+      const bool in = w0 + w < words;
+      sa[r][w] = in && i0 + r < n ? __ldg(bits + (int64_t)(i0 + r) * words + w0 + w) : 0;
+      sb[r][w] = in && j0 + r < n ? __ldg(bits + (int64_t)(j0 + r) * words + w0 + w) : 0;
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int w = 0; w < kCoWords; ++w) {
+      uint32_t a[4], b[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i] = sa[ty + 16 * i][w], b[i] = sb[tx + 16 * i][w];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] += __popc(a[i] & b[j]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int64_t y = i0 + ty + 16 * i, x = j0 + tx + 16 * j;
+      if (y >= n || x >= n) continue;
+      co[y * n + x] = acc[i][j];
+      co[x * n + y] = acc[i][j];
+    }
 }
 
 template <bool HIER>
@@ -201,7 +271,9 @@ __global__ void __launch_bounds__(kPtThreads, 4)
                    const int32_t* __restrict__ cols, const int32_t* __restrict__ chunk_row,
                    int32_t n, int64_t m, const int32_t* __restrict__ table, int64_t bn, int b,
                    int lg_max, const PatternDev pat, int sorted, const BitRows br,
-                   const int32_t* __restrict__ loops, const int4* __restrict__ parts_list,
+                   const int32_t* __restrict__ loops, const int32_t* __restrict__ co,
+                   const unsigned long long* __restrict__ squares,
+                   const int4* __restrict__ parts_list,
                    const int32_t* __restrict__ n_list, int part, int lg_grab,
                    int32_t* __restrict__ scratch, int32_t cap,
                    unsigned long long* __restrict__ count,
@@ -221,6 +293,7 @@ __global__ void __launch_bounds__(kPtThreads, 4)
   const int n_parts = part > 0 ? *n_list : 0;
   // no row holds its own vertex (known where bit rows were set)
   const bool loop_free = br.bits && *loops == 0;
+  const bool have_co = co && co_used(squares, n);
   unsigned long long hits = 0;
   // level l: m_l, its index in C_l, C_l (cs, sz), the next candidate (it)
   int map[kPatMax], idx[kPatMax], sz[kPatMax], it[kPatMax];
@@ -404,6 +477,26 @@ __global__ void __launch_bounds__(kPtThreads, 4)
               in = in && da.y > 0 && holds(ba, da, map[lane]);
             }
             in_a = __ballot_sync(kFull, in);
+          }
+          if (have_co) {  // (ascending rows, no bound, bit rows of all vertices)
+            const int32_t* co_a = co + (int64_t)ma * n;
+            for (int j = it[lv] + lane; j < end; j += 32) {
+              const int x = cs[lv][j];  // (in [0, n): bit rows)
+              if (!level_ok(sp, lv, x, map)) continue;
+              int c2 = __ldg(co_a + x);
+              if (dist && c2 > 0) {
+                const uint32_t* bx = br.of(x);
+                for (unsigned q = in_a; q; q &= q - 1) c2 -= bit_of(bx, map[__ffs(q) - 1]);
+                if (!loop_free && bit_of(bx, x)) {
+                  bool seen = false;
+                  for (int q = 0; q < lv; ++q) seen |= map[q] == x;
+                  if (!seen && bit_of(ba, x)) --c2;
+                }
+              }
+              hits += c2;
+            }
+            --lv;
+            continue;
           }
           for (int j0 = it[lv]; j0 < end; j0 += 32) {
             const int j = j0 + lane;
@@ -798,9 +891,11 @@ extern "C" reset_status reset_pattern_count(const reset_table* t, const int32_t*
   uint32_t* bits = reinterpret_cast<uint32_t*>(base + sz_scr);
   int32_t* row = reinterpret_cast<int32_t*>(base + sz_scr + sz_bits);
   int4* list = reinterpret_cast<int4*>(base + sz_scr + sz_bits + sz_row);
-  // [0..1] work cursors (u64), then the listed parts, self-loops, bit rows
+  // [0..1] work cursors, the parts' squares (u64), then the listed parts,
+  // self-loops, bit rows
   auto* cursor = reinterpret_cast<unsigned long long*>(base + sz_scr + sz_bits + sz_row + sz_list);
-  int32_t* ctr = reinterpret_cast<int32_t*>(cursor + 2);
+  auto* squares = cursor + 2;
+  int32_t* ctr = reinterpret_cast<int32_t*>(cursor + 3);
   const int warp_grid = (int)std::min<int64_t>(((int64_t)t->n + 7) / 8, (int64_t)sms * 8);
   cudaError_t e = cudaMemsetAsync(cursor, 0, 256, st);
   if (e == cudaSuccess && bit_rows > 0) {
@@ -822,20 +917,38 @@ extern "C" reset_status reset_pattern_count(const reset_table* t, const int32_t*
   if (e == cudaSuccess && part > 0) {
     note_launch();
     pattern_parts_kernel<<<warp_grid, 256, 0, st>>>(t->d_desc, d_cols, t->n, m, pat, part, list,
-                                                    ctr);
+                                                    ctr, squares);
     e = cudaGetLastError();
+  }
+  // co-degrees, where the paired last level has no bound; without memory for
+  // them the walk does as well
+  const bool bounded = (pat.flags & RESET_PATTERN_RESTRICT) && pat.restr[pat.k - 1] >= 0;
+  const int64_t co_bytes = (int64_t)sizeof(int32_t) * t->n * t->n;
+  int32_t* co = nullptr;
+  if (e == cudaSuccess && pat.pair && sorted && !bounded && bit_rows == t->n &&
+      co_bytes <= kBitBudget) {
+    if (scratch_malloc(reinterpret_cast<void**>(&co), (size_t)co_bytes, st) != cudaSuccess) {
+      cudaGetLastError();
+      co = nullptr;
+    } else {
+      const unsigned tiles = (unsigned)((t->n + kCoTile - 1) / kCoTile);
+      note_launch();
+      codegree_kernel<<<dim3(tiles, tiles), 256, 0, st>>>(bits, t->n, (int)br.words, squares, co);
+      e = cudaGetLastError();
+    }
   }
   if (e == cudaSuccess) {
     note_launch();
 #define PT_LAUNCH(H)                                                                           \
   pattern_kernel<H><<<(int)grid, kPtThreads, 0, st>>>(                                         \
       t->d_desc, d_off, d_cols, t->d_chunk_row, t->n, m, t->d_table, t->bucket_num, t->bucket, \
-      t->lg_max, pat, sorted, br, ctr + 1, list, ctr, part, lg_grab, scr, cap,                 \
+      t->lg_max, pat, sorted, br, ctr + 1, co, squares, list, ctr, part, lg_grab, scr, cap,    \
       reinterpret_cast<unsigned long long*>(d_count), cursor, t->d_status)
     if (t->hier) PT_LAUNCH(true); else PT_LAUNCH(false);
 #undef PT_LAUNCH
     e = cudaGetLastError();
   }
+  if (co) cudaFreeAsync(co, st);
   cudaFreeAsync(base, st);
   if (e != cudaSuccess) return cuda_fail(e, "pattern_kernel", __FILE__, __LINE__);
   return RESET_OK;

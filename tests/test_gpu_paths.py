@@ -122,6 +122,24 @@ def test_patterns_on_digraphs(R, cuda, oracle_mod, n, density, loops):
     t.check()
 
 
+@pytest.mark.parametrize("n", [63, 64, 65, 127, 129, 1030])
+def test_codegree_tiles(R, cuda, oracle_mod, n):
+    """Vertex counts around the tiles of the co-degree matrix and the words
+    staged at a time; a dense core among vertices that have few neighbours."""
+    rng = np.random.default_rng(n)
+    core = rng.random((n, n)) < np.where(np.arange(n) < (60 if n < 200 else 12), 0.5, 2 / n)[:, None]
+    core[-1, : n // 2] = True
+    adj = np.triu(core, 1)
+    adj |= adj.T
+    off, cols = csr([np.flatnonzero(r) for r in adj])
+    d_off, d_cols = dev(off, cuda), dev(cols, cuda)
+    t = R.Table(d_off, d_cols)
+    for name in ("Q6", "pair_distinct"):
+        p = _patterns(R)[name]
+        assert R.pattern_count(t, d_off, d_cols, p) == _oracle_pattern(oracle_mod, off, cols, p), name
+    t.check()
+
+
 def test_patterns_with_bit_rows_for_hubs_only(R, cuda, oracle_mod):
     """More vertices than a whole bit matrix takes: the long rows have bit
     rows, the others are probed in their tables."""
