@@ -25,7 +25,7 @@
 // once, where a group's probers bring hundreds of keys per slot.
 //
 // Passes (all stream-ordered, no host synchronisation):
-//   pad_*_kernel        the key rows padded to whole 32-byte chunks
+//   pad_rows_kernel     the key rows padded to whole 32-byte chunks
 //   own_count_kernel    owner of every edge; probers per owner
 //   CUB exclusive scan  group offsets
 //   own_scatter_kernel  (first chunk, keys) of every edge's prober,
@@ -169,23 +169,20 @@ __global__ void __launch_bounds__(kOT)
     cls[u] = s_c[deg_step(indeg[u] + __ldg(koff + u + 1) - __ldg(koff + u))];
 }
 
-// Chunks of every key row (pst, scanned in place afterwards), and a chunk
-// without keys at `none`.
-__global__ void __launch_bounds__(kOT)
-    pad_count_kernel(const int32_t* __restrict__ koff, int32_t n, int32_t* __restrict__ pst,
-                     int32_t* __restrict__ none) {
-  if (blockIdx.x == 0 && threadIdx.x < 8) none[threadIdx.x] = kNoKey;
-  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u <= n;
-       u += (int64_t)gridDim.x * blockDim.x)
-    pst[u] = u < n ? (max(__ldg(koff + u + 1) - __ldg(koff + u), 0) + 7) >> 3 : 0;
+// The first chunk of the padded row u, whose keys start at s: rows start at
+// least a chunk per 8 keys and one more apart, so no scan over the rows is
+// needed (three launches, 12 of 264 us at scale 16), for at most n chunks in all.
+__device__ __forceinline__ unsigned first_chunk(int s, int u, int64_t mk) {
+  return ((unsigned)min((int64_t)max(s, 0), mk) >> 3) + (unsigned)u;
 }
 
 // The padded rows, 8 lanes to a row, in class order with their lowest class
-// and class places (cls NULL: in the order they come).
+// and class places (cls NULL: in the order they come); a chunk without keys at
+// `none`.
 __global__ void __launch_bounds__(kOT)
     pad_rows_kernel(const int32_t* __restrict__ koff, const int32_t* __restrict__ kcols,
-                    int32_t n, int64_t mk, const int32_t* __restrict__ pst,
-                    const uint8_t* __restrict__ cls, int32_t* __restrict__ padded,
+                    int32_t n, int64_t mk, const uint8_t* __restrict__ cls,
+                    int32_t* __restrict__ padded, int32_t* __restrict__ none,
                     unsigned* __restrict__ info, ClassPlaces* __restrict__ places) {
   __shared__ int s_cnt[kOT / 8][kClasses];
   constexpr int kPer = kClasses / 8;  // classes a lane looks after
@@ -194,10 +191,11 @@ __global__ void __launch_bounds__(kOT)
   const unsigned group = 0xffu << (threadIdx.x & 24);
   int* cnt = s_cnt[threadIdx.x >> 3];
   const int64_t step = ((int64_t)gridDim.x * blockDim.x) >> 3;
+  if (blockIdx.x == 0 && threadIdx.x < 8) none[threadIdx.x] = kNoKey;
   for (int64_t u = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3; u < n; u += step) {
-    const int s = __ldg(koff + u), p = __ldg(pst + u);
+    const int s = max(__ldg(koff + u), 0);
     const int d = (int)min((int64_t)(__ldg(koff + u + 1) - s), mk - s);
-    int32_t* out = padded + (int64_t)(unsigned)p * 8;
+    int32_t* out = padded + (int64_t)first_chunk(s, (int)u, mk) * 8;
     int place[kPer];
     int lowest = 0;
     for (int i = 0; i < kPer; ++i) place[i] = 0;
@@ -342,7 +340,7 @@ __global__ void __launch_bounds__(kOT)
     own_scatter_kernel(const int32_t* __restrict__ eoff, const int32_t* __restrict__ ecols,
                        const int32_t* __restrict__ chunk_row, const int32_t* __restrict__ koff,
                        const unsigned* __restrict__ info, int32_t n, int64_t m,
-                       const int32_t* __restrict__ pst,
+                       int64_t mk,
                        const ClassPlaces* __restrict__ places, int32_t* __restrict__ left,
                        int2* __restrict__ ent, int32_t* __restrict__ status) {
   const int lane = threadIdx.x & 31;
@@ -365,7 +363,8 @@ __global__ void __launch_bounds__(kOT)
 #pragma unroll
     for (int i = 0; i < kIlp; ++i) {
       const bool ok = eo.owner[i] >= 0;
-      row[i] = make_int2(ok ? __ldg(pst + eo.prober[i]) : 0, eo.len[i]);
+      row[i] = make_int2(
+          ok ? (int)first_chunk(__ldg(koff + eo.prober[i]), eo.prober[i], mk) : 0, eo.len[i]);
       const int from = ok && eo.low[i] ? __ldg(&places[eo.prober[i]].at[eo.low[i]]) : 0;
       row[i].x += from;
       row[i].y -= 8 * from;
@@ -811,8 +810,7 @@ reset_status tc_owner(const reset_table* t, const int4* kdesc, const int32_t* ko
   if (mk > INT32_MAX - 16)
     return arg_fail("the owner-grouped count takes at most 2^31 - 17 keys");
   if (n == INT32_MAX) return arg_fail("the owner-grouped count takes at most 2^31 - 2 sets");
-  // scratch, one allocation: cnt/left, goff, ent, units, wlist, dlist, dunits,
-  // ctr, CUB
+  // scratch, one allocation
   size_t cub_bytes = 0;
   RST_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, (int32_t*)nullptr,
                                          (int32_t*)nullptr, (int)(n + 1), st));
@@ -822,11 +820,10 @@ reset_status tc_owner(const reset_table* t, const int4* kdesc, const int32_t* ko
   const size_t sz_ent = al(sizeof(int2) * m), sz_units = al(sizeof(int2) * max_units);
   const size_t sz_list = al(sizeof(int32_t) * n), sz_ctr = al(sizeof(int32_t) * 8);
   const size_t sz_dunits = al(sizeof(int2) * max_dunits);
-  // padded rows: up to 7 keys more for every row with keys (at most the size
-  // of the table, whose rows hold at least 8 slots)
-  const int64_t pad_chunks = (mk + 7 * std::min(n, mk) + 7) / 8;
+  // padded rows: a chunk more for every row (at most the size of the table,
+  // whose rows hold at least 8 slots), and one without keys
+  const int64_t pad_chunks = mk / 8 + n + 1;
   const size_t sz_pad = al(8 * sizeof(int32_t) * (size_t)(pad_chunks + 1));
-  const size_t sz_pst = al(sizeof(int32_t) * ((size_t)n + 1));
   // classes need the rows to be the sets of the tables (the CSR they were
   // built on), and pay on more edges than the passes cost
   const bool classes = koff == t->build_off && mk == t->m && mk >= kClassEdges;
@@ -835,20 +832,19 @@ reset_status tc_owner(const reset_table* t, const int4* kdesc, const int32_t* ko
   const size_t sz_cls = classes ? al((size_t)n) : 0;
   const size_t sz_places = classes ? al(sizeof(ClassPlaces) * (size_t)n) : 0;
   const size_t total = sz_cnt + sz_goff + sz_ent + sz_units + 2 * sz_list + sz_dunits +
-                       sz_ctr + sz_pad + sz_pst + sz_info + sz_deg + sz_cls + sz_places + al(cub_bytes);
+                       sz_ctr + sz_pad + sz_info + sz_deg + sz_cls + sz_places + al(cub_bytes);
   char* base = nullptr;
   RST_CUDA(scratch_malloc(reinterpret_cast<void**>(&base), total, st));
   char* p = base;
   int32_t* cnt = reinterpret_cast<int32_t*>(p); p += sz_cnt;
+  int32_t* ctr = reinterpret_cast<int32_t*>(p); p += sz_ctr;
   int32_t* goff = reinterpret_cast<int32_t*>(p); p += sz_goff;
   int2* ent = reinterpret_cast<int2*>(p); p += sz_ent;
   int2* units = reinterpret_cast<int2*>(p); p += sz_units;
   int32_t* wlist = reinterpret_cast<int32_t*>(p); p += sz_list;
   int32_t* dlist = reinterpret_cast<int32_t*>(p); p += sz_list;
   int2* dunits = reinterpret_cast<int2*>(p); p += sz_dunits;
-  int32_t* ctr = reinterpret_cast<int32_t*>(p); p += sz_ctr;
   int32_t* padded = reinterpret_cast<int32_t*>(p); p += sz_pad;
-  int32_t* pst = reinterpret_cast<int32_t*>(p); p += sz_pst;
   int32_t* indeg = reinterpret_cast<int32_t*>(p); p += sz_deg;
   unsigned* hist = reinterpret_cast<unsigned*>(indeg + n);
   uint8_t* cls = classes ? reinterpret_cast<uint8_t*>(p) : nullptr; p += sz_cls;
@@ -856,8 +852,7 @@ reset_status tc_owner(const reset_table* t, const int4* kdesc, const int32_t* ko
   ClassPlaces* places = reinterpret_cast<ClassPlaces*>(p); p += sz_places;
   void* cub_tmp = p;
 
-  cudaError_t e = cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (n + 1), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(ctr, 0, sizeof(int32_t) * 8, st);
+  cudaError_t e = cudaMemsetAsync(cnt, 0, sz_cnt + sz_ctr, st);
   const int sms = sm_count();
   const int64_t chunks = (m + 31) / 32;
   const int g_edges = grid_stride_blocks((chunks + kOW * kIlp - 1) / (kOW * kIlp), sms * 8);
@@ -875,16 +870,8 @@ reset_status tc_owner(const reset_table* t, const int4* kdesc, const int32_t* ko
   }
   if (e == cudaSuccess) {
     note_launch();
-    pad_count_kernel<<<grid_stride_blocks((n + kOT) / kOT, sms * 8), kOT, 0, st>>>(
-        koff, t->n, pst, padded + pad_chunks * 8);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess)
-    e = cub::DeviceScan::ExclusiveSum(cub_tmp, cub_bytes, pst, pst, (int)(n + 1), st);
-  if (e == cudaSuccess) {
-    note_launch();
     pad_rows_kernel<<<grid_stride_blocks((n * 8 + kOT - 1) / kOT, sms * 16), kOT, 0, st>>>(
-        koff, kcols, t->n, mk, pst, cls, padded, info, places);
+        koff, kcols, t->n, mk, cls, padded, padded + pad_chunks * 8, info, places);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) {
@@ -900,7 +887,7 @@ reset_status tc_owner(const reset_table* t, const int4* kdesc, const int32_t* ko
   if (e == cudaSuccess) {
     note_launch();
     own_scatter_kernel<<<g_edges, kOT, 0, st>>>(eoff, ecols, echunk_rows, koff, info, t->n, me,
-                                                pst, places, cnt, ent, t->d_status);
+                                                mk, places, cnt, ent, t->d_status);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) {
