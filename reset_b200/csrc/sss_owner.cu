@@ -158,8 +158,8 @@ __global__ void __launch_bounds__(kOT, 2)
   auto batch = [&](int g, int c, const int* S, int lg, int dw) {
     C[lane] = 0;
     __syncwarp();
-    staged_keys<HIER, R, true>(ent + g, c, elems, m, S, lg, lg_max, b, status, s_qx[warp],
-                               s_qh[warp], C);
+    staged_keys<HIER, R>(ent + g, c, elems, m, S, lg, lg_max, b, status, s_qx[warp],
+                         s_qh[warp], C);
     __syncwarp();
     if (lane < c)
       decide<FLOAT_RULE>(__ldg(pidx + g + lane), C[lane], __ldg(&ent[g + lane].y), dw, num,

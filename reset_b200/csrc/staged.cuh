@@ -1,8 +1,9 @@
-// Device helpers of the owner-grouped probe kernels (tc_owner.cu,
-// sss_owner.cu): 1-D bulk copies of a set's table into shared memory
-// (cp.async.bulk completing on an mbarrier, with bounded waits), the
-// reference probe rule walked in the staged copy, and the flattened 16-byte
-// key streaming of up to 32 probing rows against one staged table.
+// Device helpers of the owner-grouped similarity kernel (sss_owner.cu): 1-D
+// bulk copies of a set's table into shared memory (cp.async.bulk completing
+// on an mbarrier, with bounded waits), the reference probe rule walked in the
+// staged copy, and the flattened 16-byte key streaming of up to 32 probing
+// rows against one staged table.  The triangle count (tc_owner.cu) shares the
+// launch shape and the direct bin.
 #pragma once
 
 #include "common.cuh"
@@ -16,8 +17,7 @@ constexpr int kWaitLimit = 1 << 22;  // polls of a bulk-copy barrier before givi
 constexpr int kOT = 512;                 // threads per CTA (2 CTAs, 32 warps per SM)
 constexpr int kOW = kOT / 32;            // warps per CTA
 // Ints of shared memory per CTA for staged tables (80 KB): every power-of-two
-// plane size with b = 1, 2, 4 or 5 slots that 96 KB held still fits, and the
-// 16 KB saved doubles the pending-probe queues of the triangle count.
+// plane size with b = 1, 2, 4 or 5 slots that 96 KB would hold fits as well.
 constexpr int kCtaTab = 20480;
 constexpr int kWarpTab = kCtaTab / kOW;  // a warp's region (1280 ints)
 constexpr int kCtaSeg = 8192;            // probers per CTA work unit
@@ -194,88 +194,31 @@ __device__ __forceinline__ bool stage_wait(uint64_t* bar, uint32_t parity, int* 
   return ok;
 }
 
-// Walks queued keys q[0, nq) of one staged table (all lanes, nq
-// warp-uniform): each key's first two probe slots held other keys, so its
-// walk resumes after them -- slot 2 of its home bucket, or with one slot per
-// bucket the bucket after the next.  Returns this lane's hits.
-template <bool HIER>
-__device__ __forceinline__ unsigned walk_keys(const int* q, int nq, const int* S, int lg,
-                                              int lg_max, int b, int32_t* status) {
-  const int lane = threadIdx.x & 31;
-  const int L = 1 << lg;
-  const unsigned hmask = HIER ? ((1u << lg_max) - 1u) : (unsigned)(L - 1);
-  const int hsh = HIER ? (lg_max - lg) : 0;
-  const int inc1 = b > 1 ? 0 : 1;
-  const int kcont = b > 1 ? 2 : 1;
-  unsigned hits = 0;
-  __syncwarp();
-  for (int i = lane; i < nq; i += 32) {
-    const int x = q[i];
-    const int h = (int)(((unsigned)x & hmask) >> hsh);
-    hits += smem_walk(x, S, L, h + inc1, kcont, b, status);
-  }
-  __syncwarp();
-  return hits;
-}
-
-// Largest lane k < NR with P_k <= f (P nondecreasing across lanes, P_0 = 0;
-// every row at or past NR is empty).
-template <int NR>
-__device__ __forceinline__ int owner_lane_n(int P, int f) {
-  int k = 0;
-#pragma unroll
-  for (int step = NR / 2; step >= 1; step >>= 1) {
-    const int pk = __shfl_sync(kFull, P, k + step);
-    if (pk <= f) k += step;
-  }
-  return k;
-}
-
-// The keys of up to NR probing rows (NR a power of two <= 32; lane i:
-// ent[i] = {row start, row length} in cols) looked up in one staged table
-// (plane k at S + k*L; with b = 1 padded by stage_wait).  The rows' 16-byte
-// chunks are flattened across the lanes (round r: lane i loads chunk 32r+i
-// of the concatenation, its row found by a shuffle binary search over the NR
-// rows) and R rounds are in flight at once.  Elements of a chunk outside its
-// row become the sentinel -2, which matches no slot (keys are >= 0, empty
+// The keys of up to 32 probing rows (lane i: ent[i] = {row start, row length}
+// in cols) looked up in one staged table (plane k at S + k*L; with b = 1
+// padded by stage_wait); the hits of row i are added to s_cnt[i] (32
+// shared-memory counters of this warp, zeroed by the caller).  The rows'
+// 16-byte chunks are flattened across the lanes (round r: lane i loads chunk
+// 32r+i of the concatenation, its row found by a shuffle binary search over
+// the rows) and R rounds are in flight at once.  Elements of a chunk outside
+// its row become the sentinel -2, which matches no slot (keys are >= 0, empty
 // slots -1), so every element is probed without a validity test.  Every
 // key's first two probe slots (slots 0 and 1 of its home bucket; with one
 // slot per bucket, the home and next bucket) are read and resolved without
 // branching; probes that both slots leave open are queued in this warp's
-// shared-memory queue (qx, qh: QCAP entries each, QCAP >= kQueue) and walked
-// by all lanes together once more than QCAP - kQueue are pending (and before
-// returning), so the rare long walks neither idle the warp nor run with few
-// lanes.  Returns this lane's hits; with PAIRS, the hits of row i are also
-// added to s_cnt[i] (32 shared-memory counters of this warp, zeroed by the
-// caller).
-//
-// KEEP (counting only): the queue holds keys alone (their walk restarts from
-// the hash) and outlives the call: *nq_keep carries its length from call to
-// call over one staged table, and the caller walks the rest with walk_keys
-// before the table changes.
-//
-// PF: the next R chunks of keys are loaded before the current ones are
-// probed (software pipelining across rounds).
-//
-// CW: keys per lane and round (4: one 16-byte load; 8: two, so the row
-// search and chunk bookkeeping are paid once per 8 keys).
-template <bool HIER, int R, bool PAIRS = false, int NR = 32, int QCAP = kQueue,
-          bool KEEP = false, bool PF = false, int CW = 4>
-__device__ __forceinline__ unsigned staged_keys(const int2* __restrict__ ent, int cnt,
-                                                const int32_t* __restrict__ cols, int64_t m,
-                                                const int* S, int lg, int lg_max, int b,
-                                                int32_t* status, int* qx, int* qh,
-                                                int* s_cnt = nullptr, int* nq_keep = nullptr) {
-  static_assert(NR >= 1 && NR <= 32 && (NR & (NR - 1)) == 0, "NR: a power of two <= 32");
-  static_assert(CW == 4 || CW == 8, "chunks of 4 or 8 keys");
-  static_assert(QCAP >= 32 * CW, "the queue must hold one round");
-  constexpr int kShift = CW == 8 ? 3 : 2;
-  static_assert(!(KEEP && PAIRS), "a kept queue carries no rows");
+// shared-memory queue (qx, qh: kQueue entries each) and walked by all lanes
+// together after each round, so the rare long walks neither idle the warp
+// nor run with few lanes.
+template <bool HIER, int R>
+__device__ __forceinline__ void staged_keys(const int2* __restrict__ ent, int cnt,
+                                            const int32_t* __restrict__ cols, int64_t m,
+                                            const int* S, int lg, int lg_max, int b,
+                                            int32_t* status, int* qx, int* qh, int* s_cnt) {
   const int lane = threadIdx.x & 31;
   const unsigned lt = lanemask_lt();
   const int2 e = lane < cnt ? __ldg(ent + lane) : make_int2(0, 0);
   const int64_t end = (int64_t)e.x + e.y;
-  const int nc = e.y > 0 ? (int)(((end + CW - 1) >> kShift) - (e.x >> kShift)) : 0;
+  const int nc = e.y > 0 ? (int)(((end + 3) >> 2) - (e.x >> 2)) : 0;
   int total;
   const int P = warp_excl_scan(nc, &total);
   const int L = 1 << lg;
@@ -288,80 +231,53 @@ __device__ __forceinline__ unsigned staged_keys(const int2* __restrict__ ent, in
   const int inc1 = b > 1 ? 0 : 1;
   const int kcont = b > 1 ? 2 : 1;
   const int4* __restrict__ cols4 = reinterpret_cast<const int4*>(cols);
-  const int64_t full = m >> kShift;  // chunks that lie wholly inside cols
-  unsigned hits = 0;
-  int nq = KEEP ? *nq_keep : 0;  // queued probes (warp-uniform)
-  auto walk_queue = [&]() {
-    if (KEEP) {
-      hits += walk_keys<HIER>(qx, nq, S, lg, lg_max, b, status);
-      nq = 0;
-      return;
-    }
-    __syncwarp();
-    for (int i = lane; i < nq; i += 32) {
-      const int v = qh[i];
-      const unsigned hit = smem_walk(qx[i], S, L, v >> 10, (v >> 5) & 31, b, status);
-      if (PAIRS) {
-        if (hit) atomicAdd(s_cnt + (v & 31), 1);
-      } else {
-        hits += hit;
-      }
-    }
-    __syncwarp();
-    nq = 0;
-  };
-  // Loads the R chunks of rounds [base, base + 32R) of this lane: keys in
-  // x (-2 outside rows), rows in kk (-1 if none).
-  auto load = [&](int base, int (&x)[R][CW], int (&kk)[R]) {
+  const int64_t full = m >> 2;  // chunks that lie wholly inside cols
+  int nq = 0;  // queued probes (warp-uniform)
+  for (int base = 0; base < total; base += 32 * R) {
+    int x[R][4], kk[R];  // keys (-2 outside rows), rows (-1 if none)
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       kk[r] = -1;
 #pragma unroll
-      for (int j = 0; j < CW; ++j) x[r][j] = -2;
+      for (int j = 0; j < 4; ++j) x[r][j] = -2;
       if (base + r * 32 < total) {  // warp-uniform
         const int f = base + r * 32 + lane;
-        const int k = owner_lane_n<NR>(P, f);
+        const int k = owner_lane(P, f);
         const int kp = __shfl_sync(kFull, P, k);
         const int kb = __shfl_sync(kFull, e.x, k);
         const int kd = __shfl_sync(kFull, e.y, k);
         if (f < total) {
           kk[r] = k;
-          // m <= 2^31 - 16 (checked on the host): CW*c + CW - 1 fits an int
-          const int c = (kb >> kShift) + (f - kp);
-          const int i0 = c * CW;
+          // m <= 2^31 - 16 (checked on the host): 4*c + 3 fits an int
+          const int c = (kb >> 2) + (f - kp);
+          const int i0 = c * 4;
           const int lo = kb - i0;       // elements j < lo precede the row
           const int hi = kb + kd - i0;  // elements j >= hi follow it
           if (c < full) {
-#pragma unroll
-            for (int v = 0; v < CW / 4; ++v) {
-              const int4 q = __ldg(cols4 + (CW / 4) * c + v);
-              x[r][4 * v + 0] = q.x;
-              x[r][4 * v + 1] = q.y;
-              x[r][4 * v + 2] = q.z;
-              x[r][4 * v + 3] = q.w;
-            }
+            const int4 q = __ldg(cols4 + c);
+            x[r][0] = q.x;
+            x[r][1] = q.y;
+            x[r][2] = q.z;
+            x[r][3] = q.w;
           } else {
 #pragma unroll
-            for (int j = 0; j < CW; ++j)
+            for (int j = 0; j < 4; ++j)
               if (j >= lo && j < hi) x[r][j] = __ldg(cols + i0 + j);
           }
-          if (lo > 0 || hi < CW) {  // the first or last chunk of its row
+          if (lo > 0 || hi < 4) {  // the first or last chunk of its row
 #pragma unroll
-            for (int j = 0; j < CW; ++j)
+            for (int j = 0; j < 4; ++j)
               if (j < lo || j >= hi) x[r][j] = -2;
           }
         }
       }
     }
-  };
-  // Probes the keys of rounds [base, base + 32R).
-  auto probe = [&](int base, const int (&x)[R][CW], const int (&kk)[R]) {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       if (base + r * 32 >= total) break;  // warp-uniform
       unsigned hr = 0;
 #pragma unroll
-      for (int j = 0; j < CW; ++j) {
+      for (int j = 0; j < 4; ++j) {
         const int xx = x[r][j];
         const int h = (int)(((unsigned)xx & hmask) >> hsh);
         const int s0 = S[h];
@@ -371,50 +287,28 @@ __device__ __forceinline__ unsigned staged_keys(const int2* __restrict__ ent, in
         const unsigned pm = __ballot_sync(kFull, pend);
         if (pend) {
           // continue at slot 2 of the home bucket (or, one slot per bucket,
-          // at the bucket after h + 1); the row rides along for PAIRS
+          // at the bucket after h + 1); the row rides along
           const int pos = nq + __popc(pm & lt);
           qx[pos] = xx;
-          if (!KEEP) qh[pos] = ((h + inc1) << 10) | (kcont << 5) | (kk[r] & 31);
+          qh[pos] = ((h + inc1) << 10) | (kcont << 5) | (kk[r] & 31);
         }
         nq += __popc(pm);
       }
-      if (nq > QCAP - 32 * CW) walk_queue();
-      hits += hr;
-      if (PAIRS) {
-        const unsigned grp = __match_any_sync(kFull, kk[r]);
-        const unsigned sum = __reduce_add_sync(grp, hr);
-        if (kk[r] >= 0 && lane == __ffs(grp) - 1 && sum) atomicAdd(s_cnt + kk[r], (int)sum);
+      if (nq) {
+        __syncwarp();
+        for (int i = lane; i < nq; i += 32) {
+          const int v = qh[i];
+          if (smem_walk(qx[i], S, L, v >> 10, (v >> 5) & 31, b, status))
+            atomicAdd(s_cnt + (v & 31), 1);
+        }
+        __syncwarp();
+        nq = 0;
       }
-    }
-  };
-  if (PF) {
-    // the next R chunks are loaded before this round's keys are probed,
-    // so their latency hides behind the probes
-    int xn[R][CW], kn[R];
-    if (total > 0) load(0, xn, kn);
-    for (int base = 0; base < total; base += 32 * R) {
-      int x[R][CW], kk[R];
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        kk[r] = kn[r];
-#pragma unroll
-        for (int j = 0; j < CW; ++j) x[r][j] = xn[r][j];
-      }
-      if (base + 32 * R < total) load(base + 32 * R, xn, kn);
-      probe(base, x, kk);
-    }
-  } else {
-    for (int base = 0; base < total; base += 32 * R) {
-      int x[R][CW], kk[R];
-      load(base, x, kk);
-      probe(base, x, kk);
+      const unsigned grp = __match_any_sync(kFull, kk[r]);
+      const unsigned sum = __reduce_add_sync(grp, hr);
+      if (kk[r] >= 0 && lane == __ffs(grp) - 1 && sum) atomicAdd(s_cnt + kk[r], (int)sum);
     }
   }
-  if (KEEP)
-    *nq_keep = nq;
-  else if (nq)
-    walk_queue();
-  return hits;
 }
 
 }  // namespace rst

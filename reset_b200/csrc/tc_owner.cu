@@ -19,9 +19,10 @@
 // The staged form of a table is not its copy: the set it holds is inserted
 // into an open-addressing table of 8192 slots (1024 for a warp) with a
 // multiplicative hash, whatever the reference table's load, bucket size and
-// hash.  Almost every lookup is then settled by ONE shared memory read (a copy of the reference table takes two, and with 5-slot
-// buckets one lookup in four goes further), and the count runs at the same
-// speed for every table parameter.  Inserting is cheap: it reads the slots
+// hash.  Almost every lookup is then settled by ONE shared memory read (a copy
+// of the reference table takes two, and with 5-slot buckets one lookup in four
+// goes further), and the count runs at the same speed for every table
+// parameter.  Inserting is cheap: it reads the slots
 // once, where a group's probers bring hundreds of keys per slot.
 //
 // Passes (all stream-ordered, no host synchronisation):
