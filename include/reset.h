@@ -87,7 +87,7 @@ typedef struct reset_table_view {
  * calculate_length (triangle-count/hashtable.cu:21-36) exactly.  Keys are
  * placed by the reference insertion rule (hashtable.cu:53-101) applied in
  * CSR order, so the layout is deterministic.  Synchronises `stream` once
- * (to size the table).  If d_hash_order_out is not NULL it receives, in the
+ * (to size the table), and once more where a set has 2^16 keys or more.  If d_hash_order_out is not NULL it receives, in the
  * same pass, every row read back in bucket order (what
  * launch_extract_hashtable_to_csr, baseline/common/utils.cu:148-175,
  * produces). */
@@ -298,7 +298,7 @@ reset_status reset_ir(const reset_table *t, const int32_t *d_toff,
 /* 4-cliques of an oriented graph (rows sorted ascending, oriented as for
  * reset_tc_count) whose table is `t` (built on d_off/d_cols):
  *   sum over edges (u, v) of sum over w in W of |W ∩ N+(w)|,
- * W = N+(u) ∩ N+(v), every intersection by hash probes.  *d_count (device
+ * W = N+(u) ∩ N+(v): reset_clique_count with k = 4.  *d_count (device
  * u64) is overwritten.  The depth-4 clique search of SMOG's
  * DFSKernelForClique (SMOG/SMOG_hie/subgraph_match_hie.cu:58-247) over this
  * library's tables.  Synchronises `stream` once (scratch sizing). */
@@ -308,12 +308,12 @@ reset_status reset_clique4_count(const reset_table *t, const int32_t *d_off,
 
 /* k-cliques, 3 <= k <= 16, of an oriented graph whose table is `t` (built
  * on d_off/d_cols): SMOG's clique DFS (DFSKernelForClique,
- * SMOG/SMOG_hie/subgraph_match_hie.cu:58-247) with every candidate set
- * C_{j+1} = C_j ∩ N+(w) found by hash probes, starting from
- * C_0 = N+(u) ∩ N+(v) for every edge (u, v); each clique is counted once.
- * k = 3 gives the triangle count, k = 4 the 4-clique count.  *d_count
- * (device u64) is overwritten.  Synchronises `stream` once (scratch
- * sizing: k - 3 rows of the largest out-degree per warp). */
+ * SMOG/SMOG_hie/subgraph_match_hie.cu:58-247) over the candidate sets
+ * C_{j+1} = C_j ∩ N+(w), starting from C_0 = N+(u) ∩ N+(v) for every edge
+ * (u, v); each clique is counted once.  Rows that ascend strictly (sets) are
+ * searched as bit rows of the graph on N+(u), others by hash probes.  k = 3
+ * is reset_tc_count.  *d_count (device u64) is overwritten.  k > 3
+ * synchronises `stream` once (row lengths and order; scratch sizing). */
 reset_status reset_clique_count(const reset_table *t, const int32_t *d_off,
                                 const int32_t *d_cols, int64_t m, int32_t k,
                                 uint64_t *d_count, reset_stream_t stream);
@@ -356,8 +356,9 @@ typedef struct reset_pattern {
  * each level passing its restriction / distinctness check.  SMOG's
  * DFSKernelForGeneral and DFSKernelForClique
  * (SMOG/SMOG_hie/subgraph_match_hie.cu:58-406) as one warp-level DFS per
- * start edge; C_l starts from the smallest listed row (or the reused set)
- * and probes the other listed rows' tables.  Symmetric CSR for general
+ * start edge, long ones cut into parts; C_l starts from the smallest listed
+ * row (or the reused set) and looks its keys up in the other listed rows'
+ * bit rows or tables.  Symmetric CSR for general
  * patterns, oriented for cliques, as the reference loads them
  * (SMOG/SMOG_hie/common_hie.cu:61-85).  Rows in any order; strictly
  * ascending rows take shortcuts (restriction prefixes, counts without a

@@ -650,7 +650,10 @@ reset_status clique_bits(const reset_table* t, const int32_t* d_off, const int32
   const size_t smem = sizeof(uint32_t) * (kCbPack + (size_t)dcap * cb_stride(dcap));
   const void* kf =
       t->hier ? (const void*)clique_bits_kernel<true> : (const void*)clique_bits_kernel<false>;
-  RST_CUDA(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // (the same for every graph: other threads may be between here and a launch)
+  RST_CUDA(cudaFuncSetAttribute(
+      kf, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      (int)sizeof(uint32_t) * (kCbPack + kCbRowMax * cb_stride(kCbRowMax))));
   int per_sm = 0;
   RST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kf, kCbThreads, smem));
   if (per_sm < 1) return arg_fail("clique bit rows do not fit shared memory");

@@ -1015,8 +1015,9 @@ reset_status reset_intersect_count(const int32_t* d_a, int64_t na,
   if (na > 0 && nb > 0 && nb <= kPairSmem) {
     ++lg;  // (at most a quarter full)
     const int smem = (int)sizeof(int32_t) << lg;
+    // (the same for every size: other threads may be between here and a launch)
     RST_CUDA(cudaFuncSetAttribute(pair_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  smem));
+                                  (int)sizeof(int32_t) * 4 * kPairSmem));
     // a CTA looks up about as many keys as it inserts
     const int64_t share = std::max<int64_t>(4 * kPairThreads, nb);
     const int grid = (int)clamp_grid((na + share - 1) / share, sm_count());

@@ -170,11 +170,17 @@ __global__ void __launch_bounds__(kOT)
     cls[u] = s_c[deg_step(indeg[u] + __ldg(koff + u + 1) - __ldg(koff + u))];
 }
 
-// The first chunk of the padded row u, whose keys start at s: rows start at
-// least a chunk per 8 keys and one more apart, so no scan over the rows is
-// needed (three launches, 12 of 264 us at scale 16), for at most n chunks in all.
-__device__ __forceinline__ unsigned first_chunk(int s, int u, int64_t mk) {
-  return ((unsigned)min((int64_t)max(s, 0), mk) >> 3) + (unsigned)u;
+// The first chunk of the padded row u of n, whose keys start at s of mk: a
+// chunk per 8 keys and one more per row is room enough, or, in fewer chunks
+// where rows have hardly a key each, a chunk per key.  So no scan over the
+// rows is needed (three launches, 12 of 264 us at scale 16), and the rows take
+// no more memory than packed ones and the scan's result.
+__host__ __device__ __forceinline__ int64_t padded_chunks(int64_t n, int64_t mk) {
+  return mk / 8 + n < mk ? mk / 8 + n : mk;
+}
+__device__ __forceinline__ unsigned first_chunk(int s, int u, int64_t n, int64_t mk) {
+  const unsigned at = (unsigned)min((int64_t)max(s, 0), mk);
+  return mk / 8 + n < mk ? (at >> 3) + (unsigned)u : at;
 }
 
 // The padded rows, 8 lanes to a row, in class order with their lowest class
@@ -196,7 +202,7 @@ __global__ void __launch_bounds__(kOT)
   for (int64_t u = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3; u < n; u += step) {
     const int s = max(__ldg(koff + u), 0);
     const int d = (int)min((int64_t)(__ldg(koff + u + 1) - s), mk - s);
-    int32_t* out = padded + (int64_t)first_chunk(s, (int)u, mk) * 8;
+    int32_t* out = padded + (int64_t)first_chunk(s, (int)u, n, mk) * 8;
     int place[kPer];
     int lowest = 0;
     for (int i = 0; i < kPer; ++i) place[i] = 0;
@@ -365,7 +371,7 @@ __global__ void __launch_bounds__(kOT)
     for (int i = 0; i < kIlp; ++i) {
       const bool ok = eo.owner[i] >= 0;
       row[i] = make_int2(
-          ok ? (int)first_chunk(__ldg(koff + eo.prober[i]), eo.prober[i], mk) : 0, eo.len[i]);
+          ok ? (int)first_chunk(__ldg(koff + eo.prober[i]), eo.prober[i], n, mk) : 0, eo.len[i]);
       const int from = ok && eo.low[i] ? __ldg(&places[eo.prober[i]].at[eo.low[i]]) : 0;
       row[i].x += from;
       row[i].y -= 8 * from;
@@ -821,9 +827,7 @@ reset_status tc_owner(const reset_table* t, const int4* kdesc, const int32_t* ko
   const size_t sz_ent = al(sizeof(int2) * m), sz_units = al(sizeof(int2) * max_units);
   const size_t sz_list = al(sizeof(int32_t) * n), sz_ctr = al(sizeof(int32_t) * 8);
   const size_t sz_dunits = al(sizeof(int2) * max_dunits);
-  // padded rows: a chunk more for every row (at most the size of the table,
-  // whose rows hold at least 8 slots), and one without keys
-  const int64_t pad_chunks = mk / 8 + n + 1;
+  const int64_t pad_chunks = padded_chunks(n, mk) + 1;  // (and one without keys)
   const size_t sz_pad = al(8 * sizeof(int32_t) * (size_t)(pad_chunks + 1));
   // classes need the rows to be the sets of the tables (the CSR they were
   // built on), and pay on more edges than the passes cost
