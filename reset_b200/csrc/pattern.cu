@@ -879,14 +879,25 @@ extern "C" reset_status reset_pattern_count(const reset_table* t, const int32_t*
   while (lg_grab < 5 && (m >> (lg_grab + 1)) >= grid * kPtWarps * 8) ++lg_grab;
   grid = std::min<int64_t>(grid, ((m >> lg_grab) + 1 + max_parts + kPtWarps - 1) / kPtWarps);
   auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-  const bool some = bit_rows > 0 && bit_rows < t->n;
-  const size_t sz_scr = al(per_block * (size_t)grid);
-  const size_t sz_bits = al(sizeof(uint32_t) * (size_t)(bit_rows * br.words));
-  const size_t sz_row = some ? al(sizeof(int32_t) * (size_t)t->n) : 0;
-  const size_t sz_list = al(sizeof(int4) * (size_t)max_parts);
+  bool some = false;
+  size_t sz_scr = 0, sz_bits = 0, sz_row = 0, sz_list = 0;
   char* base = nullptr;
-  RST_CUDA(scratch_malloc(reinterpret_cast<void**>(&base), sz_scr + sz_bits + sz_row + sz_list + 256,
-                          st));
+  auto allocate = [&]() {
+    some = bit_rows > 0 && bit_rows < t->n;
+    sz_scr = al(per_block * (size_t)grid);
+    sz_bits = al(sizeof(uint32_t) * (size_t)(bit_rows * br.words));
+    sz_row = some ? al(sizeof(int32_t) * (size_t)t->n) : 0;
+    sz_list = al(sizeof(int4) * (size_t)max_parts);
+    return scratch_malloc(reinterpret_cast<void**>(&base),
+                          sz_scr + sz_bits + sz_row + sz_list + 256, st);
+  };
+  if (allocate() != cudaSuccess) {  // without memory for them: no bit rows, no parts
+    cudaGetLastError();
+    bit_rows = 0;
+    part = 0;
+    max_parts = 0;
+    RST_CUDA(allocate());
+  }
   int32_t* scr = reinterpret_cast<int32_t*>(base);
   uint32_t* bits = reinterpret_cast<uint32_t*>(base + sz_scr);
   int32_t* row = reinterpret_cast<int32_t*>(base + sz_scr + sz_bits);

@@ -861,8 +861,11 @@ reset_status reset_tc_count_ex(const reset_table* t, const int32_t* d_off,
   }
   if (method == 3) {
     reset_status s = tc_owner(t, ds.desc, d_off, d_cols, m, d_off, d_cols, rows, m, cnt, st);
-    if (owned_rows) cudaFreeAsync(owned_rows, st);
-    return s;
+    if (s != RESET_ERR_OOM) {
+      if (owned_rows) cudaFreeAsync(owned_rows, st);
+      return s;
+    }
+    cudaGetLastError();  // no memory for the groups (nothing ran): edge by edge
   }
   unsigned long long* cursor = nullptr;
   RST_CUDA(scratch_malloc(reinterpret_cast<void**>(&cursor), sizeof(*cursor), st));

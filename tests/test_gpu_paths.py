@@ -212,6 +212,26 @@ def test_owner_grouped_set_sizes(R, cuda, d):
         t.free()
 
 
+@pytest.mark.parametrize("n", [130, 600, 690, 700, 20000])
+def test_owner_grouped_room_for_rows(R, cuda, n):
+    """As many keys in more and more rows: a chunk per 8 keys and row, then a
+    chunk per key (from 7/8 of a row per key on)."""
+    rng = np.random.default_rng(n)
+    adj = [[] for _ in range(n)]
+    pairs = [(u, v) for u in range(40) for v in range(u + 1, 40)]  # (a core with triangles)
+    for u, v in rng.permutation(pairs)[:500].tolist():
+        adj[u].append(v)
+    for u in rng.permutation(np.arange(40, n))[:289].tolist() if n > 400 else [40] * 80:
+        adj[u].append(len(adj[u]) + 41 if n <= 400 else 0)
+    rows = [sorted(set(r)) for r in adj]
+    off, cols = csr(rows)
+    d_off, d_cols = dev(off, cuda), dev(cols, cuda)
+    t = R.Table(d_off, d_cols)
+    want = sum(len(np.intersect1d(rows[u], rows[v])) for u in range(n) for v in rows[u])
+    assert want > 0 and R.tc_count(t, d_off, d_cols, method=3) == want
+    t.check()
+
+
 def test_owner_grouped_classes_and_single_chunk_rows(R, cuda):
     """2^24 keys and more: rows in class order; long runs of rows of one chunk
     between long ones (the rings that follow the rows fill with short rows)."""
