@@ -38,14 +38,14 @@
 // intersections of at most kLaneMax keys run one candidate per lane, longer
 // ones by the whole warp, as AND + popcount over the two bit rows where that
 // is less work than looking up the shorter row's keys; without a bound, on up
-// to 8192 vertices, the sizes of all such intersections are computed first
+// to 16384 vertices, the sizes of all such intersections are computed first
 // (codegree_kernel) and a candidate costs a load.  A reusing
 // k-clique chain without checks (SMOG's Q0, Q3, Q5, Q7) runs the k-clique
 // count (clique.cu).
 //
 // Bound by instruction issue and, on small graphs, by the longest part.
 // Against one edge per warp with every lookup a hash probe (R-MAT, ms):
-// Q6 scale 8 / 11: 3.2 / 116 -> 0.16 / 0.79; Q4 scale 8 / 13: 0.57 / 19.8 ->
+// Q6 scale 8 / 11: 3.2 / 116 -> 0.16 / 0.81; Q4 scale 8 / 13: 0.57 / 19.8 ->
 // 0.15 / 4.8; Q8 scale 13: 20.6 -> 3.7; Q1 scale 8 / 14: 0.16 / 16.3 ->
 // 0.12 / 6.5; Q2 scale 14: 11.9 -> 3.1.
 //
@@ -173,13 +173,15 @@ __device__ __forceinline__ int first_set(const PatternDev& p, int du, int dv) {
   return s;
 }
 
-// Start edges with a first set above `part` keys, as (u, v, i, parts), and
-// the sum of these sets' squares.
+// Start edges with a first set above `part` keys, as (u, v, i, parts).  With
+// the bit rows of all vertices, also an estimate of the visits of a paired
+// last level, from every step-th of these edges: |C_2| (squared where two
+// levels walk it), less where rows are short and a visit costs little.
 __global__ void pattern_parts_kernel(const int4* __restrict__ desc,
                                      const int32_t* __restrict__ cols, int32_t n, int64_t m,
                                      const PatternDev pat, int part, int4* __restrict__ list,
-                                     int32_t* __restrict__ n_list,
-                                     unsigned long long* __restrict__ squares) {
+                                     int32_t* __restrict__ n_list, const BitRows br, int step,
+                                     unsigned long long* __restrict__ visits) {
   const int lane = threadIdx.x & 31;
   unsigned long long sum = 0;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -200,35 +202,51 @@ __global__ void pattern_parts_kernel(const int4* __restrict__ desc,
       int at = lane == 0 ? atomicAdd(n_list, total) : 0;
       at = __shfl_sync(kFull, at, 0) + before;
       for (int i = 0; i < np; ++i) list[at + i] = make_int4((int)u, v, i, np);
-      if (np) sum += (unsigned long long)s * s;
+      if (!br.bits) continue;
+      for (unsigned todo = __ballot_sync(kFull, np > 0 && (du.x + j) % step == 0); todo;
+           todo &= todo - 1) {
+        const int g = __ffs(todo) - 1;
+        const int vg = __shfl_sync(kFull, v, g), sg = __shfl_sync(kFull, s, g);
+        int c = 0;
+        for (int w = lane; w < br.words; w += 32) {
+          uint32_t x = ~0u;
+          for (int i = 0; i < pat.nb[2]; ++i) x &= __ldg(br.of(pat.back[2][i] == 0 ? u : vg) + w);
+          c += __popc(x);
+        }
+        const unsigned long long e = __reduce_add_sync(kFull, c);
+        if (lane == 0) sum += (pat.k > 4 ? e * e : e) * min(sg, 64);
+      }
     }
   }
-  sum = warp_sum_u64(sum);
-  if (lane == 0 && sum) atomicAdd(squares, sum);
+  if (lane == 0 && sum) atomicAdd(visits, sum * step / 64);
 }
 
 // Co-degrees |N(a) ∩ N(x)| of all pairs of vertices, from the bit rows: where
 // the paired last level has no bound, its count for a candidate x is one of
 // them, less the earlier vertices, and a visit costs a load where it took the
 // AND of two bit rows by the whole warp.  The matrix takes n^3 / 64 word
-// steps, a walk visits some part of the sum of the squared first sets: the
-// matrix is filled (and used) where that sum times kCoVisits reaches n^3, on
-// the device, since the sum is found there.  Popcounts bound
-// the matrix (n = 2048: 44 us).  Q6 on R-MAT graphs, ms a call, by ANDs / by
-// co-degrees: scale 11 3.41 / 0.79, scale 13 62.8 / 6.9 (268 MB of matrix);
-// scale 8, whose matrix is nothing, 0.26 / 0.16.
-constexpr unsigned long long kCoVisits = 1024;
+// steps of three instructions, a visit without it up to 100 warp
+// instructions: it is filled (and used) where the visits times kCoVisits reach
+// n^3, a quarter of where it pays with long rows.  Decided on the device, where
+// the estimate is.  Popcounts bound the matrix (n = 2048: 44 us).  Q6 on R-MAT
+// graphs, ms a call, by ANDs / by co-degrees: scale 11 3.41 / 0.81, scale 13
+// 62.8 / 6.9 (268 MB of matrix), scale 14 380 / 30 (1 GB); scale 8, whose matrix is
+// nothing, 0.26 / 0.16.  A random graph of 8192 vertices and 100 neighbours
+// each, with hardly a common one, is walked without.
+constexpr unsigned long long kCoVisits = 16384;
+constexpr int kCoSmall = 512;  // vertices whose matrix (2 us) costs less than the estimate
+constexpr int64_t kCoBudget = int64_t(1) << 30;  // bytes: up to 16384 vertices
 constexpr int kCoTile = 64;  // vertices on a side of a block's tile
 constexpr int kCoWords = 32;
 
-__device__ __forceinline__ bool co_used(const unsigned long long* squares, int64_t n) {
-  return *squares * kCoVisits >= (unsigned long long)(n * n * n);
+__device__ __forceinline__ bool co_used(const unsigned long long* visits, int64_t n) {
+  return n <= kCoSmall || *visits >= (unsigned long long)(n * n * n) / kCoVisits;
 }
 
 __global__ void __launch_bounds__(256)
     codegree_kernel(const uint32_t* __restrict__ bits, int32_t n, int words,
-                    const unsigned long long* __restrict__ squares, int32_t* __restrict__ co) {
-  if (!co_used(squares, n)) return;
+                    const unsigned long long* __restrict__ visits, int32_t* __restrict__ co) {
+  if (!co_used(visits, n)) return;
   const int i0 = blockIdx.y * kCoTile, j0 = blockIdx.x * kCoTile;
   if (i0 > j0) return;  // the tile below the diagonal is written with its mirror
   __shared__ uint32_t sa[kCoTile][kCoWords + 1], sb[kCoTile][kCoWords + 1];
@@ -272,7 +290,7 @@ __global__ void __launch_bounds__(kPtThreads, 4)
                    int32_t n, int64_t m, const int32_t* __restrict__ table, int64_t bn, int b,
                    int lg_max, const PatternDev pat, int sorted, const BitRows br,
                    const int32_t* __restrict__ loops, const int32_t* __restrict__ co,
-                   const unsigned long long* __restrict__ squares,
+                   const unsigned long long* __restrict__ visits,
                    const int4* __restrict__ parts_list,
                    const int32_t* __restrict__ n_list, int part, int lg_grab,
                    int32_t* __restrict__ scratch, int32_t cap,
@@ -293,7 +311,7 @@ __global__ void __launch_bounds__(kPtThreads, 4)
   const int n_parts = part > 0 ? *n_list : 0;
   // no row holds its own vertex (known where bit rows were set)
   const bool loop_free = br.bits && *loops == 0;
-  const bool have_co = co && co_used(squares, n);
+  const bool have_co = co && co_used(visits, n);
   unsigned long long hits = 0;
   // level l: m_l, its index in C_l, C_l (cs, sz), the next candidate (it)
   int map[kPatMax], idx[kPatMax], sz[kPatMax], it[kPatMax];
@@ -902,10 +920,10 @@ extern "C" reset_status reset_pattern_count(const reset_table* t, const int32_t*
   uint32_t* bits = reinterpret_cast<uint32_t*>(base + sz_scr);
   int32_t* row = reinterpret_cast<int32_t*>(base + sz_scr + sz_bits);
   int4* list = reinterpret_cast<int4*>(base + sz_scr + sz_bits + sz_row);
-  // [0..1] work cursors, the parts' squares (u64), then the listed parts,
+  // [0..1] work cursors, the visits (u64), then the listed parts,
   // self-loops, bit rows
   auto* cursor = reinterpret_cast<unsigned long long*>(base + sz_scr + sz_bits + sz_row + sz_list);
-  auto* squares = cursor + 2;
+  auto* visits = cursor + 2;
   int32_t* ctr = reinterpret_cast<int32_t*>(cursor + 3);
   const int warp_grid = (int)std::min<int64_t>(((int64_t)t->n + 7) / 8, (int64_t)sms * 8);
   cudaError_t e = cudaMemsetAsync(cursor, 0, 256, st);
@@ -925,26 +943,29 @@ extern "C" reset_status reset_pattern_count(const reset_table* t, const int32_t*
       e = cudaGetLastError();
     }
   }
-  if (e == cudaSuccess && part > 0) {
-    note_launch();
-    pattern_parts_kernel<<<warp_grid, 256, 0, st>>>(t->d_desc, d_cols, t->n, m, pat, part, list,
-                                                    ctr, squares);
-    e = cudaGetLastError();
-  }
   // co-degrees, where the paired last level has no bound; without memory for
   // them the walk does as well
   const bool bounded = (pat.flags & RESET_PATTERN_RESTRICT) && pat.restr[pat.k - 1] >= 0;
   const int64_t co_bytes = (int64_t)sizeof(int32_t) * t->n * t->n;
+  const bool co_may = pat.pair && sorted && !bounded && bit_rows == t->n && part > 0 &&
+                      co_bytes <= kCoBudget;
   int32_t* co = nullptr;
-  if (e == cudaSuccess && pat.pair && sorted && !bounded && bit_rows == t->n &&
-      co_bytes <= kBitBudget) {
+  if (e == cudaSuccess && part > 0) {
+    const int step = (int)std::max<int64_t>(1, m >> 10);  // about 2^10 edges looked at
+    note_launch();
+    pattern_parts_kernel<<<warp_grid, 256, 0, st>>>(t->d_desc, d_cols, t->n, m, pat, part, list,
+                                                    ctr, co_may && t->n > kCoSmall ? br : BitRows{}, step,
+                                                    visits);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess && co_may) {
     if (scratch_malloc(reinterpret_cast<void**>(&co), (size_t)co_bytes, st) != cudaSuccess) {
       cudaGetLastError();
       co = nullptr;
     } else {
       const unsigned tiles = (unsigned)((t->n + kCoTile - 1) / kCoTile);
       note_launch();
-      codegree_kernel<<<dim3(tiles, tiles), 256, 0, st>>>(bits, t->n, (int)br.words, squares, co);
+      codegree_kernel<<<dim3(tiles, tiles), 256, 0, st>>>(bits, t->n, (int)br.words, visits, co);
       e = cudaGetLastError();
     }
   }
@@ -953,7 +974,7 @@ extern "C" reset_status reset_pattern_count(const reset_table* t, const int32_t*
 #define PT_LAUNCH(H)                                                                           \
   pattern_kernel<H><<<(int)grid, kPtThreads, 0, st>>>(                                         \
       t->d_desc, d_off, d_cols, t->d_chunk_row, t->n, m, t->d_table, t->bucket_num, t->bucket, \
-      t->lg_max, pat, sorted, br, ctr + 1, co, squares, list, ctr, part, lg_grab, scr, cap,    \
+      t->lg_max, pat, sorted, br, ctr + 1, co, visits, list, ctr, part, lg_grab, scr, cap,    \
       reinterpret_cast<unsigned long long*>(d_count), cursor, t->d_status)
     if (t->hier) PT_LAUNCH(true); else PT_LAUNCH(false);
 #undef PT_LAUNCH
