@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(1024)
                      LongSet* __restrict__ sets, int32_t* __restrict__ crowded) {
   using Scan = cub::BlockScan<int, 1024>;
   __shared__ typename Scan::TempStorage tmp;
-  int keys = 0, buckets = 0;  // items before this round
+  int keys = 0, buckets = 0;  // items before this pass
   for (int base = 0; base < n; base += 1024) {
     const int i = base + threadIdx.x;
     LongSet s{};
