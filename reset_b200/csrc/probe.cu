@@ -118,6 +118,7 @@ constexpr int kFilterWords = kFilterBits / 32;
 constexpr int kFilterMax = 4096;  // keys of the shared set: a quarter of the bits, past
                                   // which too many unlike keys are taken for common
 constexpr int kFilterRun = 3;     // a run that pays for clearing and filling the bitmap
+constexpr int kFilterStream = 1 << 25;  // keys streamed for a pair: 32 of them fit an int
 
 __device__ __forceinline__ unsigned filter_hash(int x) { return (unsigned)x * 0x9E3779B1u; }
 
@@ -141,8 +142,8 @@ __device__ __forceinline__ bool filter_fill(const int32_t* __restrict__ row, int
   return __all_sync(kFull, ok);
 }
 
-// The first n keys of every lane's row (start in elems) looked up in the
-// bitmap, flattened across the lanes; counts into hits[lane].
+// The first n <= kFilterStream keys of every lane's row (start in elems)
+// looked up in the bitmap, flattened across the lanes; counts into hits[lane].
 __device__ __forceinline__ void filter_stream(const int32_t* __restrict__ elems, int start, int n,
                                               const uint32_t* bits, int* hits) {
   constexpr int R = 4;
@@ -279,11 +280,12 @@ __global__ void __launch_bounds__(kThreads, 4)
           const int z = after ? __ffs(after) - 1 : 32;
           const int na = __shfl_sync(kFull, da.y, k);
           if (z - k < kFilterRun || na > kFilterMax) continue;
-          const int row = __shfl_sync(kFull, da.x, k);
-          if (!filter_fill(elems + row, na, s_bits[warp])) continue;
           const bool mine = lane >= k && lane < z && ok && allowed >= 0;
           const int64_t miss = (int64_t)dq.y - need;  // of the other set's keys
           const int n = mine ? (int)min((int64_t)dq.y, miss + 8 + (miss >> 2)) : 0;
+          if (__any_sync(kFull, n > kFilterStream)) continue;  // (left to the lookups)
+          const int row = __shfl_sync(kFull, da.x, k);
+          if (!filter_fill(elems + row, na, s_bits[warp])) continue;
           filter_stream(elems, dq.x, n, s_bits[warp], s_hits[warp]);
           __syncwarp();
           if (mine && n - s_hits[warp][lane] > miss) allowed = -1;

@@ -368,6 +368,27 @@ def test_decisions_only_like_full(R, cuda, kind, num, den):
 
 # -------------------------------------------------------- prefix filter --
 
+def test_decisions_only_of_very_large_sets(R, cuda):
+    """Runs of pairs of one set whose other sets' keys together exceed 2^31."""
+    big = 70_000_000
+    held = cuda.arange(4096, dtype=cuda.int32, device="cuda") * 17000
+    few = cuda.cat([held[:1400], held[1400:] + big])
+    elems = cuda.cat([held, few, cuda.arange(big, dtype=cuda.int32, device="cuda")])
+    off = cuda.tensor([0, 4096, 8192, 8192 + big], dtype=cuda.int32, device="cuda")
+    # two slots a bucket, at most one of them taken: no lookup walks on
+    t = R.Table(off, elems, alpha=0.5, bucket=2, hierarchical=False)
+    # 1401 common keys are needed: 4096 in pairs (0, 2), 1400 in pairs (1, 2)
+    assert -(-(4096 + big) // 50001) == 1401
+    pa = cuda.arange(64, device="cuda").div(32, rounding_mode="floor").int()
+    pb = cuda.full_like(pa, 2)
+    # (a batch gives a warp 32 pairs, however few there are)
+    batch = R.Batch(t, elems, capacity=64, num=1, den=50000, decisions_only=True)
+    flags, _ = batch(pa, pb)
+    assert cuda.equal(flags, (pa == 0).to(cuda.uint8))
+    batch.close()
+    t.check()
+
+
 @pytest.mark.parametrize("num,den", [(1, 2), (7, 10), (1, 1)])
 @pytest.mark.parametrize("freq", ["skewed", "level", "repeated", "shuffled"])
 def test_prefix_selection_at_set_sizes(R, cuda, freq, num, den):
