@@ -368,6 +368,42 @@ def test_decisions_only_like_full(R, cuda, kind, num, den):
 
 # -------------------------------------------------------- prefix filter --
 
+def _best_ms(cuda, f, n=5):
+    f()
+    best = float("inf")
+    for _ in range(n):
+        a, z = (cuda.cuda.Event(enable_timing=True) for _ in range(2))
+        a.record()
+        f()
+        z.record()
+        z.synchronize()
+        best = min(best, a.elapsed_time(z))
+    return best
+
+
+@pytest.mark.parametrize("size,differ", [(63, 2), (255, 6), (300, 100), (5000, 0), (5000, 20)])
+def test_decisions_only_of_like_sets(R, cuda, size, differ):
+    """Sets that share most of their keys: as with sizes, at most twice the
+    time (a pair's lookups are all the work, whichever way they are cut)."""
+    rng = np.random.default_rng(0x5EED8100 + size + differ)
+    base = rng.choice(1 << 20, size + differ, replace=False)
+    rows = [np.sort(np.delete(base, rng.choice(base.size, differ, replace=False)))
+            for _ in range(40)]
+    off, elems = csr(rows)
+    d_off, d_elems = dev(off, cuda), dev(elems, cuda)
+    t = R.Table(d_off, d_elems)
+    pairs = rng.integers(0, 40, (2, 3000)).astype(np.int32)
+    pa, pb = dev(pairs[0], cuda), dev(pairs[1], cuda)
+    for num, den in [(1, 2), (7, 10), (19, 20), (99, 100), (1, 1)]:
+        full = R.sss(t, d_off, d_elems, pa, pb, num, den)[0]
+        only = R.sss(t, d_off, d_elems, pa, pb, num, den, with_inter=False)[0]
+        assert cuda.equal(only, full), (num, den)
+        fast = _best_ms(cuda, lambda: R.sss(t, d_off, d_elems, pa, pb, num, den,
+                                            with_inter=False))
+        assert fast <= 2 * _best_ms(cuda, lambda: R.sss(t, d_off, d_elems, pa, pb, num, den)) + 0.02
+    t.check()
+
+
 def test_decisions_only_of_very_large_sets(R, cuda):
     """Runs of pairs of one set whose other sets' keys together exceed 2^31."""
     big = 70_000_000
