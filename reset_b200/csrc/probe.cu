@@ -111,13 +111,21 @@ __global__ void __launch_bounds__(kThreads, 4)
 // reads a sector or two of HBM per key (and is bound by them).  It can only
 // take keys for common that are not, so a pair with more misses than its
 // decision allows is settled; the few others are decided by the tables.
-// 5.4 M candidate pairs of sets of up to 512 keys: 2.56 ms without the
-// bitmap, 1.50 with it.  Pairs in no order never fill one.
+// 5.4 M candidate pairs of sets of up to 1024 keys: 2.87 ms without the
+// bitmap, 1.84 with it.  Pairs in no order never fill one.
+//
+// It is taken where it is likely to settle its pairs and costs less than the
+// lookups that it spares, and given up where the keys streamed show that the
+// sets share too much.  us a call, no bitmap / every run / by this rule:
+// 400,000 pairs of one set, at 1/100 with 100 keys and 5000 a set 302 / 5060 /
+// 311; 2000 keys a set that share a third, at 7/10 873 / 1358 / 899, at 1/10
+// 1461 / 3598 / 1491; 2000 keys that share 2%, at 1/10 4330 / 2063 / 2127.
 constexpr int kFilterBits = 16384;
 constexpr int kFilterWords = kFilterBits / 32;
 constexpr int kFilterMax = 4096;  // keys of the shared set: a quarter of the bits, past
                                   // which too many unlike keys are taken for common
 constexpr int kFilterRun = 3;     // a run that pays for clearing and filling the bitmap
+constexpr int kFilterLook = 512;  // keys after which a stream is first looked at
 constexpr int kFilterStream = 1 << 25;  // keys streamed for a pair: 32 of them fit an int
 
 __device__ __forceinline__ unsigned filter_hash(int x) { return (unsigned)x * 0x9E3779B1u; }
@@ -144,14 +152,20 @@ __device__ __forceinline__ bool filter_fill(const int32_t* __restrict__ row, int
 
 // The first n <= kFilterStream keys of every lane's row (start in elems)
 // looked up in the bitmap, flattened across the lanes; counts into hits[lane].
-__device__ __forceinline__ void filter_stream(const int32_t* __restrict__ elems, int start, int n,
-                                              const uint32_t* bits, int* hits) {
+// Given up (false) where clearly more than `most` of the keys so far are held.
+__device__ __forceinline__ bool filter_stream(const int32_t* __restrict__ elems, int start, int n,
+                                              float most, const uint32_t* bits, int* hits) {
   constexpr int R = 4;
   const int lane = threadIdx.x & 31;
-  int total;
+  int total, look = kFilterLook;
   const int P = warp_excl_scan(n, &total);
   const int src = start - P;
   for (int base = 0; base < total; base += 32 * R) {
+    if (base == look) {  // (a look at 512, 1024, ... keys; three standard deviations)
+      const float mean = most * (float)base;
+      if ((float)__reduce_add_sync(kFull, hits[lane]) > mean + 3.f * sqrtf(mean)) return false;
+      if (look <= kFilterStream) look *= 2;
+    }
     int x[R], k[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -174,6 +188,7 @@ __device__ __forceinline__ void filter_stream(const int32_t* __restrict__ elems,
       __syncwarp();
     }
   }
+  return true;
 }
 
 template <bool HIER, bool FLOAT_RULE, int ROUNDS, bool LEAN, bool EARLY = false>
@@ -196,6 +211,7 @@ __global__ void __launch_bounds__(kThreads, 4)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int* const qx = s_queue[warp];
   int* const qh = qx + 32 * ROUNDS;
+  int pause = 0;  // 1: the last bitmap settled nothing; more: runs to leave out
   if (np_dev) np = *np_dev;  // pair count set on the device (captured graphs)
   const int grab = 1 << lg_grab;  // pairs a warp takes at a time, at most 32
   const int64_t n_chunks = (np + grab - 1) >> lg_grab;
@@ -290,15 +306,33 @@ __global__ void __launch_bounds__(kThreads, 4)
           const int z = after ? __ffs(after) - 1 : 32;
           const int na = __shfl_sync(kFull, da.y, k);
           if (z - k < kFilterRun || na > kFilterMax) continue;
-          const bool mine = lane >= k && lane < z && ok && allowed >= 0;
-          const int64_t miss = (int64_t)dq.y - need;  // of the other set's keys
-          const int n = mine ? (int)min((int64_t)dq.y, miss + 8 + (miss >> 2)) : 0;
+          // the keys of the other set that settle the pair, where they are
+          // likely to, and the lookups that they would spare
+          const int64_t miss = (int64_t)dq.y - need;
+          int n = 0, spared = 0;
+          if (lane >= k && lane < z && allowed >= 0 && need > 0) {
+            n = (int)min((int64_t)dq.y, miss + 8 + (miss >> 2));
+            spared = (int)min((int64_t)min(s, kFilterStream), (int64_t)allowed + 8 + (allowed >> 2));
+            // (as many are held by chance as bits are set; 1 in 20 and one more allowed for)
+            if ((float)n * (0.95f - (float)na / kFilterBits) <= (float)(miss + 1)) n = spared = 0;
+          }
           if (__any_sync(kFull, n > kFilterStream)) continue;  // (left to the lookups)
+          const int streamed = __reduce_add_sync(kFull, n);
+          const int looked_up = __reduce_add_sync(kFull, spared);
+          // a lookup costs about five keys entered or streamed
+          if ((int64_t)streamed + na + 256 >= (int64_t)5 * looked_up) continue;
+          if (pause > 1) {
+            --pause;
+            continue;
+          }
           const int row = __shfl_sync(kFull, da.x, k);
-          if (!filter_fill(elems + row, na, bits)) continue;
-          filter_stream(elems, dq.x, n, bits, s_hits[warp]);
+          const float misses = (float)__reduce_add_sync(kFull, n > 0 ? (int)miss : 0);
+          const bool settles =
+              filter_fill(elems + row, na, bits) &&
+              filter_stream(elems, dq.x, n, 1.f - misses / (float)streamed, bits, s_hits[warp]);
           __syncwarp();
-          if (mine && n - s_hits[warp][lane] > miss) allowed = -1;
+          if (settles && n > 0 && n - s_hits[warp][lane] > miss) allowed = -1;
+          pause = settles ? 0 : pause ? 9 : 1;
           __syncwarp();
           s_hits[warp][lane] = 0;
           __syncwarp();

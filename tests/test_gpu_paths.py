@@ -404,6 +404,34 @@ def test_decisions_only_of_like_sets(R, cuda, size, differ):
     t.check()
 
 
+@pytest.mark.parametrize("size,other,universe", [
+    (100, 5000, 100_000), (2000, 2000, 6000), (64, 300, 3000), (300, 300, 1 << 20), (30, 30, 80)])
+def test_decisions_only_of_one_set(R, cuda, size, other, universe):
+    """Runs of pairs with one first set, at thresholds where its bitmap settles
+    all, some or none of them: as with sizes, at most twice the time."""
+    rng = np.random.default_rng(0x5EED8200 + size)
+    rows = [np.sort(rng.choice(universe, size, replace=False))]
+    rows += [np.sort(rng.choice(universe, other, replace=False)) for _ in range(400)]
+    for r in rows[1::5]:  # near-duplicates among them
+        k = min(size, other) * 9 // 10
+        r[:k] = rng.choice(rows[0], k, replace=False)
+    rows = [np.unique(r) for r in rows]
+    off, elems = csr(rows)
+    d_off, d_elems = dev(off, cuda), dev(elems, cuda)
+    t = R.Table(d_off, d_elems)
+    n = 200_000
+    pa = cuda.zeros(n, dtype=cuda.int32, device="cuda")
+    pb = dev(rng.integers(1, 401, n).astype(np.int32), cuda)
+    for num, den in [(1, 100), (1, 20), (1, 10), (1, 2), (7, 10), (1, 1)]:
+        full = R.sss(t, d_off, d_elems, pa, pb, num, den)[0]
+        only = R.sss(t, d_off, d_elems, pa, pb, num, den, with_inter=False)[0]
+        assert cuda.equal(only, full), (num, den)
+        fast = _best_ms(cuda, lambda: R.sss(t, d_off, d_elems, pa, pb, num, den,
+                                            with_inter=False))
+        assert fast <= 2 * _best_ms(cuda, lambda: R.sss(t, d_off, d_elems, pa, pb, num, den)) + 0.02
+    t.check()
+
+
 def test_decisions_only_of_very_large_sets(R, cuda):
     """Runs of pairs of one set whose other sets' keys together exceed 2^31."""
     big = 70_000_000
