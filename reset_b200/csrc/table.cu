@@ -43,7 +43,7 @@ constexpr int kTileThreads = 512;  // threads of a tile-build CTA (3 CTAs, 48 wa
 constexpr int kTileWarps = kTileThreads / 32;
 constexpr bool kTileDynamic = true;  // warps take a tile's larger sets from a cursor
 constexpr int kThreadSetMax = 8;      // sets with deg <= this: thread per set
-constexpr int kTileSmemBudget = 72 * 1024;
+constexpr int kTileSmemBudget = 72 * 1024;  // (a multiple of 16, as g.smem is)
 constexpr int kBigFillSmemMax = 64 * 1024;  // buckets whose fill bytes fit smem
 constexpr int kHugeKeys = 1 << 16;  // crowded sets this long are built by build_huge
 
@@ -1162,9 +1162,11 @@ reset_status launch_builds(const reset_table* t, const int32_t* d_off, const int
                            const int32_t* d_long, BuildInfo* d_info, const BuildInfo& info,
                            int32_t* d_hash_out, cudaStream_t st) {
   if (n_tiles > 0) {
+    // (the same for every bucket size: other threads may be between here and a
+    // launch; g.smem is at most the budget)
     RST_CUDA(cudaFuncSetAttribute(tile_build_kernel<HIER>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)g.smem));
+                                  kTileSmemBudget));
     note_launch(); tile_build_kernel<HIER><<<n_tiles, kTileThreads, g.smem, st>>>(
         d_off, d_elems, t->d_len, t->d_off64, d_tile_first, t->bucket_num,
         t->bucket, t->lg_max, g.R_max, g.LT, t->d_table, d_hash_out,

@@ -276,6 +276,41 @@ def test_long_sets_runs_and_crowding(R, cuda, oracle_mod, alpha, bucket, hier):
     _check_build(R, cuda, oracle_mod, rows, alpha, bucket, hier)
 
 
+def test_builds_of_all_bucket_sizes_from_several_threads(R, cuda):
+    """Each thread builds tables of its own bucket size on its own stream: the
+    shared memory that a tile takes differs by bucket size."""
+    import threading
+    rng = np.random.default_rng(0x5EED7E30)
+    off, elems = csr([np.sort(rng.choice(5000, 40, replace=False)) for _ in range(50)])
+    d_off, d_el = dev(off, cuda), dev(elems, cuda)
+    sizes = (1, 5, 3, 7, 1, 5)
+    tables = {b: R.Table(d_off, d_el, bucket=b) for b in sizes}
+    want = {b: t.tensors()[0].clone() for b, t in tables.items()}
+    cuda.cuda.synchronize()
+    errors = []
+
+    def work(b):
+        try:
+            stream = cuda.cuda.Stream()
+            for i in range(300):
+                t = R.Table(d_off, d_el, bucket=b, stream=stream)
+                if i % 50 == 0:
+                    stream.synchronize()
+                    assert cuda.equal(t.tensors()[0], want[b]), b
+                    cuda.cuda.current_stream().synchronize()
+                t.free_async(stream)
+            stream.synchronize()
+        except Exception as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(b,)) for b in sizes]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not errors, errors[0]
+
+
 def test_chunk_rows_of_long_rows(R, cuda, oracle_mod):
     """Chunk rows and tile starts of rows that span many chunks and tiles
     (written by a whole warp), beside empty ones."""
