@@ -388,20 +388,23 @@ __global__ void __launch_bounds__(kThreads, 4)
 constexpr int kPairThreads = 512;
 constexpr int kPairSmem = 4096;  // keys (a set of up to 64 KB)
 
-struct PairSet {  // 1 << lg slots at S, -1 = empty
+struct PairSet {  // 1 << lg slots at S (lg 1..32), -1 = empty
   int32_t* S;
   int lg;
   __device__ __forceinline__ unsigned home(int x) const {
     return ((unsigned)x * 0x9E3779B1u) >> (32 - lg);
   }
+  __device__ __forceinline__ unsigned next(unsigned h) const {
+    return (h + 1) & (0xFFFFFFFFu >> (32 - lg));
+  }
   __device__ __forceinline__ void insert(int x) const {
-    for (unsigned h = home(x);; h = (h + 1) & ((1u << lg) - 1u)) {
+    for (unsigned h = home(x);; h = next(h)) {
       const int old = atomicCAS(S + h, -1, x);
       if (old == -1 || old == x) return;
     }
   }
   __device__ __forceinline__ bool holds(int x) const {
-    for (unsigned h = home(x);; h = (h + 1) & ((1u << lg) - 1u)) {
+    for (unsigned h = home(x);; h = next(h)) {
       const int s = S[h];
       if (s == x) return true;
       if (s == -1) return false;

@@ -350,6 +350,17 @@ def test_raw_pair_sizes(R, cuda, na, nb):
     assert R.intersect_count(dev(a, cuda), dev(b, cuda)) == int(np.isin(a, b).sum())
 
 
+def test_raw_pair_of_more_than_2_to_the_30_keys(R, cuda):
+    """The set of 2^32 slots, the largest: its index takes all 32 bits."""
+    n = (1 << 30) + 5
+    b = cuda.arange(n, dtype=cuda.int32, device="cuda")
+    a = cuda.tensor([0, 7, n - 1, n, n + 1, (1 << 31) - 1] * 50, dtype=cuda.int32, device="cuda")
+    assert R.intersect_count(a, b) == 150
+    del b
+    cuda.cuda.empty_cache()
+    R._lib().reset_release_cached_memory()
+
+
 @pytest.mark.parametrize("pairs", [1, 33, 300, 4800, 40000])
 def test_pairs_per_warp(R, cuda, pairs):
     """Few pairs are spread over the warps, one to a warp at the fewest."""
