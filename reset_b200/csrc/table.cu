@@ -552,7 +552,13 @@ __global__ void __launch_bounds__(kTileThreads)
 // Runs are a few buckets long at the loads in use.  A set with a walk of
 // kWalkMax buckets or a run of more than kRunMax keys is "crowded" (a key
 // repeated many times, a full table): one warp inserts it sequentially, or
-// build_huge builds it if it is long.
+// build_huge builds it if it is long.  Sets that their load makes likely to be
+// (crowded_by_load) are so from the start: insert and fix would come on top.
+// Builds with rows, us, one warp per set / all through insert and fix / by
+// load: 60 sets of 30,000 keys, 16 slots a bucket, load 0.92 1030 / 4340 / 680;
+// 400 of 5000, one slot, load 0.61 343 / 618 / 265; 10 of 200,000, 5 slots,
+// load 0.61 2200 / 613 / 608 (a long set is likely by its own keys: build_huge takes
+// one set, while a sequential one holds all up).
 // Bound by the latency of the scattered slot accesses.  Index of 2M documents
 // and 100k terms (8M postings, ~100 long sets), build with rows, b = 5 / b = 1:
 // one warp per set, and 20 launches per set of 2^16 keys, 7.9 / 31 ms; all
@@ -568,11 +574,21 @@ struct LongSet {
   int32_t key_item, bucket_item;  // its first items
 };
 
-// The long sets' descriptors and the prefix sums of their items (one block).
+// Whether runs of more than kRunMax keys are likely among `keys` keys at this
+// load.  Their number falls as exp(-kRunMax * (load - 1 - ln load)), the decay of
+// linear probing's runs at any bucket size; over random homes, with 1 to 16 slots
+// a bucket and loads from 0.65 to 0.9, it was 0.0035 times that per key.
+__device__ __forceinline__ bool crowded_by_load(float load, float keys) {
+  return 0.0035f * keys * expf(-kRunMax * (load - 1.f - logf(load))) > 0.25f;
+}
+
+// The long sets' descriptors, the prefix sums of their items, and which are
+// crowded by their load (one block).
 __global__ void __launch_bounds__(1024)
     long_plan_kernel(const int32_t* __restrict__ off, const int32_t* __restrict__ len,
                      const int64_t* __restrict__ off64, const int32_t* __restrict__ list, int n,
-                     LongSet* __restrict__ sets, int32_t* __restrict__ crowded) {
+                     int b, float all_keys, LongSet* __restrict__ sets,
+                     int32_t* __restrict__ crowded) {
   using Scan = cub::BlockScan<int, 1024>;
   __shared__ typename Scan::TempStorage tmp;
   int keys = 0, buckets = 0;  // items before this pass
@@ -589,7 +605,8 @@ __global__ void __launch_bounds__(1024)
       s.toff = off64[s.u];
       ki = (s.d + kKeyItem - 1) / kKeyItem;
       bi = (l + kBucketItem - 1) / kBucketItem;
-      crowded[i] = 0;
+      crowded[i] = crowded_by_load((float)s.d / ((float)l * (float)b),
+                                   s.d >= kHugeKeys ? (float)s.d : all_keys);
     }
     int total;
     __syncthreads();
@@ -628,9 +645,9 @@ __device__ __forceinline__ int long_set_of(const LongSet* __restrict__ sets, int
 
 __global__ void __launch_bounds__(kThreads)
     long_clear_kernel(const LongSet* __restrict__ sets, int n, int64_t bucket_num, int b,
-                      int32_t* __restrict__ table) {
+                      int32_t* __restrict__ table, const int32_t* __restrict__ crowded) {
   const int i = long_set_of<&LongSet::bucket_item>(sets, n, blockIdx.x);
-  if (i < 0) return;
+  if (i < 0 || crowded[i]) return;  // (crowded sets are cleared where they are built)
   const LongSet s = sets[i];
   const int h0 = ((int)blockIdx.x - s.bucket_item) * kBucketItem;
   const int q = min(kBucketItem, (1 << s.lg) - h0) >> 2;
@@ -647,7 +664,7 @@ __global__ void __launch_bounds__(kThreads)
                        int64_t bucket_num, int b, int lg_max, int32_t* __restrict__ table,
                        int32_t* __restrict__ crowded) {
   const int i = long_set_of<&LongSet::key_item>(sets, n, blockIdx.x);
-  if (i < 0) return;
+  if (i < 0 || *(volatile int32_t*)(crowded + i)) return;
   const LongSet s = sets[i];
   const int j0 = ((int)blockIdx.x - s.key_item) * kKeyItem;
   int32_t* G = table + s.toff;
@@ -1201,8 +1218,10 @@ reset_status launch_builds(const reset_table* t, const int32_t* d_off, const int
     RST_CUDA(cudaFuncSetAttribute(long_crowded_kernel<HIER>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, fill_smem));
     note_launch(5);
-    long_plan_kernel<<<1, 1024, 0, st>>>(d_off, t->d_len, t->d_off64, d_long, n, sets, crowded);
-    long_clear_kernel<<<(unsigned)bucket_items, kThreads, 0, st>>>(sets, n, bn, b, t->d_table);
+    long_plan_kernel<<<1, 1024, 0, st>>>(d_off, t->d_len, t->d_off64, d_long, n, b,
+                                         (float)info.long_keys, sets, crowded);
+    long_clear_kernel<<<(unsigned)bucket_items, kThreads, 0, st>>>(sets, n, bn, b, t->d_table,
+                                                                   crowded);
     long_insert_kernel<HIER><<<(unsigned)key_items, kThreads, 0, st>>>(
         d_elems, sets, n, bn, b, t->lg_max, t->d_table, crowded);
     long_fix_kernel<HIER><<<(unsigned)bucket_items, kThreads, 0, st>>>(
