@@ -87,10 +87,10 @@ typedef struct reset_table_view {
  * calculate_length (triangle-count/hashtable.cu:21-36) exactly.  Keys are
  * placed by the reference insertion rule (hashtable.cu:53-101) applied in
  * CSR order, so the layout is deterministic.  Synchronises `stream` once
- * (to size the table), and once more where a set has 2^16 keys or more.  If d_hash_order_out is not NULL it receives, in the
- * same pass, every row read back in bucket order (what
- * launch_extract_hashtable_to_csr, baseline/common/utils.cu:148-175,
- * produces). */
+ * (to size the table), and once more where a set has 2^16 keys or more.  If
+ * d_hash_order_out is not NULL it receives, in the same pass, every row read
+ * back in bucket order (what launch_extract_hashtable_to_csr,
+ * baseline/common/utils.cu:148-175, produces). */
 reset_status reset_table_build(const int32_t *d_off, const int32_t *d_elems,
                                int32_t n, int64_t m, const reset_params *params,
                                int32_t hierarchical, int32_t *d_hash_order_out,

@@ -30,6 +30,7 @@
 
 #include <cstring>
 #include <mutex>
+#include <vector>
 
 #include "common.cuh"
 #include "probe_common.cuh"
@@ -1231,12 +1232,13 @@ reset_status launch_builds(const reset_table* t, const int32_t* d_off, const int
     RST_CUDA(cudaGetLastError());
     if (info.n_huge > 0) {  // one more sync, only for tables that have such sets
       int32_t nc = 0;
+      std::vector<LongSet> list((size_t)info.n_huge);  // (the first nc are written)
       RST_CUDA(cudaMemcpyAsync(&nc, &d_info->n_crowded, sizeof(nc), cudaMemcpyDeviceToHost, st));
+      RST_CUDA(cudaMemcpyAsync(list.data(), huge, sizeof(LongSet) * list.size(),
+                               cudaMemcpyDeviceToHost, st));
       RST_CUDA(cudaStreamSynchronize(st));
       for (int i = 0; i < nc; ++i) {
-        LongSet s;
-        RST_CUDA(cudaMemcpyAsync(&s, huge + i, sizeof(s), cudaMemcpyDeviceToHost, st));
-        RST_CUDA(cudaStreamSynchronize(st));
+        const LongSet& s = list[(size_t)i];
         RST_CHECK(build_huge<HIER>(t, d_elems, s.rs, s.d, (int64_t)1 << s.lg, s.toff, st));
       }
     }

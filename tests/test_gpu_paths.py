@@ -291,6 +291,20 @@ def test_builds_near_full_load(R, cuda, oracle_mod, bucket, keys):
     assert _best_ms(cuda, build) < 1e-4 * keys
 
 
+@pytest.mark.parametrize("alpha,bucket", [(0.2, 5), (1.0, 1), (0.95, 16)])
+def test_builds_of_several_crowded_long_sets(R, cuda, oracle_mod, alpha, bucket):
+    """Sets of 2^16 keys and more, crowded by a repeated key or by their load,
+    among others that are not: the crowded ones are listed in any order."""
+    rng = np.random.default_rng(0x5EED7E50)
+    rows = []
+    for i, d in enumerate((65536, 65535, 124000, 70000, 66000, 124000)):
+        x = rng.choice(1 << 27, d, replace=False)
+        if i % 2 == 0:
+            x[rng.choice(d, 400, replace=False)] = x[0]
+        rows += [x, np.arange(i)]
+    _check_build(R, cuda, oracle_mod, rows, alpha, bucket, False)
+
+
 def test_builds_of_all_bucket_sizes_from_several_threads(R, cuda):
     """Each thread builds tables of its own bucket size on its own stream: the
     shared memory that a tile takes differs by bucket size."""
