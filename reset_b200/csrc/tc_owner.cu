@@ -31,16 +31,21 @@
 //   CUB exclusive scan  group offsets
 //   own_scatter_kernel  (first chunk, keys) of every edge's prober,
 //                       grouped by owner
-//   own_classify_kernel one of three bins per owner:
+//   own_classify_kernel one of four bins per owner:
 //     CTA    large groups (or sets above a warp's share of shared memory):
 //            the whole CTA stages the set, its warps split the probers,
 //            groups of more than kSeg probers are cut into several units;
 //     warp   a warp stages the set in its own region and walks the probers;
+//     large  sets above a CTA's share: one CTA per SM stages them in 32768
+//            slots;
 //     direct small groups, where staging costs more than it saves, and
 //            sets too large for shared memory: probes go to the HBM table,
 //            flattened across the lanes (thread granularity).
-//   tc_owner_kernel     one persistent launch: CTA units, then warp owners,
-//                       then direct owners, each from its own work counter.
+//   tc_owner_kernel     one persistent launch: CTA units, then direct units,
+//                       warp owners and direct owners, each from its own work
+//                       counter.
+//   tc_owner_large_kernel  only for tables that have larger sets: large units,
+//                       then the direct units of still larger ones.
 //
 // Bound by the shared-memory pipe: a lookup's slot read takes 3.1 wavefronts
 // for 32 random banks, 25 of the ~40 wavefronts of a step of 256 keys, at
@@ -400,14 +405,38 @@ constexpr int kCtaProbers = 128;  // groups above this, or with this many keys
 constexpr int kCtaKeys = 8192;    // to look up, are CTA work
 static_assert((kWTab & (kWTab - 1)) == 0 && kTake <= 32 && kRing >= 64, "staged table shapes");
 
-// Bin of every owner with a non-empty group (see the file comment).
-// ctr[0] CTA units, ctr[1] warp owners, ctr[2] small direct owners,
-// ctr[6] direct units.
+// Sets of more than kTab / 2 keys, by a launch of its own: one CTA of 1024
+// threads per SM with a table of 128 KB, up to 5/8 full (the reference's tables
+// of up to 20480 slots, at any load).  The direct units of larger sets are in
+// this launch too: they read HBM tables through L1, of which tc_owner_kernel's
+// five tables leave nothing.  500 rows of 8000 keys among 20,000 vertices, ms a
+// count, probing HBM tables in tc_owner_kernel / this way: alpha 0.5, 4 slots
+// 53 / 3.3 (staged whole with 20480 slots, 4.7); alpha 0.2, 5 slots 32 / 3.4.
+constexpr int kLT = 1024;
+constexpr int kLW = kLT / 32;
+constexpr int kLTab = 32768;
+constexpr int kLargeKeys = 20480;
+constexpr int kLSeg = 2048;  // probers per large unit
+constexpr int kLDirSeg = 16;  // ... per direct unit: 32 rows of 30,000 keys held one warp 7 ms
+constexpr size_t kLargeSmem = sizeof(int) * (kLTab + kLW * 32 * kQueueLane) + 8 * kLW * kRing;
+
+// Lists of the bins, and the counters in ctr: entries, then the cursors.
+enum : int {
+  kCtrUnits = 0, kCtrWarp = 1, kCtrDirect = 2, kCtrDirectUnits = 6,
+  kCtrUnitsNext = 3, kCtrWarpNext = 4, kCtrDirectNext = 5, kCtrDirectUnitsNext = 7,
+  kCtrLarge = 8, kCtrLargeDirect = 9, kCtrLargeNext = 10, kCtrLargeDirectNext = 11,
+  kCtrs = 12
+};
+
+// Bin of every owner with a non-empty group (see the file comment).  The lists
+// of the large launch grow from the ends of the other launch's: an owner is in
+// one bin, so they do not meet.
 __global__ void __launch_bounds__(kOT)
     own_classify_kernel(const int4* __restrict__ desc, const int32_t* __restrict__ goff,
                         const int2* __restrict__ ent, int32_t n, int b, float alpha,
                         int2* __restrict__ units, int32_t* __restrict__ wlist,
                         int32_t* __restrict__ dlist, int2* __restrict__ dunits,
+                        int2* __restrict__ units_last, int2* __restrict__ dunits_last,
                         int32_t* __restrict__ ctr) {
   const int lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -427,11 +456,18 @@ __global__ void __launch_bounds__(kOT)
           big = work >= kCtaKeys;
         }
         // staging pays when there are at most ~4 slots to insert per lookup;
-        // a staged table is at most half full, and probing rows (no longer
-        // than the owner's) of 2^20 keys keep a unit's quads within 32 bits
-        if (keys > kTab / 2 || d.y > (1 << 20) || !(P > kCtaProbers || T <= 4 * work)) {
-          bin = P > 32 ? 3 : 2;
-          if (bin == 3) nunits = (P + kDirSeg - 1) / kDirSeg;
+        // a CTA's staged table is at most half full, and probing rows (no
+        // longer than the owner's) of 2^20 keys keep a unit's quads within 32
+        // bits
+        const bool small = keys <= kTab / 2;
+        if ((!small && keys > kLargeKeys) || d.y > (1 << 20) ||
+            !(P > kCtaProbers || T <= 4 * work)) {
+          bin = P <= 32 ? 2 : small ? 3 : 5;
+          const int seg = bin == 5 ? kLDirSeg : kDirSeg;
+          if (bin != 2) nunits = (P + seg - 1) / seg;
+        } else if (!small) {
+          bin = 4;
+          nunits = (P + kLSeg - 1) / kLSeg;
         } else if (big || keys > kWTab / 4) {
           bin = 0;
           nunits = (P + kSeg - 1) / kSeg;
@@ -441,23 +477,26 @@ __global__ void __launch_bounds__(kOT)
       }
     }
     // warp-aggregated appends
-#pragma unroll
-    for (int which = 0; which <= 3; which += 3) {
+    auto append = [&](int which, int at, int2* list, int step) {
       int tot;
       const int pre = warp_excl_scan(bin == which ? nunits : 0, &tot);
-      int* c = ctr + (which == 0 ? 0 : 6);
       int b0 = 0;
-      if (lane == 0 && tot) b0 = atomicAdd(c, tot);
+      if (lane == 0 && tot) b0 = atomicAdd(ctr + at, tot);
       b0 = __shfl_sync(kFull, b0, 0);
-      int2* u = which == 0 ? units : dunits;
       if (bin == which)
-        for (int s = 0; s < nunits; ++s) u[b0 + pre + s] = make_int2((int)w, s);
+        for (int s = 0; s < nunits; ++s) list[step * (b0 + pre + s)] = make_int2((int)w, s);
+    };
+    append(0, kCtrUnits, units, 1);
+    append(3, kCtrDirectUnits, dunits, 1);
+    if (__any_sync(kFull, bin >= 4)) {
+      append(4, kCtrLarge, units_last, -1);
+      append(5, kCtrLargeDirect, dunits_last, -1);
     }
 #pragma unroll
     for (int which = 1; which <= 2; ++which) {
       const unsigned bm = __ballot_sync(kFull, bin == which);
       int b0 = 0;
-      if (lane == 0 && bm) b0 = atomicAdd(ctr + which, __popc(bm));
+      if (lane == 0 && bm) b0 = atomicAdd(ctr + (which == 1 ? kCtrWarp : kCtrDirect), __popc(bm));
       b0 = __shfl_sync(kFull, b0, 0);
       if (bin == which) (which == 1 ? wlist : dlist)[b0 + __popc(bm & lanemask_lt())] = (int)w;
     }
@@ -478,7 +517,7 @@ struct Staged {
     return (h + 1) & ((1u << LG) - 1u);
   }
   static __device__ __forceinline__ int key(int s) { return s & 0x7fffffff; }
-  // (ends: the table is at most half full)
+  // (ends: the table is at most 5/8 full)
   __device__ __forceinline__ void insert(int y) const {
     unsigned h = home(y);
     int old = atomicCAS(S + h, kFree, y);
@@ -631,6 +670,90 @@ __device__ __forceinline__ unsigned stream_rows(const int2* __restrict__ ent, Gr
   return hits;
 }
 
+// This warp's `hits` credited to owner w (OWN; warp-collective).
+template <bool OWN>
+__device__ __forceinline__ void credit(unsigned long long* owner_hits, int w,
+                                       unsigned long long hits) {
+  if (OWN) {
+    const unsigned long long d = warp_sum_u64(hits);
+    if ((threadIdx.x & 31) == 0 && d) atomicAdd(owner_hits + w, d);
+  }
+}
+
+// CTA units: the whole CTA (NT threads) stages one set, its warps share the
+// SEG probers of a unit; unit i at units[STEP * i].  Returns this lane's hits.
+template <int LG, int NT, int SEG, int STEP, bool OWN>
+__device__ __forceinline__ unsigned long long cta_units(
+    const Staged<LG>& st, const int4* __restrict__ desc, const int32_t* __restrict__ goff,
+    const int2* __restrict__ ent, const int4* __restrict__ quads, unsigned none,
+    const int2* __restrict__ units, int n_units, int32_t* __restrict__ cursor,
+    const int32_t* __restrict__ table, int64_t bn, int b, OpenQueue& open, RingRow* ring,
+    unsigned long long* __restrict__ owner_hits) {
+  __shared__ int s_item, s_next;
+  const int tid = threadIdx.x, lane = tid & 31;
+  unsigned long long hits = 0;
+  for (;;) {
+    if (tid == 0) {
+      s_item = atomicAdd(cursor, 1);
+      s_next = 0;
+    }
+    __syncthreads();
+    const int ui = s_item;
+    if (ui >= n_units) break;
+    const int2 unit = __ldg(units + STEP * ui);
+    const int4 dw = __ldg(desc + unit.x);
+    stage_set(st, table, desc_toff(dw), desc_lg(dw), bn, b, tid, NT, [] { __syncthreads(); });
+    const int g0 = __ldg(goff + unit.x) + unit.y * SEG;
+    const int g1 = min(__ldg(goff + unit.x + 1), g0 + SEG);
+    unsigned long long h = stream_rows(
+        ent,
+        [&] {
+          int g = 0;
+          if (lane == 0) g = g0 + atomicAdd(&s_next, kTake);
+          g = __shfl_sync(kFull, g, 0);
+          return make_int2(g, max(0, min(kTake, g1 - g)));
+        },
+        quads, none, st, open, ring);
+    h += open.drain(st);
+    credit<OWN>(owner_hits, unit.x, h);
+    hits += h;
+    __syncthreads();
+  }
+  return hits;
+}
+
+// Direct units: up to SEG probers of one owner whose table stays in HBM, 32
+// probers at a time, their probes flattened across the lanes; unit i at
+// dunits[STEP * i].
+template <bool HIER, int SEG, int STEP, bool OWN>
+__device__ __forceinline__ unsigned long long direct_units(
+    const int4* __restrict__ desc, const int32_t* __restrict__ goff, const int2* __restrict__ ent,
+    const int32_t* __restrict__ rows, const int2* __restrict__ dunits, int n_dunits,
+    int32_t* __restrict__ cursor, const int32_t* __restrict__ table, int64_t bn, int b, int lg_max,
+    unsigned long long* __restrict__ owner_hits, int32_t* __restrict__ status) {
+  const int lane = threadIdx.x & 31;
+  unsigned long long hits = 0;
+  for (;;) {
+    int ui = 0;
+    if (lane == 0) ui = atomicAdd(cursor, 1);
+    ui = __shfl_sync(kFull, ui, 0);
+    if (ui >= n_dunits) break;
+    const int2 unit = __ldg(dunits + STEP * ui);
+    const int4 dw = __ldg(desc + unit.x);
+    const int g0 = __ldg(goff + unit.x) + unit.y * SEG;
+    const int g1 = min(__ldg(goff + unit.x + 1), g0 + SEG);
+    unsigned long long h = 0;
+    for (int g = g0; g < g1; g += 32) {
+      const int2 e = g + lane < g1 ? __ldg(ent + g + lane) : make_int2(0, 0);
+      h += flat_probe<HIER, PaddedRows>(rows, table, e.y, e.x, desc_toff(dw), desc_lg(dw), lg_max,
+                                        bn, b, status, [](int) {});
+    }
+    credit<OWN>(owner_hits, unit.x, h);
+    hits += h;
+  }
+  return hits;
+}
+
 // OWN: every owner's hits are also added to owner_hits[owner] (per-graph
 // counts of a batch of disjoint graphs are sums over their vertex ranges).
 template <bool HIER, bool OWN = false>
@@ -644,78 +767,25 @@ __global__ void __launch_bounds__(kTT, 5)
                     unsigned long long* __restrict__ count,
                     unsigned long long* __restrict__ owner_hits, int32_t* __restrict__ status) {
   extern __shared__ __align__(128) int sm[];  // the CTA's staged table or the warps', queues, rings
-  __shared__ int s_item, s_next;
   constexpr int kLgTab = 31 - __builtin_clz(kTab), kLgWTab = 31 - __builtin_clz(kWTab);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int4* quads = reinterpret_cast<const int4*>(rows);
   int* queue = sm + kTab + warp * 32 * kQueueLane;
   RingRow* ring = reinterpret_cast<RingRow*>(sm + kTab + kTW * 32 * kQueueLane) + warp * kRing;
   OpenQueue open{queue + lane};
-  unsigned long long hits = 0;
-  const int n_units = ctr[0], n_warp = ctr[1], n_direct = ctr[2], n_dunits = ctr[6];
-  // this warp's hits since h0 credited to owner w (warp-collective)
-  auto credit = [&](int w, unsigned long long h0) {
-    if (OWN) {
-      const unsigned long long d = warp_sum_u64(hits - h0);
-      if (lane == 0 && d) atomicAdd(owner_hits + w, d);
-    }
-  };
-
-  // ---- CTA units: the whole CTA stages one set, warps share its probers
-  for (;;) {
-    if (tid == 0) {
-      s_item = atomicAdd(ctr + 3, 1);
-      s_next = 0;
-    }
-    __syncthreads();
-    const int ui = s_item;
-    if (ui >= n_units) break;
-    const int2 unit = __ldg(units + ui);
-    const int4 dw = __ldg(desc + unit.x);
-    const int lg = desc_lg(dw);
-    const Staged<kLgTab> st{sm};
-    stage_set(st, table, desc_toff(dw), lg, bn, b, tid, kTT, [] { __syncthreads(); });
-    const int g0 = __ldg(goff + unit.x) + unit.y * kSeg;
-    const int g1 = min(__ldg(goff + unit.x + 1), g0 + kSeg);
-    const unsigned long long h0 = hits;
-    hits += stream_rows(
-        ent,
-        [&] {
-          int g = 0;
-          if (lane == 0) g = g0 + atomicAdd(&s_next, kTake);
-          g = __shfl_sync(kFull, g, 0);
-          return make_int2(g, max(0, min(kTake, g1 - g)));
-        },
-        quads, none, st, open, ring);
-    hits += open.drain(st);
-    credit(unit.x, h0);
-    __syncthreads();
-  }
-
-  // ---- direct units: up to kDirSeg probers of one owner whose table stays
-  // in HBM, 32 probers at a time, their probes flattened across the lanes
-  for (;;) {
-    int ui = 0;
-    if (lane == 0) ui = atomicAdd(ctr + 7, 1);
-    ui = __shfl_sync(kFull, ui, 0);
-    if (ui >= n_dunits) break;
-    const int2 unit = __ldg(dunits + ui);
-    const int4 dw = __ldg(desc + unit.x);
-    const int g0 = __ldg(goff + unit.x) + unit.y * kDirSeg;
-    const int g1 = min(__ldg(goff + unit.x + 1), g0 + kDirSeg);
-    const unsigned long long h0 = hits;
-    for (int g = g0; g < g1; g += 32) {
-      const int2 e = g + lane < g1 ? __ldg(ent + g + lane) : make_int2(0, 0);
-      hits += flat_probe<HIER, PaddedRows>(rows, table, e.y, e.x, desc_toff(dw), desc_lg(dw), lg_max,
-                               bn, b, status, [](int) {});
-    }
-    credit(unit.x, h0);
-  }
+  const int n_warp = ctr[kCtrWarp], n_direct = ctr[kCtrDirect];
+  unsigned long long hits =
+      cta_units<kLgTab, kTT, kSeg, 1, OWN>(Staged<kLgTab>{sm}, desc, goff, ent, quads, none, units,
+                                        ctr[kCtrUnits], ctr + kCtrUnitsNext, table, bn, b, open,
+                                        ring, owner_hits);
+  hits += direct_units<HIER, kDirSeg, 1, OWN>(desc, goff, ent, rows, dunits, ctr[kCtrDirectUnits],
+                                  ctr + kCtrDirectUnitsNext, table, bn, b, lg_max, owner_hits,
+                                  status);
 
   // ---- warp owners: each warp stages a set in its own region
   for (;;) {
     int wi = 0;
-    if (lane == 0) wi = atomicAdd(ctr + 4, 1);
+    if (lane == 0) wi = atomicAdd(ctr + kCtrWarpNext, 1);
     wi = __shfl_sync(kFull, wi, 0);
     if (wi >= n_warp) break;
     const int w = __ldg(wlist + wi);
@@ -724,9 +794,8 @@ __global__ void __launch_bounds__(kTT, 5)
     const Staged<kLgWTab> st{sm + warp * kWTab};
     stage_set(st, table, desc_toff(dw), lg, bn, b, lane, 32, [] { __syncwarp(); });
     const int g0 = __ldg(goff + w), g1 = __ldg(goff + w + 1);
-    const unsigned long long h0 = hits;
     int g = g0;
-    hits += stream_rows(
+    unsigned long long h = stream_rows(
         ent,
         [&] {
           const int2 r = make_int2(g, min(32, g1 - g));
@@ -734,15 +803,16 @@ __global__ void __launch_bounds__(kTT, 5)
           return r;
         },
         quads, none, st, open, ring);
-    hits += open.drain(st);
-    credit(w, h0);
+    h += open.drain(st);
+    credit<OWN>(owner_hits, w, h);
+    hits += h;
   }
 
   // ---- direct owners: 32 owners per warp, their (owner, prober) pairs
   // flattened across the lanes, probes into the HBM tables flattened again
   for (;;) {
     int ci = 0;
-    if (lane == 0) ci = atomicAdd(ctr + 5, 1);
+    if (lane == 0) ci = atomicAdd(ctr + kCtrDirectNext, 1);
     ci = __shfl_sync(kFull, ci, 0);
     const int64_t i = (int64_t)ci * 32 + lane;
     if ((int64_t)ci * 32 >= n_direct) break;
@@ -789,6 +859,31 @@ __global__ void __launch_bounds__(kTT, 5)
   if (lane == 0 && hits) atomicAdd(count, hits);
 }
 
+template <bool HIER, bool OWN = false>
+__global__ void __launch_bounds__(kLT, 1)
+    tc_owner_large_kernel(const int4* __restrict__ desc, const int32_t* __restrict__ goff,
+                          const int2* __restrict__ ent, const int32_t* __restrict__ rows,
+                          unsigned none, const int2* __restrict__ units_last,
+                          const int2* __restrict__ dunits_last, int32_t* __restrict__ ctr,
+                          const int32_t* __restrict__ table, int64_t bn, int b, int lg_max,
+                          unsigned long long* __restrict__ count,
+                          unsigned long long* __restrict__ owner_hits,
+                          int32_t* __restrict__ status) {
+  extern __shared__ __align__(128) int sm[];  // the staged table, the warps' queues, rings
+  constexpr int kLg = 31 - __builtin_clz(kLTab);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  OpenQueue open{sm + kLTab + warp * 32 * kQueueLane + lane};
+  RingRow* ring = reinterpret_cast<RingRow*>(sm + kLTab + kLW * 32 * kQueueLane) + warp * kRing;
+  unsigned long long hits = cta_units<kLg, kLT, kLSeg, -1, OWN>(
+      Staged<kLg>{sm}, desc, goff, ent, reinterpret_cast<const int4*>(rows), none, units_last,
+      ctr[kCtrLarge], ctr + kCtrLargeNext, table, bn, b, open, ring, owner_hits);
+  hits += direct_units<HIER, kLDirSeg, -1, OWN>(desc, goff, ent, rows, dunits_last, ctr[kCtrLargeDirect],
+                                  ctr + kCtrLargeDirectNext, table, bn, b, lg_max, owner_hits,
+                                  status);
+  hits = warp_sum_u64(hits);
+  if (lane == 0 && hits) atomicAdd(count, hits);
+}
+
 // Key rows are put in class order from this many keys on: the passes cost
 // ~25 us and ~20 ps a key, and what they save grows with the row lengths.
 // Measured without / with (R-MAT, edge factor 16): scale 18 573 / 620 us,
@@ -821,11 +916,14 @@ reset_status tc_owner(const reset_table* t, const int4* kdesc, const int32_t* ko
   size_t cub_bytes = 0;
   RST_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, (int32_t*)nullptr,
                                          (int32_t*)nullptr, (int)(n + 1), st));
-  const int64_t max_units = n + m / kSeg + 1, max_dunits = n + m / kDirSeg + 1;
+  // the largest set, as own_classify_kernel bounds it
+  const bool large = t->alpha * (float)((int64_t)t->bucket << t->lg_max) > kTab / 2;
+  const int64_t max_units = n + m / kSeg + 1;
+  const int64_t max_dunits = n + m / (large ? kLDirSeg : kDirSeg) + 1;
   auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
   const size_t sz_cnt = al(sizeof(int32_t) * (n + 1)), sz_goff = sz_cnt;
   const size_t sz_ent = al(sizeof(int2) * m), sz_units = al(sizeof(int2) * max_units);
-  const size_t sz_list = al(sizeof(int32_t) * n), sz_ctr = al(sizeof(int32_t) * 8);
+  const size_t sz_list = al(sizeof(int32_t) * n), sz_ctr = al(sizeof(int32_t) * kCtrs);
   const size_t sz_dunits = al(sizeof(int2) * max_dunits);
   const int64_t pad_chunks = padded_chunks(n, mk) + 1;  // (and one without keys)
   const size_t sz_pad = al(8 * sizeof(int32_t) * (size_t)(pad_chunks + 1));
@@ -849,6 +947,7 @@ reset_status tc_owner(const reset_table* t, const int4* kdesc, const int32_t* ko
   int32_t* wlist = reinterpret_cast<int32_t*>(p); p += sz_list;
   int32_t* dlist = reinterpret_cast<int32_t*>(p); p += sz_list;
   int2* dunits = reinterpret_cast<int2*>(p); p += sz_dunits;
+  int2 *units_last = units + max_units - 1, *dunits_last = dunits + max_dunits - 1;
   int32_t* padded = reinterpret_cast<int32_t*>(p); p += sz_pad;
   int32_t* indeg = reinterpret_cast<int32_t*>(p); p += sz_deg;
   unsigned* hist = reinterpret_cast<unsigned*>(indeg + n);
@@ -898,7 +997,8 @@ reset_status tc_owner(const reset_table* t, const int4* kdesc, const int32_t* ko
   if (e == cudaSuccess) {
     note_launch();
     own_classify_kernel<<<grid_stride_blocks((n + kOT - 1) / kOT, sms * 8), kOT, 0, st>>>(
-        kdesc, goff, ent, t->n, t->bucket, t->alpha, units, wlist, dlist, dunits, ctr);
+        kdesc, goff, ent, t->n, t->bucket, t->alpha, units, wlist, dlist, dunits, units_last,
+        dunits_last, ctr);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) {
@@ -926,6 +1026,25 @@ reset_status tc_owner(const reset_table* t, const int4* kdesc, const int32_t* ko
 #undef OWN_LAUNCH
 #undef OWN_K
       e = cudaGetLastError();
+    }
+    if (e == cudaSuccess && large) {
+#define OWN_L(H, O)                                                                             \
+  do {                                                                                          \
+    e = cudaFuncSetAttribute(tc_owner_large_kernel<H, O>,                                       \
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLargeSmem);     \
+    if (e != cudaSuccess) break;                                                                \
+    note_launch();                                                                              \
+    tc_owner_large_kernel<H, O><<<sms, kLT, kLargeSmem, st>>>(                                  \
+        kdesc, goff, ent, padded, (unsigned)pad_chunks, units_last, dunits_last, ctr, t->d_table, \
+        t->bucket_num, t->bucket, t->lg_max, count, owner_hits, t->d_status);                   \
+    e = cudaGetLastError();                                                                     \
+  } while (0)
+      if (t->hier) {
+        if (own) OWN_L(true, true); else OWN_L(true, false);
+      } else {
+        if (own) OWN_L(false, true); else OWN_L(false, false);
+      }
+#undef OWN_L
     }
   }
   cudaFreeAsync(base, st);

@@ -212,6 +212,45 @@ def test_owner_grouped_set_sizes(R, cuda, d):
         t.free()
 
 
+@pytest.mark.parametrize("alpha,bucket", [(0.2, 5), (0.5, 4), (0.9, 2), (1.0, 5), (0.25, 1)])
+def test_owner_grouped_large_sets(R, cuda, oracle_mod, alpha, bucket):
+    """Sets around 4096 keys, the largest staged by five CTAs per SM, up to
+    20480, the largest staged at all, and past it; one more prober than a unit
+    takes; in one graph and in a batch of two."""
+    rng = np.random.default_rng(0x5EED7E60 + bucket)
+    n = 22000
+    sizes = [4095, 4096, 4097, 5000, 8192, 10000, 16384, 20479, 20480, 20481, 21900]
+    rows = [np.sort(rng.choice(n, d, replace=False)) for d in sizes]
+    rows += [np.sort(rng.choice(len(sizes), 3, replace=False)) for _ in range(2049)]
+    rows += [np.sort(rng.choice(n, 40, replace=False)) for _ in range(n - len(rows))]
+    off, cols = csr(rows)
+    d_off, d_cols = dev(off, cuda), dev(cols, cuda)
+    t = R.Table(d_off, d_cols, alpha=alpha, bucket=bucket)
+    want = oracle_mod.tc_merge(off, cols)
+    assert R.tc_count(t, d_off, d_cols, method=3) == want
+    t.check()
+    two_off = cuda.cat([d_off, d_off[1:] + d_cols.numel()])
+    two_cols = cuda.cat([d_cols, d_cols + n])
+    t2 = R.Table(two_off, two_cols, alpha=alpha, bucket=bucket, hierarchical=False)
+    counts = R.tc_count_batch(t2, two_off, two_cols, dev(np.array([0, n, 2 * n], np.int32), cuda))
+    assert counts.tolist() == [want, want]
+    t2.check()
+
+
+def test_owner_grouped_large_sets_are_staged(R, cuda):
+    """Many probers of large sets: faster in shared memory than from HBM."""
+    rng = np.random.default_rng(0x5EED7E70)
+    n = 20000
+    off, cols = csr([np.sort(rng.choice(n, 8000 if u < 300 else 60, replace=False))
+                     for u in range(n)])
+    d_off, d_cols = dev(off, cuda), dev(cols, cuda)
+    for alpha, bucket in [(0.5, 4), (0.9, 2)]:
+        t = R.Table(d_off, d_cols, alpha=alpha, bucket=bucket)
+        ms = {k: _best_ms(cuda, lambda: R.tc_count_async(t, d_off, d_cols, method=k), 3)
+              for k in (1, 3)}
+        assert ms[3] < ms[1]
+
+
 @pytest.mark.parametrize("n", [130, 600, 690, 700, 20000])
 def test_owner_grouped_room_for_rows(R, cuda, n):
     """As many keys in more and more rows: a chunk per 8 keys and row, then a
