@@ -140,7 +140,8 @@ reset_status reset_tc_count(const reset_table *t, const int32_t *d_off,
                             uint64_t *d_count, reset_stream_t stream);
 
 /* reset_tc_count with an explicit method (same count either way):
- *   0 = default: 3 from 2^19 edges on where d_cols is 16-byte aligned, else 1;
+ *   0 = default: 3 from 2^19 edges on where some row may have 96 keys or more
+ *       (by its table's size) and d_cols is 16-byte aligned, else 1;
  *   1 = edge-flattened: up to 32 edges per warp; pairs with at least
  *       warp_pair_min keys (reset_tuning, default 64) probed by the whole
  *       warp, smaller ones flattened across the lanes, both sides read from
@@ -179,9 +180,9 @@ reset_status reset_tc_count_ex(const reset_table *t, const int32_t *d_off,
  * d_graph_off[n_graphs] = n; edges stay inside their graph) with one table.
  * d_counts[g] (device u64) receives graph g's triangle count -- the
  * reference's dynamic_triangle_count (triangle-count/TC.cu:128-190) run once
- * per graph -- from a single owner-grouped count over the whole batch (each
- * triangle is credited to the graph of the vertex whose table it is found
- * in).  d_off/m must be the CSR the table was built on and d_cols 16-byte
+ * per graph -- from a single count over the whole batch, owner-grouped or, if
+ * no row has 96 keys, edge by edge (each triangle is credited to the graph of
+ * one of its vertices).  d_off/m must be the CSR the table was built on and d_cols 16-byte
  * aligned.  No host synchronisation. */
 reset_status reset_tc_count_batch(const reset_table *t, const int32_t *d_off,
                                   const int32_t *d_cols, int64_t m,

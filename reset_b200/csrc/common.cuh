@@ -152,6 +152,13 @@ reset_status tc_owner(const reset_table* t, const int4* kdesc, const int32_t* ko
                       const int32_t* ecols, const int32_t* echunk_rows, int64_t me,
                       unsigned long long* count, cudaStream_t st,
                       unsigned long long* owner_hits = nullptr);
+// The same count edge by edge (probe.cu), without scratch for the edges.
+reset_status tc_edges(const reset_table* t, const int4* kdesc, const int32_t* kcols,
+                      const int32_t* eoff, const int32_t* ecols, const int32_t* echunk_rows,
+                      int64_t me, unsigned long long* count, cudaStream_t st,
+                      unsigned long long* owner_hits = nullptr);
+// Whether the graph that t was built on is better counted so (probe.cu).
+bool tc_sparse(const reset_table* t);
 // Owner-grouped pair decisions (sss_owner.cu).  Scratch for n sets and up to
 // `cap` pairs comes from one stream-ordered allocation.
 struct PairOwnerScratch {

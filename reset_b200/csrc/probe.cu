@@ -34,16 +34,20 @@ constexpr int64_t kOwnerEdges = 1 << 19;  // edges from which they are grouped b
 
 // ----------------------------------------------------------------- TC ----
 
-template <bool HIER, int ROUNDS, bool LEAN>
+// desc, kcols: the key rows; off, cols, chunk_row: the edges (u, v), whose rows
+// are intersected.  OWN: every edge's hits are also added to owner_hits[u].
+template <bool HIER, int ROUNDS, bool LEAN, bool OWN = false>
 __global__ void __launch_bounds__(kThreads, 4)
-    tc_kernel(const int4* __restrict__ desc, const int32_t* __restrict__ off,
-              const int32_t* __restrict__ cols,
+    tc_kernel(const int4* __restrict__ desc, const int32_t* __restrict__ kcols,
+              const int32_t* __restrict__ off, const int32_t* __restrict__ cols,
               const int32_t* __restrict__ chunk_row, int32_t n, int64_t m,
               const int32_t* __restrict__ table, int64_t bn, int b, int lg_max,
               unsigned long long* __restrict__ count,
+              unsigned long long* __restrict__ owner_hits,
               unsigned long long* __restrict__ cursor, int lg_grab, int warp_pair_min,
               int32_t* __restrict__ status) {
   __shared__ int s_qx[kWarps][32 * ROUNDS], s_qh[kWarps][32 * ROUNDS];
+  __shared__ int s_own[OWN ? kWarps : 1][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // edges past off[n] have no row: never read them (nor their chunk rows)
   const int64_t me = min(m, (int64_t)__ldg(off + n));
@@ -82,6 +86,10 @@ __global__ void __launch_bounds__(kThreads, 4)
     unsigned bigm = __ballot_sync(kFull, big);
     const int64_t bt = desc_toff(B);
     const int blg = desc_lg(B);
+    if (OWN) {
+      s_own[warp][lane] = 0;
+      __syncwarp();
+    }
     while (bigm) {
       const int k = __ffs(bigm) - 1;
       bigm &= bigm - 1;
@@ -89,15 +97,29 @@ __global__ void __launch_bounds__(kThreads, 4)
       const int ka = __shfl_sync(kFull, A.x, k);
       const int klg = __shfl_sync(kFull, blg, k);
       const int64_t kt = __shfl_sync(kFull, bt, k);
+      int h;
       if (LEAN)
-        hits += warp_probe_pair_lean<HIER, ROUNDS>(cols + ka, ks, table + kt, klg, lg_max,
-                                                   bn, b, status, s_qx[warp], s_qh[warp]);
+        h = warp_probe_pair_lean<HIER, ROUNDS>(kcols + ka, ks, table + kt, klg, lg_max, bn, b,
+                                               status, s_qx[warp], s_qh[warp]);
       else
-        hits += warp_probe_pair<HIER, ROUNDS>(cols + ka, ks, table + kt, klg, lg_max,
-                                              bn, b, status, s_qx[warp], s_qh[warp]);
+        h = warp_probe_pair<HIER, ROUNDS>(kcols + ka, ks, table + kt, klg, lg_max, bn, b, status,
+                                          s_qx[warp], s_qh[warp]);
+      hits += h;
+      if (OWN) {
+        h = __reduce_add_sync(kFull, h);
+        if (lane == 0) s_own[warp][k] = h;
+      }
     }
-    hits += flat_probe<HIER>(cols, table, big ? 0 : s, A.x, bt, blg, lg_max,
-                             bn, b, status, [](int) {});
+    hits += flat_probe<HIER>(kcols, table, big ? 0 : s, A.x, bt, blg, lg_max, bn, b, status,
+                             [&](int k) {
+                               if (OWN) atomicAdd(&s_own[warp][k], 1);
+                             });
+    if (OWN) {
+      __syncwarp();
+      if (s_own[warp][lane])
+        atomicAdd(owner_hits + u, (unsigned long long)(unsigned)s_own[warp][lane]);
+      __syncwarp();
+    }
   }
   hits = warp_sum_u64(hits);
   if (lane == 0 && hits) atomicAdd(count, hits);
@@ -820,6 +842,59 @@ reset_status resolve_desc(const reset_table* t, const int32_t* d_off,
 
 }  // namespace
 
+// Edges of a graph without long rows have few keys to look up: the groups'
+// passes take longer than the lookups, edge by edge, do.  The bound on the
+// longest row is alpha times its table's slots, so it moves in steps of two.
+// Measured, us, methods 1 / 3: a grid of 4 M vertices 465 / 990; random graphs of
+// 2 M vertices, bound 64 with 10 edges each 1349 / 2691, with 14 2310 / 3318, bound
+// 128 with 20 4154 / 4211, with 28 7550 / 5474.  Past it hubs decide: 96 R-MAT
+// graphs of scales 8 to 12, bound 128, 269 / 249; scale 19 with 4 a vertex, bound
+// 256, 443 / 347.
+bool tc_sparse(const reset_table* t) {
+  return (double)t->alpha * t->bucket * t->max_len < 96;
+}
+
+reset_status tc_edges(const reset_table* t, const int4* kdesc, const int32_t* kcols,
+                      const int32_t* eoff, const int32_t* ecols, const int32_t* echunk_rows,
+                      int64_t me, unsigned long long* count, cudaStream_t st,
+                      unsigned long long* owner_hits) {
+  unsigned long long* cursor = nullptr;
+  RST_CUDA(scratch_malloc(reinterpret_cast<void**>(&cursor), sizeof(*cursor), st));
+  cudaError_t e = cudaMemsetAsync(cursor, 0, sizeof(*cursor), st);
+  const reset_tuning tun = tuning();
+#define TC_LAUNCH(...)                                                         \
+  do {                                                                         \
+    const int most = persistent_grid((const void*)tc_kernel<__VA_ARGS__>);     \
+    /* 32 edges at a time, fewer where that leaves warps idle (at least 4) */  \
+    int lg_grab = 5;                                                           \
+    while (lg_grab > 2 && (me >> lg_grab) < (int64_t)most * kWarps) --lg_grab; \
+    const int64_t g = clamp_grid(((me >> lg_grab) + kWarps) / kWarps, most);   \
+    note_launch();                                                             \
+    tc_kernel<__VA_ARGS__><<<(int)g, kThreads, 0, st>>>(                       \
+        kdesc, kcols, eoff, ecols, echunk_rows, t->n, me, t->d_table,          \
+        t->bucket_num, t->bucket, t->lg_max, count, owner_hits, cursor,        \
+        lg_grab, tun.warp_pair_min, t->d_status);                              \
+  } while (0)
+#define TC_VARIANT(H)                                                          \
+  do {                                                                         \
+    if (owner_hits) TC_LAUNCH(H, 4, false, true);                              \
+    else if (tun.probe_variant == 1 && tun.probe_rounds == 2) TC_LAUNCH(H, 2, true); \
+    else if (tun.probe_variant == 1 && tun.probe_rounds == 8) TC_LAUNCH(H, 8, true); \
+    else if (tun.probe_variant == 1) TC_LAUNCH(H, 4, true);                    \
+    else if (tun.probe_rounds == 2) TC_LAUNCH(H, 2, false);                    \
+    else TC_LAUNCH(H, 4, false);                                               \
+  } while (0)
+  if (e == cudaSuccess) {
+    if (t->hier) TC_VARIANT(true); else TC_VARIANT(false);
+    e = cudaGetLastError();
+  }
+#undef TC_VARIANT
+#undef TC_LAUNCH
+  cudaFreeAsync(cursor, st);
+  if (e != cudaSuccess) return cuda_fail(e, "tc_kernel launch", __FILE__, __LINE__);
+  return RESET_OK;
+}
+
 // Persistent pair kernel for the batched form: pair count read on the device
 // (np_dev), dynamic 32-pair chunks (cursor, zeroed by the caller), exact
 // rule.  No allocation and no synchronisation, so it can be captured.
@@ -894,12 +969,12 @@ reset_status reset_tc_count_ex(const reset_table* t, const int32_t* d_off,
   const bool cols16 = (reinterpret_cast<uintptr_t>(d_cols) & 15) == 0;
   if (method == 3 && !cols16)
     return arg_fail("method 3 needs a 16-byte aligned column array");
-  // Grouping the edges by owner takes seven launches and reads every edge
-  // twice; up to half a million edges the edge-flattened count, whose tables
-  // then lie in L2, is done by that time.  Measured (R-MAT, methods 1 / 3):
-  // 10k edges 36 / 92 us, 213k 93 / 109, 441k 149 / 148, 909k 288 / 197.
+  // Up to half a million edges the edge-flattened count, whose tables then lie
+  // in L2, is done by the time that grouping takes.  Measured (R-MAT, methods
+  // 1 / 3): 10k edges 36 / 92 us, 213k 93 / 109, 441k 149 / 148, 909k 288 / 197.
   if (method == 0)
-    method = cols16 && m >= kOwnerEdges && m <= INT32_MAX - 16 && t->n < INT32_MAX ? 3 : 1;
+    method = cols16 && m >= kOwnerEdges && m <= INT32_MAX - 16 && t->n < INT32_MAX &&
+                     !tc_sparse(t) ? 3 : 1;
   cudaStream_t st = as_stream(stream);
   RST_CUDA(cudaMemsetAsync(d_count, 0, sizeof(uint64_t), st));
   if (m == 0 || t->n == 0) return RESET_OK;
@@ -913,57 +988,15 @@ reset_status reset_tc_count_ex(const reset_table* t, const int32_t* d_off,
     RST_CHECK(make_chunk_rows(d_off, t->n, m, &owned_rows, st));
     rows = owned_rows;
   }
+  reset_status s = RESET_ERR_OOM;
   if (method == 3) {
-    reset_status s = tc_owner(t, ds.desc, d_off, d_cols, m, d_off, d_cols, rows, m, cnt, st);
-    if (s != RESET_ERR_OOM) {
-      if (owned_rows) cudaFreeAsync(owned_rows, st);
-      return s;
-    }
-    cudaGetLastError();  // no memory for the groups (nothing ran): edge by edge
+    s = tc_owner(t, ds.desc, d_off, d_cols, m, d_off, d_cols, rows, m, cnt, st);
+    if (s == RESET_ERR_OOM) cudaGetLastError();  // (nothing ran)
   }
-  unsigned long long* cursor = nullptr;
-  RST_CUDA(scratch_malloc(reinterpret_cast<void**>(&cursor), sizeof(*cursor), st));
-  cudaError_t e = cudaMemsetAsync(cursor, 0, sizeof(*cursor), st);
-  const reset_tuning tun = tuning();
-  const int wpm = tun.warp_pair_min;
-#define TC_LAUNCH(H, R, LN)                                                    \
-  do {                                                                         \
-    const int most = persistent_grid((const void*)tc_kernel<H, R, LN>);        \
-    /* 32 edges at a time, fewer where that leaves warps idle (at least 4) */  \
-    int lg_grab = 5;                                                           \
-    while (lg_grab > 2 && (m >> lg_grab) < (int64_t)most * kWarps) --lg_grab;  \
-    const int64_t g = clamp_grid(((m >> lg_grab) + kWarps) / kWarps, most);    \
-    note_launch();                                                             \
-    tc_kernel<H, R, LN><<<(int)g, kThreads, 0, st>>>(                          \
-        ds.desc, d_off, d_cols, rows, t->n, m, t->d_table, t->bucket_num,      \
-        t->bucket, t->lg_max, cnt, cursor, lg_grab, wpm, t->d_status);                  \
-  } while (0)
-  if (e == cudaSuccess) {
-    const bool lean = tun.probe_variant == 1;
-    if (t->hier) {
-      if (lean) {
-        if (tun.probe_rounds == 2) TC_LAUNCH(true, 2, true);
-        else if (tun.probe_rounds == 8) TC_LAUNCH(true, 8, true);
-        else TC_LAUNCH(true, 4, true);
-      } else {
-        if (tun.probe_rounds == 2) TC_LAUNCH(true, 2, false); else TC_LAUNCH(true, 4, false);
-      }
-    } else {
-      if (lean) {
-        if (tun.probe_rounds == 2) TC_LAUNCH(false, 2, true);
-        else if (tun.probe_rounds == 8) TC_LAUNCH(false, 8, true);
-        else TC_LAUNCH(false, 4, true);
-      } else {
-        if (tun.probe_rounds == 2) TC_LAUNCH(false, 2, false); else TC_LAUNCH(false, 4, false);
-      }
-    }
-    e = cudaGetLastError();
-  }
-#undef TC_LAUNCH
-  cudaFreeAsync(cursor, st);
+  if (s == RESET_ERR_OOM)
+    s = tc_edges(t, ds.desc, d_cols, d_off, d_cols, rows, m, cnt, st);
   if (owned_rows) cudaFreeAsync(owned_rows, st);
-  if (e != cudaSuccess) return cuda_fail(e, "tc_kernel launch", __FILE__, __LINE__);
-  return RESET_OK;
+  return s;
 }
 
 reset_status reset_tc_count(const reset_table* t, const int32_t* d_off,

@@ -1082,9 +1082,13 @@ extern "C" reset_status reset_tc_count_batch(const reset_table* t, const int32_t
   auto* total = reinterpret_cast<unsigned long long*>(buf + own_bytes);
   cudaError_t e = cudaMemsetAsync(buf, 0, own_bytes + 256, st);
   reset_status s = RESET_OK;
-  if (e == cudaSuccess)
-    s = tc_owner(t, t->d_desc, d_off, d_cols, m, d_off, d_cols, t->d_chunk_row, m, total, st,
-                 owner_hits);
+  if (e == cudaSuccess) {
+    if (!tc_sparse(t))
+      s = tc_owner(t, t->d_desc, d_off, d_cols, m, d_off, d_cols, t->d_chunk_row, m, total, st,
+                   owner_hits);
+    else
+      s = tc_edges(t, t->d_desc, d_cols, d_off, d_cols, t->d_chunk_row, m, total, st, owner_hits);
+  }
   if (e == cudaSuccess && s == RESET_OK)
     e = cub::DeviceSegmentedReduce::Sum(buf + own_bytes + 256, cub_bytes, owner_hits,
                                         reinterpret_cast<unsigned long long*>(d_counts), n_graphs,

@@ -283,6 +283,33 @@ def test_owner_grouped_classes_and_single_chunk_rows(R, cuda):
     t.check()
 
 
+@pytest.mark.parametrize("alpha,bucket", [(0.2, 5), (0.25, 1)])
+def test_sparse_graphs_edge_by_edge(R, cuda, oracle_mod, alpha, bucket):
+    """Graphs without long rows: whole and in a batch (every graph's own count)
+    edge by edge, and grouped on demand."""
+    rng = np.random.default_rng(0x5EED7E80)
+    graphs = []
+    for n, d in [(40000, 20), (700, 3), (1, 0), (33, 9), (90000, 5)]:
+        e = np.unique(rng.integers(0, n, (n * d, 2)), axis=0)
+        e = e[e[:, 0] < e[:, 1]]
+        off = np.zeros(n + 1, np.int32)
+        off[1:] = np.cumsum(np.bincount(e[:, 0], minlength=n))
+        graphs.append((off, e[:, 1].astype(np.int32)))
+    want = [oracle_mod.tc_merge(o, c) for o, c in graphs]
+    assert min(want[0], want[3]) > 0
+    starts = np.cumsum([0] + [o.size - 1 for o, _ in graphs]).astype(np.int32)
+    ends = np.cumsum([0] + [c.size for _, c in graphs])
+    off = np.concatenate([o[:-1] + z for (o, _), z in zip(graphs, ends)] + [ends[-1:]])
+    cols = np.concatenate([c + v for (_, c), v in zip(graphs, starts)])
+    d_off, d_cols = dev(off.astype(np.int32), cuda), dev(cols.astype(np.int32), cuda)
+    t = R.Table(d_off, d_cols, alpha=alpha, bucket=bucket, hierarchical=bucket == 1)
+    before = R._lib().reset_kernel_launches()
+    assert R.tc_count_batch(t, d_off, d_cols, dev(starts, cuda)).tolist() == want
+    assert R._lib().reset_kernel_launches() - before == 1  # (a grouped count takes five)
+    assert R.tc_count(t, d_off, d_cols) == R.tc_count(t, d_off, d_cols, method=3) == sum(want)
+    t.check()
+
+
 # ------------------------------------------------------------ table build --
 
 def _check_build(R, cuda, oracle_mod, rows, alpha, bucket, hier):
