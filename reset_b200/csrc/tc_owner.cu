@@ -26,7 +26,8 @@
 // once, where a group's probers bring hundreds of keys per slot.
 //
 // Passes (all stream-ordered, no host synchronisation):
-//   pad_rows_kernel     the key rows padded to whole 32-byte chunks
+//   pad_rows_kernel     the key rows padded to whole 32-byte chunks (long ones
+//                       by pad_long_kernel)
 //   own_count_kernel    owner of every edge; probers per owner
 //   CUB exclusive scan  group offsets
 //   own_scatter_kernel  (first chunk, keys) of every edge's prober,
@@ -102,6 +103,9 @@ struct PaddedRows {
 // in any other graph, whatever the lowest classes show.
 constexpr int kClasses = 24;
 constexpr int kClassRow = 2040;  // longest row put in order (chunk places in a byte)
+// Longer rows are padded by pad_long_kernel, in parts: 8 lanes take 7.6 ms for a
+// row of 900,000 keys.  (Launched where the table may have such sets.)
+constexpr int kPadPart = 8192;
 
 // A key row's length and lowest class in one word, so that an edge costs one
 // random read (of n words, in L2) for its target; rows of kLongRow keys or
@@ -195,7 +199,8 @@ __global__ void __launch_bounds__(kOT)
     pad_rows_kernel(const int32_t* __restrict__ koff, const int32_t* __restrict__ kcols,
                     int32_t n, int64_t mk, const uint8_t* __restrict__ cls,
                     int32_t* __restrict__ padded, int32_t* __restrict__ none,
-                    unsigned* __restrict__ info, ClassPlaces* __restrict__ places) {
+                    unsigned* __restrict__ info, ClassPlaces* __restrict__ places,
+                    int2* __restrict__ parts, int max_parts, int* __restrict__ n_parts) {
   __shared__ int s_cnt[kOT / 8][kClasses];
   constexpr int kPer = kClasses / 8;  // classes a lane looks after
   constexpr int kHold = 6;
@@ -260,13 +265,44 @@ __global__ void __launch_bounds__(kOT)
       }
       __syncwarp(group);
     } else {
-      for (int j = l8; j < d; j += 8) out[j] = mix_key(__ldg(kcols + s + j));
+      int at = max_parts;
+      const int np = (d + kPadPart - 1) / kPadPart;
+      if (d > kClassRow && max_parts > 0) {
+        if (l8 == 0) at = atomicAdd(n_parts, np);
+        at = __shfl_sync(group, at, 0, 8);
+      }
+      if (at <= max_parts - np) {  // left to pad_long_kernel
+        for (int i = l8; i < np; i += 8) parts[at + i] = make_int2((int)u, i * kPadPart);
+      } else {
+        if (at < max_parts) {  // (places it took without filling them)
+          for (int i = at + l8; i < max_parts; i += 8) parts[i] = make_int2(-1, 0);
+        }
+        for (int j = l8; j < d; j += 8) out[j] = mix_key(__ldg(kcols + s + j));
+      }
     }
     const int pad = d + l8;
     if (d > 0 && pad < ((d + 7) & ~7)) out[pad] = kNoKey;
     if (cls)
       for (int i = 0; i < kPer; ++i) places[u].at[l8 * kPer + i] = (uint8_t)place[i];
     if (l8 == 0) info[u] = (unsigned)min(max(d, 0), kLongRow) | (unsigned)lowest << 27;
+  }
+}
+
+// The long rows, a CTA per kPadPart keys.
+__global__ void __launch_bounds__(kOT)
+    pad_long_kernel(const int32_t* __restrict__ koff, const int32_t* __restrict__ kcols, int32_t n,
+                    int64_t mk, const int2* __restrict__ parts, int max_parts,
+                    const int* __restrict__ n_parts, int32_t* __restrict__ padded) {
+  const int np = min(*n_parts, max_parts);
+  for (int i = blockIdx.x; i < np; i += gridDim.x) {
+    const int2 part = __ldg(parts + i);
+    if (part.x < 0) continue;
+    const int s = max(__ldg(koff + part.x), 0);
+    const int d = (int)min((int64_t)(__ldg(koff + part.x + 1) - s), mk - s);
+    int32_t* out = padded + (int64_t)first_chunk(s, part.x, n, mk) * 8;
+    const int end = min(d, part.y + kPadPart);
+#pragma unroll 4
+    for (int j = part.y + threadIdx.x; j < end; j += kOT) out[j] = mix_key(__ldg(kcols + s + j));
   }
 }
 
@@ -425,7 +461,7 @@ enum : int {
   kCtrUnits = 0, kCtrWarp = 1, kCtrDirect = 2, kCtrDirectUnits = 6,
   kCtrUnitsNext = 3, kCtrWarpNext = 4, kCtrDirectNext = 5, kCtrDirectUnitsNext = 7,
   kCtrLarge = 8, kCtrLargeDirect = 9, kCtrLargeNext = 10, kCtrLargeDirectNext = 11,
-  kCtrs = 12
+  kCtrPadParts = 12, kCtrs = 13
 };
 
 // Bin of every owner with a non-empty group (see the file comment).  The lists
@@ -483,8 +519,16 @@ __global__ void __launch_bounds__(kOT)
       int b0 = 0;
       if (lane == 0 && tot) b0 = atomicAdd(ctr + at, tot);
       b0 = __shfl_sync(kFull, b0, 0);
-      if (bin == which)
-        for (int s = 0; s < nunits; ++s) list[step * (b0 + pre + s)] = make_int2((int)w, s);
+      // (a hub's many units by all lanes)
+      const int mine = bin == which ? nunits : 0;
+      if (mine <= 32)
+        for (int s = 0; s < mine; ++s) list[step * (b0 + pre + s)] = make_int2((int)w, s);
+      for (unsigned wide = __ballot_sync(kFull, mine > 32); wide; wide &= wide - 1) {
+        const int k = __ffs(wide) - 1;
+        const int hub = __shfl_sync(kFull, (int)w, k), from = __shfl_sync(kFull, b0 + pre, k);
+        const int ns = __shfl_sync(kFull, mine, k);
+        for (int s = lane; s < ns; s += 32) list[step * (from + s)] = make_int2(hub, s);
+      }
     };
     append(0, kCtrUnits, units, 1);
     append(3, kCtrDirectUnits, dunits, 1);
@@ -932,10 +976,15 @@ reset_status tc_owner(const reset_table* t, const int4* kdesc, const int32_t* ko
   const bool classes = koff == t->build_off && mk == t->m && mk >= kClassEdges;
   const size_t sz_deg = classes ? al(sizeof(int32_t) * ((size_t)n + kDegSteps)) : 0;
   const size_t sz_info = al(sizeof(unsigned) * (size_t)n);
+  // (rows of more than kClassRow keys: at most mk / kClassRow)
+  const bool pad_long = t->alpha * (float)((int64_t)t->bucket << t->lg_max) > kClassRow;
+  const int max_parts = pad_long ? (int)(mk / kPadPart + mk / kClassRow + 1) : 0;
+  const size_t sz_parts = al(sizeof(int2) * (size_t)max_parts);
   const size_t sz_cls = classes ? al((size_t)n) : 0;
   const size_t sz_places = classes ? al(sizeof(ClassPlaces) * (size_t)n) : 0;
   const size_t total = sz_cnt + sz_goff + sz_ent + sz_units + 2 * sz_list + sz_dunits +
-                       sz_ctr + sz_pad + sz_info + sz_deg + sz_cls + sz_places + al(cub_bytes);
+                       sz_ctr + sz_pad + sz_info + sz_deg + sz_cls + sz_places + sz_parts +
+                       al(cub_bytes);
   char* base = nullptr;
   RST_CUDA(scratch_malloc(reinterpret_cast<void**>(&base), total, st));
   char* p = base;
@@ -954,6 +1003,7 @@ reset_status tc_owner(const reset_table* t, const int4* kdesc, const int32_t* ko
   uint8_t* cls = classes ? reinterpret_cast<uint8_t*>(p) : nullptr; p += sz_cls;
   unsigned* info = reinterpret_cast<unsigned*>(p); p += sz_info;
   ClassPlaces* places = reinterpret_cast<ClassPlaces*>(p); p += sz_places;
+  int2* parts = reinterpret_cast<int2*>(p); p += sz_parts;
   void* cub_tmp = p;
 
   cudaError_t e = cudaMemsetAsync(cnt, 0, sz_cnt + sz_ctr, st);
@@ -975,7 +1025,13 @@ reset_status tc_owner(const reset_table* t, const int4* kdesc, const int32_t* ko
   if (e == cudaSuccess) {
     note_launch();
     pad_rows_kernel<<<grid_stride_blocks((n * 8 + kOT - 1) / kOT, sms * 16), kOT, 0, st>>>(
-        koff, kcols, t->n, mk, cls, padded, padded + pad_chunks * 8, info, places);
+        koff, kcols, t->n, mk, cls, padded, padded + pad_chunks * 8, info, places, parts,
+        max_parts, ctr + kCtrPadParts);
+    if (pad_long) {
+      note_launch();
+      pad_long_kernel<<<sms * 4, kOT, 0, st>>>(koff, kcols, t->n, mk, parts, max_parts,
+                                               ctr + kCtrPadParts, padded);
+    }
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) {

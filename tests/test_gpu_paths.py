@@ -251,6 +251,36 @@ def test_owner_grouped_large_sets_are_staged(R, cuda):
         assert ms[3] < ms[1]
 
 
+@pytest.mark.parametrize("d", [2040, 2041, 8192, 8193, 300_000])
+def test_owner_grouped_long_rows(R, cuda, oracle_mod, d):
+    """Rows padded in parts, at their limits; hubs whose units are many."""
+    rng = np.random.default_rng(0x5EED7E90 + d)
+    n = max(3000, d + 500)
+    rows = [np.sort(rng.choice(n, d, replace=False)) for _ in range(3)]
+    rows += [np.sort(rng.choice(n, 4, replace=False)) for _ in range(200)]
+    rows += [np.array([0, 1])] * 1000 + [np.zeros(0, np.int64)] * (n - 1203)
+    off, cols = csr(rows)
+    d_off, d_cols = dev(off, cuda), dev(cols, cuda)
+    want = oracle_mod.tc_merge(off, cols)
+    for alpha, bucket in ((0.2, 5), (0.25, 1)):
+        t = R.Table(d_off, d_cols, alpha=alpha, bucket=bucket)
+        assert R.tc_count(t, d_off, d_cols, method=3) == want
+        t.check()
+
+
+def test_owner_grouped_one_hub(R, cuda):
+    """One row of 900,000 keys, which 8 lanes took 4 ms and more to pad."""
+    n = 1_000_000
+    hub = np.arange(1, 900_001, dtype=np.int32)
+    rest = (np.arange(1, n)[:, None] * np.array([3, 5, 7]) + 11) % n
+    off = np.concatenate([[0], hub.size + 3 * np.arange(n)]).astype(np.int32)
+    d_off, d_cols = dev(off, cuda), dev(np.concatenate([hub, rest.ravel()]).astype(np.int32), cuda)
+    t = R.Table(d_off, d_cols)
+    assert R.tc_count(t, d_off, d_cols, method=3) == R.tc_count(t, d_off, d_cols, method=1)
+    assert _best_ms(cuda, lambda: R.tc_count_async(t, d_off, d_cols, method=3)) < 2
+    t.check()
+
+
 @pytest.mark.parametrize("n", [130, 600, 690, 700, 20000])
 def test_owner_grouped_room_for_rows(R, cuda, n):
     """As many keys in more and more rows: a chunk per 8 keys and row, then a
