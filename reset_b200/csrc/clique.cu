@@ -637,7 +637,8 @@ reset_status clique_probe(const reset_table* t, const int32_t* d_off, const int3
   return RESET_OK;
 }
 
-// The bit-row search (strictly ascending rows).  *d_count is added to.
+// The bit-row search (strictly ascending rows), or the hash-probe search where
+// its lists find no memory.  *d_count, 0 before, is the count.
 //
 // R-MAT scale 16, k = 5 (15.7M triangles): hash probes 62 ms, bit rows 1.77 ms.
 reset_status clique_bits(const reset_table* t, const int32_t* d_off, const int32_t* d_cols,
@@ -664,8 +665,11 @@ reset_status clique_bits(const reset_table* t, const int32_t* d_off, const int32
   const size_t sz_small = al(sizeof(int32_t) * ((size_t)t->n + 1));
   const size_t sz_edges = overflow ? al(sizeof(int32_t) * (size_t)m) : 0;
   char* base = nullptr;
-  RST_CUDA(scratch_malloc(reinterpret_cast<void**>(&base),
-                          sz_items + sz_small + sz_edges + al(sizeof(int32_t) * 8), st));
+  if (scratch_malloc(reinterpret_cast<void**>(&base),
+                     sz_items + sz_small + sz_edges + al(sizeof(int32_t) * 8), st) != cudaSuccess) {
+    cudaGetLastError();  // no memory for the work lists
+    return clique_probe(t, d_off, d_cols, m, k, (int64_t)rs.longest, nullptr, nullptr, d_count, st);
+  }
   int4* items = reinterpret_cast<int4*>(base);
   int32_t* small = reinterpret_cast<int32_t*>(base + sz_items);
   int32_t* elist = reinterpret_cast<int32_t*>(base + sz_items + sz_small);
@@ -692,6 +696,11 @@ reset_status clique_bits(const reset_table* t, const int32_t* d_off, const int32
     s = clique_probe(t, d_off, d_cols, m, k, (int64_t)rs.longest, elist, ctr + 4, d_count, st);
   cudaFreeAsync(base, st);
   if (e != cudaSuccess) return cuda_fail(e, "clique bit rows", __FILE__, __LINE__);
+  if (s == RESET_ERR_OOM) {  // the lists left no memory for the probes: all edges anew
+    cudaGetLastError();
+    RST_CUDA(cudaMemsetAsync(d_count, 0, sizeof(*d_count), st));
+    s = clique_probe(t, d_off, d_cols, m, k, (int64_t)rs.longest, nullptr, nullptr, d_count, st);
+  }
   return s;
 }
 

@@ -142,9 +142,15 @@ reset_status reset_tc_count_shard(const reset_table* t, const int32_t* d_key_off
   }
   int32_t* rows = nullptr;
   reset_status s = make_chunk_rows(d_edge_off, t->n, m_edges, &rows, st);
-  if (s == RESET_OK)
+  if (s == RESET_OK) {
+    unsigned long long* count = reinterpret_cast<unsigned long long*>(d_count);
     s = tc_owner(t, kdesc, d_key_off, d_key_cols, m_keys, d_edge_off, d_edge_cols, rows, m_edges,
-                 reinterpret_cast<unsigned long long*>(d_count), st);
+                 count, st);
+    if (s == RESET_ERR_OOM) {
+      cudaGetLastError();  // no memory for the groups (nothing ran)
+      s = tc_edges(t, kdesc, d_key_cols, d_edge_off, d_edge_cols, rows, m_edges, count, st);
+    }
+  }
   if (rows) cudaFreeAsync(rows, st);
   if (owned_desc) cudaFreeAsync(owned_desc, st);
   return s;

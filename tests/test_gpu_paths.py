@@ -733,3 +733,61 @@ def test_retrieval_of_many_slices(R, cuda):
         got = res[int(roff[q]):int(roff[q + 1])]
         assert int(cnt[q]) == want.numel() and cuda.equal(got[: want.numel()], want)
         assert bool((got[want.numel():] == -1).all())
+
+
+# ---------------------------------------------------------- scarce memory --
+
+@pytest.mark.parametrize("call", ["tc", "tc_batch", "tc_shard", "clique", "pattern"])
+def test_calls_where_memory_is_scarce(R, cuda, libreset, call):
+    """Calls whose larger scratch does not fit run without it: 8 M vertices,
+    with 400 MB (groups) or 80 MB (work lists, bit rows) left on the device."""
+    from reset_b200 import shard
+    rng = np.random.default_rng(0x5EED8300)
+    n = 8_000_000
+    core = [np.sort(rng.choice(np.arange(u + 1, 1200), 300, replace=False)) for u in range(200)]
+    core += [np.sort(rng.choice(np.arange(u + 1, 2101), 20, replace=False)) for u in range(200, 2000)]
+    deg = np.ones(n, np.int64)
+    deg[:2000] = [r.size for r in core]
+    off = np.concatenate([[0], np.cumsum(deg)])
+    cols = np.concatenate(core + [np.arange(2000, n) * 7 % 2000])
+    d_off, d_cols = dev(off.astype(np.int32), cuda), dev(cols.astype(np.int32), cuda)
+    if call == "tc_shard":
+        d_koff, d_kcols = shard.shard_csr(d_off, d_cols, 1, 0)
+    else:
+        d_koff, d_kcols = d_off, d_cols
+    t = R.Table(d_koff, d_kcols, alpha=0.25, bucket=1)
+    graphs = dev(np.array([0, 2000, 5_000_000, n], np.int32), cuda)
+    out = cuda.zeros(1, dtype=cuda.int64, device="cuda")
+    out3 = cuda.zeros(3, dtype=cuda.int64, device="cuda")
+
+    def run():
+        if call == "tc":
+            return R.tc_count_async(t, d_off, d_cols, out, method=3).tolist()
+        if call == "tc_batch":
+            return R.tc_count_batch(t, d_off, d_cols, graphs, out3).tolist()
+        if call == "tc_shard":
+            s = libreset.reset_tc_count_shard(
+                t.handle, d_koff.data_ptr(), d_kcols.data_ptr(), d_kcols.numel(),
+                d_off.data_ptr(), d_cols.data_ptr(), d_cols.numel(), out.data_ptr(),
+                cuda.cuda.current_stream().cuda_stream)
+            return s, out.tolist()
+        if call == "clique":
+            return R.clique_count(t, d_off, d_cols, 5)
+        return R.pattern_count(t, d_off, d_cols, R.PatternSpec(4, (0, 1, 2, 4), (0, 0, 1, 2), None,
+                                                               None, 2))
+
+    want = run()
+    assert sum(np.atleast_1d(want[-1] if isinstance(want, tuple) else want)) > 0
+    cuda.cuda.synchronize()
+    libreset.reset_release_cached_memory()
+    cuda.cuda.empty_cache()
+    left = (80 if call in ("clique", "pattern") else 400) << 20
+    ballast = cuda.empty(cuda.cuda.mem_get_info()[0] - left, dtype=cuda.uint8, device="cuda")
+    try:
+        got = run()
+        cuda.cuda.synchronize()
+    finally:
+        del ballast
+        cuda.cuda.empty_cache()
+    assert got == want
+    t.check()
