@@ -8,7 +8,9 @@
 namespace rst {
 
 // Row of edge e (warp-collective).  u0 is the row of the chunk's first edge;
-// row(e) = u0 + #{j : off[u0+1+j] <= e}, searched 32 rows at a time.
+// row(e) = u0 + #{j : off[u0+1+j] <= e}, searched 32 rows at a time, and past
+// 128 rows (a graph with many empty ones: 32 rows a step were 80 us for 6400) by
+// halving.
 __device__ __forceinline__ int row_of_edge(const int32_t* __restrict__ off,
                                            int n, int u0, int e) {
   const int lane = threadIdx.x & 31;
@@ -26,6 +28,18 @@ __device__ __forceinline__ int row_of_edge(const int32_t* __restrict__ off,
     if (c == 31 && q31 <= e) c = 32;
     if (row < 0 && c < 32) row = ub + c;
     if (__all_sync(kFull, row >= 0)) break;
+    if (ub - u0 >= 96) {
+      if (row < 0) {  // off[ub + 32] <= e
+        int lo = min(ub + 32, n), hi = n;
+        while (lo < hi) {
+          const int mid = lo + (hi - lo + 1) / 2;
+          if (__ldg(off + mid) <= e) lo = mid; else hi = mid - 1;
+        }
+        row = lo;
+      }
+      __syncwarp();
+      break;
+    }
   }
   return row;
 }
