@@ -69,8 +69,11 @@ constexpr int kPtWarps = kPtThreads / 32;
 // Scratch rows of all resident warps together stay below this; a graph
 // whose largest row would need more runs fewer warps.
 constexpr size_t kPtScratchBudget = size_t(1) << 30;
-// Bytes of bit rows at most (2x the L2; n = 46340 vertices get a whole matrix).
-constexpr int64_t kBitBudget = int64_t(1) << 28;
+// Bytes of bit rows at most (2x the L2; n = 46340 vertices get a whole matrix),
+// and per unit of the sum of the squared row lengths, which bounds the keys that
+// the second level looks up: clearing a matrix that hardly any lookup reads took
+// most of a call (40,000 vertices with 200 edges: 260 us, 88 without).
+constexpr int64_t kBitBudget = int64_t(1) << 28, kBitPerSquare = 64;
 // Rows shorter than this get no bit row of their own on larger graphs: their
 // hash table spans no more cache lines than the bit row's hits would.
 constexpr int kBitMinRow = 64;
@@ -80,6 +83,11 @@ constexpr int kBitMinRow = 64;
 constexpr int kPartDeep = 8, kPartFlat = 64;
 // ... and are made longer where there would be more parts than this.
 constexpr int64_t kMaxParts = int64_t(1) << 20;
+// Longest row up to which neither bit rows nor parts are used: a set is then a
+// step of a warp, and the launches that prepare them cost more than they save.
+// 10,000 vertices with 10 neighbours each, Q6 / Q4: 220 / 197 us with them, 146 / 142
+// without; 100 with one each 103 / 90 and 82 / 84.
+constexpr int kShortRows = 32;
 
 struct PatternDev {
   int32_t k, flags;
@@ -870,8 +878,11 @@ extern "C" reset_status reset_pattern_count(const reset_table* t, const int32_t*
   BitRows br{nullptr, nullptr, ((int64_t)t->n + 127) / 128 * 4};
   int64_t bit_rows = 0;
   int bit_min = 0;
-  if (stats.outside == 0) {
-    const int64_t most = kBitBudget / (4 * br.words);
+  const bool short_rows = stats.longest <= kShortRows;
+  if (stats.outside == 0 && !short_rows) {
+    const int64_t budget = (int64_t)std::min<unsigned long long>(
+        kBitBudget, std::max<unsigned long long>(1 << 20, kBitPerSquare * stats.squares));
+    const int64_t most = budget / (4 * br.words);
     if (t->n <= most) {
       bit_rows = t->n;
     } else {
@@ -885,7 +896,7 @@ extern "C" reset_status reset_pattern_count(const reset_table* t, const int32_t*
   // parts of long start edges: there are at most 2 * squares / part of them
   int part = 0;
   int64_t max_parts = 0;
-  if (pat.k > 3) {
+  if (pat.k > 3 && !short_rows) {
     const int least = pat.k > 4 ? kPartDeep : kPartFlat;
     const unsigned long long by_count = 2 * stats.squares / (unsigned long long)kMaxParts;
     part = (int)std::min<unsigned long long>(std::max<unsigned long long>(least, by_count), INT_MAX);
@@ -947,8 +958,12 @@ extern "C" reset_status reset_pattern_count(const reset_table* t, const int32_t*
   // them the walk does as well
   const bool bounded = (pat.flags & RESET_PATTERN_RESTRICT) && pat.restr[pat.k - 1] >= 0;
   const int64_t co_bytes = (int64_t)sizeof(int32_t) * t->n * t->n;
+  // (the visits at most: of |C_2| or |C_2|^2 per edge)
+  const double most_visits = pat.k > 4 ? stats.cubes : (double)stats.squares;
   const bool co_may = pat.pair && sorted && !bounded && bit_rows == t->n && part > 0 &&
-                      co_bytes <= kCoBudget;
+                      co_bytes <= kCoBudget &&
+                      (t->n <= kCoSmall ||
+                       most_visits >= (double)t->n * t->n * t->n / kCoVisits);
   int32_t* co = nullptr;
   if (e == cudaSuccess && part > 0) {
     const int step = (int)std::max<int64_t>(1, m >> 10);  // about 2^10 edges looked at

@@ -156,6 +156,41 @@ def test_patterns_with_bit_rows_for_hubs_only(R, cuda, oracle_mod):
 
 # ----------------------------------------------------- owner-grouped count --
 
+def _random_symmetric(rng, n, edges, hub):
+    """`edges` random edges and one vertex with `hub` neighbours."""
+    e = rng.integers(0, n, (edges, 2))
+    e = np.concatenate([e, np.stack([np.full(hub, 7), rng.choice(np.arange(8, n), hub, False)], 1)])
+    e = np.unique(np.concatenate([e, e[:, ::-1]]), axis=0)
+    e = e[e[:, 0] != e[:, 1]]
+    off = np.zeros(n + 1, np.int32)
+    off[1:] = np.cumsum(np.bincount(e[:, 0], minlength=n))
+    return off, e[:, 1].astype(np.int32)
+
+
+@pytest.mark.parametrize("n,edges,hub", [
+    (300, 3000, 0), (500, 1500, 29), (500, 1500, 40), (3000, 4000, 400), (40000, 300, 31),
+    (40000, 300, 200), (47000, 50000, 300)])
+def test_patterns_of_sparse_graphs(R, cuda, oracle_mod, n, edges, hub):
+    """Rows of at most 32 keys (no bit rows, no parts) and just more; few edges
+    on many vertices, whose bit matrix would be large."""
+    off, cols = _random_symmetric(np.random.default_rng(0x5EED8400 + n + hub), n, edges, hub)
+    d_off, d_cols = dev(off, cuda), dev(cols, cuda)
+    t = R.Table(d_off, d_cols, hierarchical=bool(hub % 2))
+    for name, p in _patterns(R).items():
+        assert R.pattern_count(t, d_off, d_cols, p) == _oracle_pattern(oracle_mod, off, cols, p), name
+    t.check()
+
+
+def test_patterns_do_not_pay_for_vertices_without_edges(R, cuda):
+    times = []
+    for n in (400, 40000):
+        off, cols = _random_symmetric(np.random.default_rng(0x5EED8500), n, 100, 0)
+        d_off, d_cols = dev(off, cuda), dev(cols, cuda)
+        t = R.Table(d_off, d_cols)
+        times.append(_best_ms(cuda, lambda: R.pattern_count(t, d_off, d_cols, "Q6"), 20))
+    assert times[1] <= 1.5 * times[0] + 0.02
+
+
 def _multiset_tc(off, cols):
     """The reference's count: every key of the shorter row (ties: the edge's
     source) looked up in the other row's set."""
