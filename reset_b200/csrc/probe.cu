@@ -784,14 +784,16 @@ reset_status ir_run(const reset_table* t, const int4* desc, const int32_t* docs,
                     const int64_t* res_off, int32_t* res, int32_t* stage,
                     int32_t* sl_cnt, int64_t* pos, int32_t* cnt,
                     int64_t* packed_off, cudaStream_t st, bool yield) {
-  // yield: one warp per slice and no persistent grid, so the blocks retire
-  // as they finish and the block scheduler can interleave other streams'
-  // (higher-priority) work; otherwise a persistent grid walks the slices
-  const int64_t per_slice = std::min<int64_t>((total_slices + kWarps - 1) / kWarps, INT32_MAX);
+  // yield: a warp per slice (or kGatherSlices of them) and no persistent grid,
+  // so the blocks retire as they finish and the block scheduler can interleave
+  // other streams' (higher-priority) work; otherwise a persistent grid walks
+  // the slices
+  auto blocks = [&](int64_t slices, const void* kernel) {
+    const int64_t want = std::min<int64_t>((total_slices + slices - 1) / slices, INT32_MAX);
+    return yield ? want : clamp_grid(want, persistent_grid(kernel));
+  };
   if (total_slices > 0) {
-    const int64_t g = yield ? per_slice
-                            : clamp_grid(per_slice,
-                                         persistent_grid((const void*)ir_slice_kernel<HIER>));
+    const int64_t g = blocks(kWarps, (const void*)ir_slice_kernel<HIER>);
     note_launch();
     ir_slice_kernel<HIER><<<(int)g, kThreads, 0, st>>>(
         desc, t->n, docs, query, qoff, nq, sl_off, stage, sl_cnt, t->d_table,
@@ -803,8 +805,7 @@ reset_status ir_run(const reset_table* t, const int4* desc, const int32_t* docs,
                       0, st>>>(sl_cnt, total_slices, pos);
   RST_CUDA(cudaGetLastError());
   if (total_slices > 0) {
-    const int64_t g = yield ? per_slice
-                            : clamp_grid(per_slice, persistent_grid((const void*)ir_gather_kernel));
+    const int64_t g = blocks(kWarps * kGatherSlices, (const void*)ir_gather_kernel);
     note_launch();
     ir_gather_kernel<<<(int)g, kThreads, 0, st>>>(sl_off, nq, sl_cnt, pos, stage, res_off,
                                                    res);

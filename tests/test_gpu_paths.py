@@ -770,6 +770,21 @@ def test_retrieval_of_many_slices(R, cuda):
         assert bool((got[want.numel():] == -1).all())
 
 
+def test_served_retrieval_of_many_slices(R, cuda):
+    """A request above the cost cap: a block per so many slices, the last one
+    with one of them."""
+    from reset_b200 import server
+    n = 512 * 64 * 150 + 5
+    rows = [cuda.arange(0, n, dtype=cuda.int32), cuda.arange(0, n, 7, dtype=cuda.int32)]
+    off = cuda.tensor(np.cumsum([0] + [r.numel() for r in rows]), dtype=cuda.int32).cuda()
+    t = R.Table(off, cuda.cat(rows).cuda())
+    with server.Server(max_batch_cost=100_000) as s:
+        ix = s.add_index(t)
+        for terms, want in (([0], rows[0]), ([0, 1], rows[1]), ([1, 0], rows[1])):
+            r = s.wait(s.submit_ir(ix, terms))
+            assert r.status == 0 and np.array_equal(r.docs, want.numpy())
+
+
 # ---------------------------------------------------------- scarce memory --
 
 @pytest.mark.parametrize("call", ["tc", "tc_batch", "tc_shard", "clique", "pattern"])
