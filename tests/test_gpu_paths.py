@@ -375,6 +375,40 @@ def test_sparse_graphs_edge_by_edge(R, cuda, oracle_mod, alpha, bucket):
     t.check()
 
 
+@pytest.mark.parametrize("kind", ["symmetric", "shuffled", "repeated", "batch"])
+def test_owner_grouped_classes_of_every_kind(R, cuda, kind):
+    """2^24 keys and more, rows in class order: rows that hold lower classes
+    than their own, out of order, with repeated keys, and a batch of graphs."""
+    gen = cuda.Generator(device="cuda")
+    gen.manual_seed(0x5EED7E24)
+    scale = 20 if kind in ("symmetric", "shuffled", "repeated") else 19
+    off, cols = R.gen_rmat(scale, 9, 0x5EED7E24, oriented=False)
+    n = off.numel() - 1
+    row = cuda.repeat_interleave(cuda.arange(n, device="cuda"), (off[1:] - off[:-1]).long())
+    if kind == "shuffled":
+        order = cuda.randperm(cols.numel(), generator=gen, device="cuda")
+        cols = cols[order[row[order].argsort(stable=True)]].contiguous()
+    if kind == "repeated":
+        twice = cuda.arange(cols.numel(), device="cuda") % 5 == 0
+        cols = cuda.repeat_interleave(cols, 1 + twice.long())
+        off = cuda.cat([cuda.zeros(1, device="cuda", dtype=cuda.int64),
+                        cuda.cumsum(cuda.bincount(cuda.repeat_interleave(row, 1 + twice.long()),
+                                                  minlength=n), 0)]).int()
+    if kind == "batch":
+        g = 3
+        cols = cuda.cat([cols + k * n for k in range(g)])
+        off = cuda.cat([off[:-1] + k * (cols.numel() // g) for k in range(g)] +
+                       [cuda.tensor([cols.numel()], dtype=cuda.int32, device="cuda")])
+    assert cols.numel() >= 1 << 24
+    t = R.Table(off, cols, alpha=0.25, bucket=1)
+    want = R.tc_count(t, off, cols, method=1)
+    if kind == "batch":
+        starts = cuda.arange(g + 1, dtype=cuda.int32, device="cuda") * n
+        assert R.tc_count_batch(t, off, cols, starts).tolist() == [want // g] * g
+    assert R.tc_count(t, off, cols, method=3) == want
+    t.check()
+
+
 # ------------------------------------------------------------ table build --
 
 def _check_build(R, cuda, oracle_mod, rows, alpha, bucket, hier):
