@@ -272,7 +272,7 @@ reset_status reset_prefix_candidates(const int32_t *d_off, const int32_t *d_toke
 /* The same with the outputs in the caller's device memory: alloc(bytes, ctx)
  * is called on the calling thread, twice, when the number of pairs is known,
  * and returns memory that `stream` may write at once, or NULL
- * (RESET_ERR_CUDA).  What it returned stays the caller's, on errors too. */
+ * (RESET_ERR_OOM).  What it returned stays the caller's, on errors too. */
 typedef void *(*reset_alloc_fn)(int64_t bytes, void *ctx);
 reset_status reset_prefix_candidates_alloc(const int32_t *d_off, const int32_t *d_tokens,
                                            int32_t n, int64_t m, int32_t universe_log2,

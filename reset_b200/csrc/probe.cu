@@ -216,7 +216,7 @@ __device__ __forceinline__ bool filter_stream(const int32_t* __restrict__ elems,
 template <bool HIER, bool FLOAT_RULE, int ROUNDS, bool LEAN, bool EARLY = false>
 __global__ void __launch_bounds__(kThreads, 4)
     sss_kernel(const int4* __restrict__ desc, int32_t n,
-               const int32_t* __restrict__ elems, int64_t n_elems,
+               const int32_t* __restrict__ elems,
                const int32_t* __restrict__ pa, const int32_t* __restrict__ pb,
                int64_t np, const int64_t* __restrict__ np_dev,
                unsigned long long* __restrict__ cursor, int lg_grab,
@@ -914,7 +914,7 @@ reset_status sss_launch_persistent(const reset_table* t, const int32_t* elems,
                                  persistent_grid((const void*)sss_kernel<H, false, R, LN, E>)); \
     note_launch();                                                             \
     sss_kernel<H, false, R, LN, E><<<(int)g, kThreads, 0, st>>>(               \
-        t->d_desc, t->n, elems, t->m, pa, pb, capacity, np_dev, cursor, 5,     \
+        t->d_desc, t->n, elems, pa, pb, capacity, np_dev, cursor, 5,           \
         t->d_table, t->bucket_num, t->bucket, t->lg_max, num, den, 0.f, wpm,   \
         flags, E ? nullptr : inter, t->d_status);                              \
   } while (0)
@@ -1037,7 +1037,7 @@ static reset_status sss_common(const reset_table* t, const int32_t* d_off,
     while (lg_grab > 0 && (np >> lg_grab) < (int64_t)most * kWarps) --lg_grab; \
     const int64_t g = clamp_grid(((np >> lg_grab) + kWarps) / kWarps, most); \
     note_launch(); sss_kernel<H, F, R, LN, ##__VA_ARGS__><<<(int)g, kThreads, 0, st>>>( \
-        ds.desc, t->n, d_elems, t->m, d_pa, d_pb, np, nullptr, nullptr, lg_grab, \
+        ds.desc, t->n, d_elems, d_pa, d_pb, np, nullptr, nullptr, lg_grab,   \
         t->d_table, t->bucket_num, t->bucket, t->lg_max, num, den, thr,       \
         tun.warp_pair_min, d_flags, d_inter, t->d_status);                    \
   } while (0)

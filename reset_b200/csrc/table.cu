@@ -411,10 +411,10 @@ __global__ void __launch_bounds__(kTileThreads)
   const int s0 = tile_first[blockIdx.x], s1 = tile_first[blockIdx.x + 1];
   int u = s0;
   while (u < s1) {
-    // Next segment: big sets are skipped (built by big_build_kernel or
-    // build_huge); a run is the maximal span of consecutive tile-sized
-    // sets.  Every warp finds it (the same answer, from L1-cached lengths),
-    // so no barrier waits for one warp's scan.
+    // Next segment: long sets are skipped (built after the tiles); a run is
+    // the maximal span of consecutive tile-sized sets.  Every warp finds it
+    // (the same answer, from L1-cached lengths), so no barrier waits for one
+    // warp's scan.
     int r = u;
     if (len[u] > LT) {
       r = -(u + 1);
@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(kTileThreads)
         r += 32;
       }
     }
-    if (r < 0) {  // a big set
+    if (r < 0) {  // a long set
       u = -r;
       continue;
     }
@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// blk_cnt (optional): occupied slots of every bucket item.
+// The runs that start in a bucket item (step 2 above).
 template <bool HIER>
 __global__ void __launch_bounds__(kThreads)
     long_fix_kernel(const int32_t* __restrict__ elems, const LongSet* __restrict__ sets, int n,

@@ -150,7 +150,7 @@ __device__ __forceinline__ int staged_batch(
 // in HBM, as in the reference kernel.
 template <bool HIER>
 __device__ __forceinline__ int global_batch(
-    int j0, int je, int4 du4, const int32_t* __restrict__ cols, int64_t n_cols,
+    int j0, int je, int4 du4, const int32_t* __restrict__ cols,
     const int4* __restrict__ desc, int n, const int32_t* __restrict__ table,
     int64_t bn, int b, int lg_max, int32_t* status) {
   const int lane = threadIdx.x & 31;
@@ -174,7 +174,7 @@ __device__ __forceinline__ int global_batch(
 template <bool HIER>
 __global__ void __launch_bounds__(kT, 2)
     tc_staged_kernel(const int4* __restrict__ desc,
-                     const int32_t* __restrict__ cols, int64_t n_cols, int32_t n,
+                     const int32_t* __restrict__ cols, int32_t n,
                      const int2* __restrict__ units,
                      const int32_t* __restrict__ n_units_p, int units_cap,
                      int32_t* __restrict__ cursors,
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(kT, 2)
                                    bn, b, lg_max, status);
     } else {
       for (int j0 = e0 + warp * 32; j0 < e1; j0 += kT)
-        hits += global_batch<HIER>(j0, e1, du4, cols, n_cols, desc, n, table, bn,
+        hits += global_batch<HIER>(j0, e1, du4, cols, desc, n, table, bn,
                                    b, lg_max, status);
     }
     __syncthreads();
@@ -344,11 +344,11 @@ reset_status tc_staged(const reset_table* t, const int4* desc,
       note_launch();
       if (t->hier)
         tc_staged_kernel<true><<<grid, kT, smem, st>>>(
-            desc, d_cols, m, t->n, units, ctr + 2, cap, ctr, t->d_table,
+            desc, d_cols, t->n, units, ctr + 2, cap, ctr, t->d_table,
             t->bucket_num, t->bucket, t->lg_max, count, t->d_status);
       else
         tc_staged_kernel<false><<<grid, kT, smem, st>>>(
-            desc, d_cols, m, t->n, units, ctr + 2, cap, ctr, t->d_table,
+            desc, d_cols, t->n, units, ctr + 2, cap, ctr, t->d_table,
             t->bucket_num, t->bucket, t->lg_max, count, t->d_status);
       e = cudaGetLastError();
     }
@@ -448,11 +448,11 @@ extern "C" reset_status reset_tc_count_noalloc(const reset_table* t,
   note_launch();
   if (t->hier)
     tc_staged_kernel<true><<<grid, kT, smem, st>>>(
-        t->d_desc, d_cols, m, t->n, units, ctr + 2, kNoAllocUnits, ctr, t->d_table,
+        t->d_desc, d_cols, t->n, units, ctr + 2, kNoAllocUnits, ctr, t->d_table,
         t->bucket_num, t->bucket, t->lg_max, cnt, t->d_status);
   else
     tc_staged_kernel<false><<<grid, kT, smem, st>>>(
-        t->d_desc, d_cols, m, t->n, units, ctr + 2, kNoAllocUnits, ctr, t->d_table,
+        t->d_desc, d_cols, t->n, units, ctr + 2, kNoAllocUnits, ctr, t->d_table,
         t->bucket_num, t->bucket, t->lg_max, cnt, t->d_status);
   RST_CUDA(cudaGetLastError());
   return RESET_OK;
