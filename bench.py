@@ -8,15 +8,18 @@ degree (ties by id), int32 CSR, generated on the device (synthetic: the
 reference's graph datasets are not available).
 
 One step = the hot path over the whole graph: build the per-vertex bucketed
-hash tables (hierarchical hash, alpha 0.2, 5 slots per bucket) emitting the
-hash-ordered rows in the same pass, then count triangles by probing.
+hash tables (hierarchical hash, autotuned load and slots per bucket) emitting
+the hash-ordered rows in the same pass, then count triangles by probing.
   value : TC edges/s with the CSR resident in HBM (device-timed, max over
           ranks), inputs (6+ GB of tables and rows) far larger than L2.
   e2e   : the same through the C ABI from pinned HOST buffers, with the
           H2D copy of the CSR and the D2H read of the count inside the timed
           region.
-  roofline: the probe kernel (tc_kernel) against measured HBM bandwidth,
-          with the algorithmic bytes sum_e (8*min(d+u, d+v) + 36) + 4(n+1).
+  roofline: owner-grouped, sum_e min(d+u, d+v) lookups against the rate at
+          which shared memory reads a slot per lookup (32 random banks take
+          3.1 wavefronts), with the DRAM traffic of a profiled launch beside
+          it; the other methods against measured HBM bandwidth, with the
+          algorithmic bytes sum_e (8*min(d+u, d+v) + 36) + 4(n+1).
   cpu_baseline: the CPU oracle (sorted-row merge, all host threads) on a
           bounded vertex sample of the same graph, rank 0 at N=1.
 
@@ -430,6 +433,26 @@ def run_ours(a, rank, world, local):
     except Exception:
         pass
 
+    timed = "the whole reset_tc_count_ex call (CUDA events on its stream)"
+    if a.tc_method in (0, 3):
+        rate = sum_s / (probe_avg / 1e3)
+        sms = torch.cuda.get_device_properties(0).multi_processor_count
+        mhz = peaks.get("sm_max_mhz") or 1965.0
+        smem = sms * mhz * 1e6 * 32 / 3.1
+        roofline = {"bound": "shared memory",
+                    "kernel": "tc_owner_kernel + its grouping passes", "timed": timed,
+                    "achieved": rate, "peak": smem, "unit": "lookups/s", "frac": rate / smem,
+                    "peak_source": f"{sms} SMs x {mhz:.0f} MHz x 32 lanes / 3.1 wavefronts "
+                                   "(ncu) per slot read of 32 random banks",
+                    "traffic": traffic, "traffic_source": traffic_note,
+                    "hbm": {"peak_gbs": hbm, "peak_source": peak_src,
+                            "frac": traffic and traffic / (probe_avg / 1e3) / 1e9 / hbm}}
+    else:
+        roofline = {"bound": "hbm", "kernel": ["", "tc_kernel", "tc_staged_kernel"][a.tc_method],
+                    "timed": timed, "achieved": achieved, "peak": hbm, "unit": "GB/s",
+                    "frac": achieved / hbm, "peak_source": peak_src, "traffic": traffic,
+                    "traffic_source": traffic_note, "algorithmic_bytes_per_launch": alg_bytes}
+
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world,
         "steps": a.steps, "warmup": a.warmup, "ms_per_step": step_ms,
@@ -451,16 +474,7 @@ def run_ours(a, rank, world, local):
                 "ms_per_step": e2e_step},
         "probe_only": {"value": weak_value(m, world, probe_avg), "unit": UNIT,
                        "ms_per_launch": probe_avg},
-        "roofline": {"bound": "hbm",
-                     "kernel": ["tc_owner_kernel + its grouping passes", "tc_kernel",
-                                "tc_staged_kernel",
-                                "tc_owner_kernel + its grouping passes"][a.tc_method],
-                     "timed": "the whole reset_tc_count_ex call (CUDA events on its stream)",
-                     "achieved": achieved,
-                     "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
-                     "peak_source": peak_src, "traffic": traffic,
-                     "traffic_source": traffic_note,
-                     "algorithmic_bytes_per_launch": alg_bytes},
+        "roofline": roofline,
         "gpu_launches": launches,
     }
     line["clocks"] = clk.summary()
