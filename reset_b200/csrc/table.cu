@@ -98,7 +98,6 @@ struct BuildInfo {
   int32_t max_len;
   int32_t n_long;   // sets whose table does not fit a tile
   int32_t n_huge;   // ... of kHugeKeys keys or more
-  int32_t n_crowded;  // ... of those, left to build_huge (after long_insert)
   unsigned long long long_keys, long_buckets;
   int64_t bucket_num;
 };
@@ -570,7 +569,8 @@ constexpr int kWalkMax = 256;
 constexpr int kRunMax = 96;
 
 struct LongSet {
-  int32_t u, rs, d, lg;
+  int32_t crowded;  // by its load: nothing is tried first
+  int32_t rs, d, lg;
   int64_t toff;
   int32_t key_item, bucket_item;  // its first items
 };
@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(1024)
     long_plan_kernel(const int32_t* __restrict__ off, const int32_t* __restrict__ len,
                      const int64_t* __restrict__ off64, const int32_t* __restrict__ list, int n,
                      int b, float all_keys, LongSet* __restrict__ sets,
-                     int32_t* __restrict__ crowded) {
+                     LongSet* __restrict__ huge, int32_t* __restrict__ crowded) {
   using Scan = cub::BlockScan<int, 1024>;
   __shared__ typename Scan::TempStorage tmp;
   int keys = 0, buckets = 0;  // items before this pass
@@ -598,16 +598,17 @@ __global__ void __launch_bounds__(1024)
     LongSet s{};
     int ki = 0, bi = 0;
     if (i < n) {
-      s.u = list[i];
-      s.rs = off[s.u];
-      s.d = off[s.u + 1] - s.rs;
-      const int l = len[s.u];
+      const int u = list[i];
+      s.rs = off[u];
+      s.d = off[u + 1] - s.rs;
+      const int l = len[u];
       s.lg = 31 - __clz(l);
-      s.toff = off64[s.u];
+      s.toff = off64[u];
       ki = (s.d + kKeyItem - 1) / kKeyItem;
       bi = (l + kBucketItem - 1) / kBucketItem;
-      crowded[i] = crowded_by_load((float)s.d / ((float)l * (float)b),
-                                   s.d >= kHugeKeys ? (float)s.d : all_keys);
+      s.crowded = crowded_by_load((float)s.d / ((float)l * (float)b),
+                                  s.d >= kHugeKeys ? (float)s.d : all_keys);
+      crowded[i] = s.crowded;
     }
     int total;
     __syncthreads();
@@ -625,6 +626,7 @@ __global__ void __launch_bounds__(1024)
     end.key_item = keys;
     end.bucket_item = buckets;
     sets[n] = end;
+    huge[0] = LongSet{};
   }
 }
 
@@ -646,10 +648,11 @@ __device__ __forceinline__ int long_set_of(const LongSet* __restrict__ sets, int
 
 __global__ void __launch_bounds__(kThreads)
     long_clear_kernel(const LongSet* __restrict__ sets, int n, int64_t bucket_num, int b,
-                      int32_t* __restrict__ table, const int32_t* __restrict__ crowded) {
+                      int32_t* __restrict__ table) {
   const int i = long_set_of<&LongSet::bucket_item>(sets, n, blockIdx.x);
-  if (i < 0 || crowded[i]) return;  // (crowded sets are cleared where they are built)
+  if (i < 0) return;
   const LongSet s = sets[i];
+  if (s.crowded) return;  // (cleared where it is built)
   const int h0 = ((int)blockIdx.x - s.bucket_item) * kBucketItem;
   const int q = min(kBucketItem, (1 << s.lg) - h0) >> 2;
   const int4 neg = make_int4(-1, -1, -1, -1);
@@ -665,8 +668,9 @@ __global__ void __launch_bounds__(kThreads)
                        int64_t bucket_num, int b, int lg_max, int32_t* __restrict__ table,
                        int32_t* __restrict__ crowded) {
   const int i = long_set_of<&LongSet::key_item>(sets, n, blockIdx.x);
-  if (i < 0 || *(volatile int32_t*)(crowded + i)) return;
+  if (i < 0) return;
   const LongSet s = sets[i];
+  if (s.crowded) return;
   const int j0 = ((int)blockIdx.x - s.key_item) * kKeyItem;
   int32_t* G = table + s.toff;
   const int lmask = (1 << s.lg) - 1;
@@ -750,18 +754,18 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // Crowded sets, sequentially, a CTA each (those of kHugeKeys keys or more are
-// listed for build_huge).
+// listed for build_huge, huge[0].d of them from huge[1] on).
 template <bool HIER>
 __global__ void __launch_bounds__(kThreads)
     long_crowded_kernel(const int32_t* __restrict__ elems, const LongSet* __restrict__ sets,
                         const int32_t* __restrict__ crowded, int64_t bucket_num, int b, int lg_max,
                         int32_t* __restrict__ table, LongSet* __restrict__ huge,
-                        BuildInfo* __restrict__ info, int32_t* __restrict__ status) {
+                        int32_t* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char fill[];
   if (!crowded[blockIdx.x]) return;
   const LongSet s = sets[blockIdx.x];
   if (s.d >= kHugeKeys) {
-    if (threadIdx.x == 0) huge[atomicAdd(&info->n_crowded, 1)] = s;
+    if (threadIdx.x == 0) huge[1 + atomicAdd(&huge->d, 1)] = s;
     return;
   }
   const int l = 1 << s.lg;
@@ -1177,7 +1181,7 @@ reset_status build_huge(const reset_table* t, const int32_t* d_elems, int64_t rs
 template <bool HIER>
 reset_status launch_builds(const reset_table* t, const int32_t* d_off, const int32_t* d_elems,
                            const int32_t* d_tile_first, int32_t n_tiles, const Geom& g,
-                           const int32_t* d_long, BuildInfo* d_info, const BuildInfo& info,
+                           const int32_t* d_long, const BuildInfo& info,
                            int32_t* d_hash_out, cudaStream_t st) {
   if (n_tiles > 0) {
     // (the same for every bucket size: other threads may be between here and a
@@ -1220,24 +1224,21 @@ reset_status launch_builds(const reset_table* t, const int32_t* d_off, const int
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, fill_smem));
     note_launch(5);
     long_plan_kernel<<<1, 1024, 0, st>>>(d_off, t->d_len, t->d_off64, d_long, n, b,
-                                         (float)info.long_keys, sets, crowded);
-    long_clear_kernel<<<(unsigned)bucket_items, kThreads, 0, st>>>(sets, n, bn, b, t->d_table,
-                                                                   crowded);
+                                         (float)info.long_keys, sets, huge, crowded);
+    long_clear_kernel<<<(unsigned)bucket_items, kThreads, 0, st>>>(sets, n, bn, b, t->d_table);
     long_insert_kernel<HIER><<<(unsigned)key_items, kThreads, 0, st>>>(
         d_elems, sets, n, bn, b, t->lg_max, t->d_table, crowded);
     long_fix_kernel<HIER><<<(unsigned)bucket_items, kThreads, 0, st>>>(
         d_elems, sets, n, bn, b, t->lg_max, t->d_table, crowded);
     long_crowded_kernel<HIER><<<n, kThreads, fill_smem, st>>>(
-        d_elems, sets, crowded, bn, b, t->lg_max, t->d_table, huge, d_info, t->d_status);
+        d_elems, sets, crowded, bn, b, t->lg_max, t->d_table, huge, t->d_status);
     RST_CUDA(cudaGetLastError());
     if (info.n_huge > 0) {  // one more sync, only for tables that have such sets
-      int32_t nc = 0;
-      std::vector<LongSet> list((size_t)info.n_huge);  // (the first nc are written)
-      RST_CUDA(cudaMemcpyAsync(&nc, &d_info->n_crowded, sizeof(nc), cudaMemcpyDeviceToHost, st));
+      std::vector<LongSet> list((size_t)info.n_huge + 1);
       RST_CUDA(cudaMemcpyAsync(list.data(), huge, sizeof(LongSet) * list.size(),
                                cudaMemcpyDeviceToHost, st));
       RST_CUDA(cudaStreamSynchronize(st));
-      for (int i = 0; i < nc; ++i) {
+      for (int i = 1; i <= list[0].d; ++i) {
         const LongSet& s = list[(size_t)i];
         RST_CHECK(build_huge<HIER>(t, d_elems, s.rs, s.d, (int64_t)1 << s.lg, s.toff, st));
       }
@@ -1379,9 +1380,9 @@ reset_status reset_table_build(const int32_t* d_off, const int32_t* d_elems,
   if (n > 0) {
     const reset_status rs =
         t->hier ? launch_builds<true>(t, d_off, d_elems, d_tile_first, (int32_t)n_tiles64, g,
-                                      d_long, d_info, info, d_hash_out, st)
+                                      d_long, info, d_hash_out, st)
                 : launch_builds<false>(t, d_off, d_elems, d_tile_first, (int32_t)n_tiles64, g,
-                                       d_long, d_info, info, d_hash_out, st);
+                                       d_long, info, d_hash_out, st);
     if (rs != RESET_OK) return fail(rs);
   }
   if (scratch) cudaFreeAsync(scratch, st);
