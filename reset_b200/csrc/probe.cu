@@ -319,7 +319,8 @@ __global__ void __launch_bounds__(kThreads, 4)
       int allowed = s - need;  // keys that may miss; negative: settled
       const int before = __shfl_up_sync(kFull, a, 1);
       const unsigned runs = __ballot_sync(kFull, ok && lane > 0 && before == a);
-      if (__popc(runs) >= kFilterRun - 1) {
+      if (__popc(runs) >= kFilterRun - 1 &&
+          __popc(__ballot_sync(kFull, allowed >= 0 && need > 0)) >= kFilterRun) {
         uint32_t* const bits = reinterpret_cast<uint32_t*>(qx);
         for (unsigned heads = ~runs; heads; heads &= heads - 1) {
           const int k = __ffs(heads) - 1;
