@@ -419,17 +419,18 @@ def run_ours(a, rank, world, local):
     peak_src = "measured" if hbm else "fallback"
     hbm = hbm or 6650.0
     achieved = alg_bytes / (probe_avg / 1e3) / 1e9
-    # DRAM bytes per launch of the count kernel from a committed ncu record
-    # of the same method, scale and slots per bucket (alpha within 0.05)
+    # DRAM bytes per launch of the count kernel from a committed ncu record of
+    # the same method and scale, nearest load (the kernel stages sets of its own:
+    # the table's load and slots per bucket change the few slots it reads)
     traffic, traffic_note = None, None
     try:
         prof = json.load(open(os.path.join(ROOT, "profiles", "tc_owner_kernel_traffic.json")))
         if a.tc_method in (0, 3):
-            for rec in prof["records"]:
-                if (rec["scale"] == a.scale and abs(rec["alpha"] - a.alpha) <= 0.05 + 1e-9
-                        and rec["bucket"] == a.bucket):
-                    traffic = rec["dram_bytes_per_launch"]
-                    traffic_note = rec["how"]
+            recs = [r for r in prof["records"] if r["scale"] == a.scale]
+            if recs:
+                rec = min(recs, key=lambda r: abs(r["alpha"] - a.alpha))
+                traffic = rec["dram_bytes_per_launch"]
+                traffic_note = f"alpha {rec['alpha']}, {rec['bucket']} slot: {rec['how']}"
     except Exception:
         pass
 
