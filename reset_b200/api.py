@@ -138,8 +138,9 @@ class Table:
             pass
 
 
-# reset_tc_count_ex methods: 0 default (owner-grouped when the columns are
-# 16-byte aligned, else edge-flattened), 1 edge-flattened, 2 vertex-staged,
+# reset_tc_count_ex methods: 0 default (owner-grouped from 2^19 edges on where
+# some row may have 96 keys or more and the columns are 16-byte aligned, else
+# edge-flattened), 1 edge-flattened, 2 vertex-staged,
 # 3 owner-grouped (probed tables staged in shared memory)
 TC_DEFAULT, TC_EDGE, TC_STAGED, TC_OWNER = 0, 1, 2, 3
 

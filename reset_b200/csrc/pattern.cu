@@ -880,8 +880,8 @@ extern "C" reset_status reset_pattern_count(const reset_table* t, const int32_t*
   int bit_min = 0;
   const bool short_rows = stats.longest <= kShortRows;
   if (stats.outside == 0 && !short_rows) {
-    const int64_t budget = (int64_t)std::min<unsigned long long>(
-        kBitBudget, std::max<unsigned long long>(1 << 20, kBitPerSquare * stats.squares));
+    const int64_t squares = (int64_t)std::min<unsigned long long>(stats.squares, kBitBudget);
+    const int64_t budget = std::min(kBitBudget, std::max<int64_t>(1 << 20, kBitPerSquare * squares));
     const int64_t most = budget / (4 * br.words);
     if (t->n <= most) {
       bit_rows = t->n;
