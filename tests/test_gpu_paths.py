@@ -544,6 +544,15 @@ def test_raw_pair_sizes(R, cuda, na, nb):
     assert R.intersect_count(dev(a, cuda), dev(b, cuda)) == int(np.isin(a, b).sum())
 
 
+@pytest.mark.parametrize("nb", [1, 100, 1025, 4096])
+def test_raw_pair_of_many_keys_and_few(R, cuda, nb):
+    """Several blocks per SM, each with the whole set of B."""
+    rng = np.random.default_rng(nb)
+    a = rng.integers(0, 6 * nb, 3_000_001).astype(np.int32)
+    b = rng.integers(0, 6 * nb, nb).astype(np.int32)
+    assert R.intersect_count(dev(a, cuda), dev(b, cuda)) == int(np.isin(a, b).sum())
+
+
 def test_raw_pair_of_more_than_2_to_the_30_keys(R, cuda):
     """The set of 2^32 slots, the largest: its index takes all 32 bits."""
     n = (1 << 30) + 5
