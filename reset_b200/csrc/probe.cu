@@ -993,7 +993,10 @@ reset_status reset_tc_count_ex(const reset_table* t, const int32_t* d_off,
   reset_status s = RESET_ERR_OOM;
   if (method == 3) {
     s = tc_owner(t, ds.desc, d_off, d_cols, m, d_off, d_cols, rows, m, cnt, st);
-    if (s == RESET_ERR_OOM) cudaGetLastError();  // (nothing ran)
+    if (s == RESET_ERR_OOM) {  // no memory for the groups
+      cudaGetLastError();
+      RST_CUDA(cudaMemsetAsync(d_count, 0, sizeof(uint64_t), st));
+    }
   }
   if (s == RESET_ERR_OOM)
     s = tc_edges(t, ds.desc, d_cols, d_off, d_cols, rows, m, cnt, st);

@@ -147,8 +147,11 @@ reset_status reset_tc_count_shard(const reset_table* t, const int32_t* d_key_off
     s = tc_owner(t, kdesc, d_key_off, d_key_cols, m_keys, d_edge_off, d_edge_cols, rows, m_edges,
                  count, st);
     if (s == RESET_ERR_OOM) {
-      cudaGetLastError();  // no memory for the groups (nothing ran)
-      s = tc_edges(t, kdesc, d_key_cols, d_edge_off, d_edge_cols, rows, m_edges, count, st);
+      cudaGetLastError();  // no memory for the groups
+      const cudaError_t e = cudaMemsetAsync(d_count, 0, sizeof(uint64_t), st);
+      s = e == cudaSuccess ? tc_edges(t, kdesc, d_key_cols, d_edge_off, d_edge_cols, rows, m_edges,
+                                      count, st)
+                           : cuda_fail(e, "cudaMemsetAsync", __FILE__, __LINE__);
     }
   }
   if (rows) cudaFreeAsync(rows, st);

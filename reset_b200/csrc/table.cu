@@ -29,8 +29,9 @@
 #include <cub/cub.cuh>
 
 #include <cstring>
+#include <memory>
 #include <mutex>
-#include <vector>
+#include <new>
 
 #include "common.cuh"
 #include "probe_common.cuh"
@@ -1234,12 +1235,14 @@ reset_status launch_builds(const reset_table* t, const int32_t* d_off, const int
         d_elems, sets, crowded, bn, b, t->lg_max, t->d_table, huge, t->d_status);
     RST_CUDA(cudaGetLastError());
     if (info.n_huge > 0) {  // one more sync, only for tables that have such sets
-      std::vector<LongSet> list((size_t)info.n_huge + 1);
-      RST_CUDA(cudaMemcpyAsync(list.data(), huge, sizeof(LongSet) * list.size(),
-                               cudaMemcpyDeviceToHost, st));
+      const size_t count = (size_t)info.n_huge + 1;
+      std::unique_ptr<LongSet[]> list(new (std::nothrow) LongSet[count]);
+      if (!list) return cuda_fail(cudaErrorMemoryAllocation, "long sets", __FILE__, __LINE__);
+      RST_CUDA(cudaMemcpyAsync(list.get(), huge, sizeof(LongSet) * count, cudaMemcpyDeviceToHost,
+                               st));
       RST_CUDA(cudaStreamSynchronize(st));
       for (int i = 1; i <= list[0].d; ++i) {
-        const LongSet& s = list[(size_t)i];
+        const LongSet& s = list[i];
         RST_CHECK(build_huge<HIER>(t, d_elems, s.rs, s.d, (int64_t)1 << s.lg, s.toff, st));
       }
     }

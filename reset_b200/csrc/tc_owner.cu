@@ -1143,8 +1143,11 @@ extern "C" reset_status reset_tc_count_batch(const reset_table* t, const int32_t
     if (!sparse)
       s = tc_owner(t, t->d_desc, d_off, d_cols, m, d_off, d_cols, t->d_chunk_row, m, total, st,
                    owner_hits);
-    if (s == RESET_ERR_OOM) cudaGetLastError();  // no memory for the groups (nothing ran)
-    if (sparse || s == RESET_ERR_OOM)
+    if (s == RESET_ERR_OOM) {  // no memory for the groups
+      cudaGetLastError();
+      e = cudaMemsetAsync(buf, 0, own_bytes + 256, st);
+    }
+    if (e == cudaSuccess && (sparse || s == RESET_ERR_OOM))
       s = tc_edges(t, t->d_desc, d_cols, d_off, d_cols, t->d_chunk_row, m, total, st, owner_hits);
   }
   if (e == cudaSuccess && s == RESET_OK)
