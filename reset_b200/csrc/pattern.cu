@@ -661,8 +661,9 @@ __global__ void __launch_bounds__(kPtThreads, 4)
               continue;
             }
             if (!level_ok(sp, lv, x, map)) continue;
+            int4 dx = make_int4(0, 0, 0, 0);
             if (!fixed) {
-              const int4 dx = __ldg(desc + x);
+              dx = __ldg(desc + x);
               base = cols + dx.x;
               nbase = dx.y;
               if (rcut && rr != lv) nbase = lower_bound_key(base, nbase, map[rr]);
@@ -675,14 +676,14 @@ __global__ void __launch_bounds__(kPtThreads, 4)
               for (int q = 0; q < lv; ++q) seen |= map[q] == x;
               at_bound = same ? j : lower_bound_key(base, nbase, x);
               c2 = kept - (!seen && at_bound < nbase && (same || base[at_bound] == x));
-            } else if (dist) {
+            } else if (dist && nbase > 0) {  // (no bound then) N(x) but the earlier vertices
+              const uint32_t* bx = br.of(x);
               for (int i = 0; i <= lv; ++i) {
+                if (i == lv && loop_free) break;
                 const int y = i == lv ? x : map[i];
                 bool seen = false;
                 for (int q = 0; q < i; ++q) seen |= map[q] == y;
-                if (seen) continue;
-                const int at = lower_bound_key(base, nbase, y);
-                if (at < nbase && base[at] == y) --c2;
+                if (!seen) c2 -= holds(bx, dx, y);
               }
             }
             hits += c2;
