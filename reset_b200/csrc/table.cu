@@ -101,6 +101,7 @@ struct BuildInfo {
   int32_t n_huge;   // ... of kHugeKeys keys or more
   unsigned long long long_keys, long_buckets;
   int64_t bucket_num;
+  unsigned long long keys_lg[16];  // keys of the long sets of 2^i .. 2^(i+1) - 1 keys
 };
 
 // Sets [bid * per, (bid + 1) * per) of block bid.
@@ -127,6 +128,7 @@ __global__ void __launch_bounds__(kThreads)
       const int at = atomicAdd(&info->n_long, 1);
       if (at < long_cap) long_list[at] = (int32_t)u;
       if (d >= kHugeKeys) atomicAdd(&info->n_huge, 1);
+      else atomicAdd(&info->keys_lg[31 - __clz(max(d, 1))], (unsigned long long)d);
       atomicAdd(&info->long_keys, (unsigned long long)d);
       atomicAdd(&info->long_buckets, (unsigned long long)l);
     }
@@ -570,10 +572,12 @@ constexpr int kWalkMax = 256;
 constexpr int kRunMax = 96;
 
 struct LongSet {
-  int32_t crowded;  // by its load: nothing is tried first
+  int32_t crowded;  // from the start: a warp inserts it, or build_huge
   int32_t rs, d, lg;
   int64_t toff;
-  int32_t key_item, bucket_item;  // its first items
+  // its first items: keys, buckets, and buckets of sets that are not crowded
+  // from the start (which have no items of keys either)
+  int32_t key_item, bucket_item, work_item;
 };
 
 // Whether runs of more than kRunMax keys are likely among `keys` keys at this
@@ -585,19 +589,19 @@ __device__ __forceinline__ bool crowded_by_load(float load, float keys) {
 }
 
 // The long sets' descriptors, the prefix sums of their items, and which are
-// crowded by their load (one block).
+// crowded by their load or inserted by a warp each for their number (one block).
 __global__ void __launch_bounds__(1024)
     long_plan_kernel(const int32_t* __restrict__ off, const int32_t* __restrict__ len,
                      const int64_t* __restrict__ off64, const int32_t* __restrict__ list, int n,
-                     int b, float all_keys, LongSet* __restrict__ sets,
+                     int b, float all_keys, int warp_keys, LongSet* __restrict__ sets,
                      LongSet* __restrict__ huge, int32_t* __restrict__ crowded) {
   using Scan = cub::BlockScan<int, 1024>;
   __shared__ typename Scan::TempStorage tmp;
-  int keys = 0, buckets = 0;  // items before this pass
+  int keys = 0, buckets = 0, work = 0;  // items before this pass
   for (int base = 0; base < n; base += 1024) {
     const int i = base + threadIdx.x;
     LongSet s{};
-    int ki = 0, bi = 0;
+    int ki = 0, bi = 0, wi = 0;
     if (i < n) {
       const int u = list[i];
       s.rs = off[u];
@@ -605,11 +609,15 @@ __global__ void __launch_bounds__(1024)
       const int l = len[u];
       s.lg = 31 - __clz(l);
       s.toff = off64[u];
-      ki = (s.d + kKeyItem - 1) / kKeyItem;
       bi = (l + kBucketItem - 1) / kBucketItem;
-      s.crowded = crowded_by_load((float)s.d / ((float)l * (float)b),
+      s.crowded = s.d < warp_keys ||
+                  crowded_by_load((float)s.d / ((float)l * (float)b),
                                   s.d >= kHugeKeys ? (float)s.d : all_keys);
       crowded[i] = s.crowded;
+      if (!s.crowded) {
+        ki = (s.d + kKeyItem - 1) / kKeyItem;
+        wi = bi;
+      }
     }
     int total;
     __syncthreads();
@@ -620,12 +628,17 @@ __global__ void __launch_bounds__(1024)
     Scan(tmp).ExclusiveSum(bi, s.bucket_item, total);
     s.bucket_item += buckets;
     buckets += total;
+    __syncthreads();
+    Scan(tmp).ExclusiveSum(wi, s.work_item, total);
+    s.work_item += work;
+    work += total;
     if (i < n) sets[i] = s;
   }
   if (threadIdx.x == 0) {
     LongSet end{};
     end.key_item = keys;
     end.bucket_item = buckets;
+    end.work_item = work;
     sets[n] = end;
     huge[0] = LongSet{};
   }
@@ -636,7 +649,8 @@ template <int32_t LongSet::*FIRST>
 __device__ __forceinline__ int long_set_of(const LongSet* __restrict__ sets, int n, int item) {
   __shared__ int s_i;
   if (threadIdx.x == 0) {
-    int lo = 0, hi = n;  // largest i with first item <= item
+    // largest i with first item <= item
+    int lo = sets[n].*FIRST <= item ? n : 0, hi = n;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
       if (sets[mid].*FIRST <= item) lo = mid; else hi = mid - 1;
@@ -650,11 +664,10 @@ __device__ __forceinline__ int long_set_of(const LongSet* __restrict__ sets, int
 __global__ void __launch_bounds__(kThreads)
     long_clear_kernel(const LongSet* __restrict__ sets, int n, int64_t bucket_num, int b,
                       int32_t* __restrict__ table) {
-  const int i = long_set_of<&LongSet::bucket_item>(sets, n, blockIdx.x);
+  const int i = long_set_of<&LongSet::work_item>(sets, n, blockIdx.x);
   if (i < 0) return;
   const LongSet s = sets[i];
-  if (s.crowded) return;  // (cleared where it is built)
-  const int h0 = ((int)blockIdx.x - s.bucket_item) * kBucketItem;
+  const int h0 = ((int)blockIdx.x - s.work_item) * kBucketItem;
   const int q = min(kBucketItem, (1 << s.lg) - h0) >> 2;
   const int4 neg = make_int4(-1, -1, -1, -1);
   for (int k = 0; k < b; ++k) {
@@ -671,7 +684,6 @@ __global__ void __launch_bounds__(kThreads)
   const int i = long_set_of<&LongSet::key_item>(sets, n, blockIdx.x);
   if (i < 0) return;
   const LongSet s = sets[i];
-  if (s.crowded) return;
   const int j0 = ((int)blockIdx.x - s.key_item) * kKeyItem;
   int32_t* G = table + s.toff;
   const int lmask = (1 << s.lg) - 1;
@@ -705,13 +717,13 @@ __global__ void __launch_bounds__(kThreads)
     long_fix_kernel(const int32_t* __restrict__ elems, const LongSet* __restrict__ sets, int n,
                     int64_t bucket_num, int b, int lg_max, int32_t* __restrict__ table,
                     int32_t* __restrict__ crowded) {
-  const int i = long_set_of<&LongSet::bucket_item>(sets, n, blockIdx.x);
+  const int i = long_set_of<&LongSet::work_item>(sets, n, blockIdx.x);
   if (i < 0) return;
   const LongSet s = sets[i];
   if (crowded[i]) return;
   int32_t* G = table + s.toff;
   const int lmask = (1 << s.lg) - 1;
-  const int h0 = ((int)blockIdx.x - s.bucket_item) * kBucketItem;
+  const int h0 = ((int)blockIdx.x - s.work_item) * kBucketItem;
   const int h1 = min(h0 + kBucketItem, lmask + 1);
   const int64_t last = (int64_t)(b - 1) * bucket_num;  // a bucket's last slot
   for (int h = h0 + threadIdx.x; h < h1; h += kThreads) {
@@ -1219,18 +1231,35 @@ reset_status launch_builds(const reset_table* t, const int32_t* d_off, const int
   int32_t* blk = reinterpret_cast<int32_t*>(base + 2 * sz_sets + sz_flag);
   int32_t* blk_off = reinterpret_cast<int32_t*>(base + 2 * sz_sets + sz_flag + sz_blk);
   void* scan_tmp = base + 2 * sz_sets + sz_flag + 2 * sz_blk;
+  // Sets short enough beside their number: a warp each fills the chip and takes
+  // fewer accesses per key, but no less than the longest one's chain.  Without
+  // rows, us, key-parallel / a warp per set: 10,000 sets of 1500 keys, 5 slots
+  // 914 / 780, one slot 1624 / 834; 2000 of 3000, one slot 723 / 382; 400 of 5000, 5
+  // slots 290 / 690.
+  int warp_keys = 0;
+  unsigned long long below = 0, by_warps = 0;
+  for (int i = 0; i < 16; ++i) {
+    below += info.keys_lg[i];
+    if (below >= 1000ull << (i + 1)) {
+      warp_keys = 2 << i;
+      by_warps = below;
+    }
+  }
+  const bool parallel = by_warps < info.long_keys;  // some are left
   auto run = [&]() -> reset_status {
     const int fill_smem = kBigFillSmemMax;
     RST_CUDA(cudaFuncSetAttribute(long_crowded_kernel<HIER>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, fill_smem));
-    note_launch(5);
+    note_launch(parallel ? 5 : 2);
     long_plan_kernel<<<1, 1024, 0, st>>>(d_off, t->d_len, t->d_off64, d_long, n, b,
-                                         (float)info.long_keys, sets, huge, crowded);
-    long_clear_kernel<<<(unsigned)bucket_items, kThreads, 0, st>>>(sets, n, bn, b, t->d_table);
-    long_insert_kernel<HIER><<<(unsigned)key_items, kThreads, 0, st>>>(
-        d_elems, sets, n, bn, b, t->lg_max, t->d_table, crowded);
-    long_fix_kernel<HIER><<<(unsigned)bucket_items, kThreads, 0, st>>>(
-        d_elems, sets, n, bn, b, t->lg_max, t->d_table, crowded);
+                                         (float)info.long_keys, warp_keys, sets, huge, crowded);
+    if (parallel) {
+      long_clear_kernel<<<(unsigned)bucket_items, kThreads, 0, st>>>(sets, n, bn, b, t->d_table);
+      long_insert_kernel<HIER><<<(unsigned)key_items, kThreads, 0, st>>>(
+          d_elems, sets, n, bn, b, t->lg_max, t->d_table, crowded);
+      long_fix_kernel<HIER><<<(unsigned)bucket_items, kThreads, 0, st>>>(
+          d_elems, sets, n, bn, b, t->lg_max, t->d_table, crowded);
+    }
     long_crowded_kernel<HIER><<<n, kThreads, fill_smem, st>>>(
         d_elems, sets, crowded, bn, b, t->lg_max, t->d_table, huge, t->d_status);
     RST_CUDA(cudaGetLastError());

@@ -456,6 +456,35 @@ def test_builds_near_full_load(R, cuda, oracle_mod, bucket, keys):
     assert _best_ms(cuda, build) < 1e-4 * keys
 
 
+@pytest.mark.parametrize("alpha,bucket", [(0.2, 5), (0.25, 1)])
+def test_builds_of_many_long_sets(R, cuda, oracle_mod, alpha, bucket):
+    """So many sets just past a tile that a warp each inserts them, longer ones
+    among them key-parallel."""
+    rng = np.random.default_rng(0x5EED7E60)
+    rows = [rng.choice(1 << 26, 1300 + i % 700, replace=False) for i in range(2200)]
+    _check_build(R, cuda, oracle_mod, rows, alpha, bucket, False)
+    rows[100:2200:700] = [rng.choice(1 << 26, 9000, replace=False) for _ in range(3)]
+    _check_build(R, cuda, oracle_mod, rows, alpha, bucket, True)
+
+
+@pytest.mark.parametrize("n,edges,hub", [(300, 3000, 0), (500, 1500, 40), (2000, 30000, 300)])
+def test_path_patterns(R, cuda, oracle_mod, n, edges, hub):
+    """A last level that is the row of the vertex before it, less the earlier
+    vertices; rows with and without loops, with and without bit rows."""
+    off, cols = _random_symmetric(np.random.default_rng(0x5EED8600 + n), n, edges, hub)
+    rows = [cols[off[u]:off[u + 1]] for u in range(n)]
+    for loops in (False, True):
+        if loops:
+            rows = [np.union1d(r, [u]) if u % 3 == 0 else r for u, r in enumerate(rows)]
+        o, c = csr(rows)
+        d_off, d_cols = dev(o, cuda), dev(c, cuda)
+        t = R.Table(d_off, d_cols)
+        for p in (R.PatternSpec(4, (0, 1, 2, 3), (0, 1, 2), None, None, 2),
+                  R.PatternSpec(4, (0, 1, 3, 4), (0, 0, 1, 2), (-1, 0, -1, -1), None, 3)):
+            assert R.pattern_count(t, d_off, d_cols, p) == _oracle_pattern(oracle_mod, o, c, p)
+        t.check()
+
+
 @pytest.mark.parametrize("alpha,bucket", [(0.2, 5), (1.0, 1), (0.95, 16)])
 def test_builds_of_several_crowded_long_sets(R, cuda, oracle_mod, alpha, bucket):
     """Sets of 2^16 keys and more, crowded by a repeated key or by their load,
